@@ -33,7 +33,7 @@ struct Group {
   FftPlan plan{};
   float2 *tw = nullptr;       // float twiddles [f]
   double2 *tw64 = nullptr;    // double twiddles [f]
-  float2 *P[2] = {nullptr, nullptr};   // packed matrices [slot][nkp half blocks][nrow][RS]
+  float2 *P[2] = {nullptr, nullptr};   // packed matrices [slot][nkp half blocks][nrow][NP][C, D]
   bool built[2] = {false, false};
   std::vector<int> planes;    // plane ids of the group, ascending (slot = index)
   int *d_ids = nullptr;       // device copy of `planes`
@@ -68,9 +68,7 @@ struct flf_ctx {
   std::vector<int> h[2];
   Geometry geo;
   // index tables (device)
-  short4 *d_rowS = nullptr, *d_oslots = nullptr;
-  short *d_rowF = nullptr;
-  short *d_slotcol = nullptr, *d_colslot = nullptr;
+  short4 *d_rowS = nullptr;
   int *d_rep_ch = nullptr, *d_rep_row = nullptr, *d_rep_kind = nullptr;
   int *d_planes_all = nullptr;
   int *d_planes_user = nullptr;   // per-call plane subsets: ids then slots, per group
@@ -265,116 +263,58 @@ void free_all_geometries(flf_ctx *ctx) {
   ctx->parked.clear();
 }
 
-// Host-side index tables of the packed layout (see flf_internal.cuh).
+// Host-side index tables of the packed layout (see Layout in flf_internal.cuh).
 int build_tables(flf_ctx *ctx) {
   const int N = ctx->N, NN = N * N, c = N / 2;
   const Layout &L = ctx->L;
   auto My = [&](int i) { return (N - 1 - i / N) * N + i % N; };
   auto Mx = [&](int i) { return (i / N) * N + (N - 1 - i % N); };
   auto Mxy = [&](int i) { return NN - 1 - i; };
-  // Slot order of a stored row: for the c^2 generic orbits o = be*c + al,
-  // four blocks of c^2 slots (q, My q, Mx q, Mxy q of every orbit), then the
-  // c orbits [q, My q] (alpha = c) as two blocks of c, the c orbits [q, Mx q]
-  // (beta = c) as two blocks of c, then the centre.  A warp's threads (one
-  // orbit each) read each block with consecutive addresses.
-  const int c2 = c * c;
-  std::vector<short> slotcol(NN, -1);
-  for (int be = 0; be < c; be++)
-    for (int al = 0; al < c; al++) {
-      const int o = be * c + al, q = be * N + al;
-      slotcol[o] = q; slotcol[c2 + o] = My(q); slotcol[2 * c2 + o] = Mx(q); slotcol[3 * c2 + o] = Mxy(q);
-    }
-  for (int j = 0; j < c; j++) {
-    const int qa = j * N + c, qb = c * N + j;
-    slotcol[4 * c2 + j] = qa; slotcol[4 * c2 + c + j] = My(qa);
-    slotcol[4 * c2 + 2 * c + j] = qb; slotcol[4 * c2 + 3 * c + j] = Mx(qb);
-  }
-  slotcol[4 * c2 + 4 * c] = c * N + c;
-  for (int sl = 0; sl < NN; sl++)
-    if (slotcol[sl] < 0) return fail(ctx, FLF_E_STATE, "internal: slot table");
-  std::vector<short> colslot(NN, -1);
-  for (int s = 0; s < NN; s++) colslot[slotcol[s]] = s;
-
   auto Tr = [&](int i) { return (i % N) * N + i / N; };
-  // virtual slots [q, My q, Mx q, Mxy q] of each output orbit (degenerate orbits
-  // repeat their entries) and the slots of the transposed channels in the same order
-  std::vector<short4> oslots(2 * L.nthr);
-  for (int o = 0; o < L.nthr; o++) {
-    int off[4];
-    if (o < c2) {
-      off[0] = o; off[1] = c2 + o; off[2] = 2 * c2 + o; off[3] = 3 * c2 + o;
-    } else if (o < c2 + c) {
-      const int j = o - c2;
-      off[0] = off[2] = 4 * c2 + j; off[1] = off[3] = 4 * c2 + c + j;
-    } else if (o < c2 + 2 * c) {
-      const int j = o - c2 - c;
-      off[0] = off[1] = 4 * c2 + 2 * c + j; off[2] = off[3] = 4 * c2 + 3 * c + j;
-    } else {
-      off[0] = off[1] = off[2] = off[3] = NN - 1;
-    }
-    int offT[4];
-    for (int k = 0; k < 4; k++) offT[k] = colslot[Tr(slotcol[off[k]])];
-    oslots[o] = make_short4(off[0], off[1], off[2], off[3]);
-    oslots[L.nthr + o] = make_short4(offT[0], offT[1], offT[2], offT[3]);
-  }
-  // row groups of a half block with their operands for the own frequency pair
-  // (use 0) and, through the transpose, for the other one of the quad (use 1)
-  std::vector<short4> rowS(2 * L.ngrp, make_short4(0, 0, 0, 0));
-  std::vector<short> rowF(2 * L.ngrp, 0);
+  // per row the operand channels (sa, sb at u; sa, sb at u*) for the own
+  // frequency pair, then for the other one of the quad, then the flags
+  std::vector<short4> rowS(3 * L.nrow, make_short4(-1, -1, -1, -1));
   ctx->rep_ch.clear(); ctx->rep_row.clear(); ctx->rep_kind.clear();
-  auto generic_ops = [&](int x, bool mxrow, short4 &si, short &fl) {
-    si = make_short4(x, Mxy(x), NN + My(x), NN + Mx(x));
-    fl = (short)((1 << 1) | (1 << 3) | (mxrow ? 0xF0 : 0));
-  };
-  int row = 0, grp = 0;
-  std::vector<std::pair<int, int>> orbits;   // transposable orbits (a' < b) first, then the diagonal ones
-  for (int b = 0; b < c; b++)
-    for (int ap = 0; ap < b; ap++) orbits.push_back({b, ap});
-  for (int b = 0; b < c; b++) orbits.push_back({b, b});
-  for (const auto &ob : orbits) {
-    const int b = ob.first, ap = ob.second;
-    for (int a : {ap, N - 1 - ap}) {
-        const int i = b * N + a;
-        const bool trans = ap < b, mxrow = a > c;
-        generic_ops(i, mxrow, rowS[grp], rowF[grp]);
-        if (trans) {
-          generic_ops(Tr(i), mxrow, rowS[L.ngrp + grp], rowF[L.ngrp + grp]);
-          rowF[grp] |= kRowTransposable;
-          rowF[L.ngrp + grp] |= kRowTransposable;
-        }
-        ctx->rep_ch.push_back(i); ctx->rep_row.push_back(row); ctx->rep_kind.push_back(0);
-        row++; grp++;
-      }
-  }
-  if (row != L.nrowG) return fail(ctx, FLF_E_STATE, "internal: generic row table size");
-  for (int k = 0; k <= c; k++) {
-    const bool centre = k == c;
-    const int i = centre ? c * N + c : k * N + c;
-    if (centre) {
-      rowS[grp] = make_short4(i, NN + i, 0, 0);
-      rowF[grp] = (short)((1 << 5) | (1 << 10) | (1 << 11));
-    } else {
-      rowS[grp] = make_short4(i, NN + i, NN + My(i), My(i));
-      rowF[grp] = (short)((1 << 5) | (1 << 7) | kRowTransposable);
-      const int x = Tr(i);   // (c, b): the row pair read through the transpose, conjugated u* terms
-      rowS[L.ngrp + grp] = make_short4(x, NN + x, NN + Mx(x), Mx(x));
-      rowF[L.ngrp + grp] = (short)((1 << 1) | (1 << 2) | (1 << 5) | (1 << 7) | kRowTransposable);
+  int row = 0;
+  auto add_row = [&](short4 own, short4 other, bool second) {
+    if (row < L.nrow) {
+      rowS[row] = own;
+      rowS[L.nrow + row] = other;
+      rowS[2 * L.nrow + row] = make_short4(second ? kRowSecond : 0, 0, 0, 0);
     }
-    ctx->rep_ch.push_back(i); ctx->rep_row.push_back(row); ctx->rep_kind.push_back(1);
-    row += 2; grp++;
+    row++;
+  };
+  auto add_rep = [&](int ch, int kind) {
+    ctx->rep_ch.push_back(ch); ctx->rep_row.push_back(row); ctx->rep_kind.push_back(kind);
+  };
+  const short4 none = make_short4(-1, -1, -1, -1);
+  auto generic = [&](int x) { return make_short4(x, Mxy(x), My(x), Mx(x)); };
+  auto add_orbit = [&](int b, int ap) {   // rows (b, a') and its Mx mirror
+    for (int a : {ap, N - 1 - ap}) {
+      const int x = b * N + a;
+      add_rep(x, 0);
+      add_row(generic(x), ap < b ? generic(Tr(x)) : none, a > c);
+    }
+  };
+  for (int b = 0; b < c; b++)
+    for (int ap = 0; ap < b; ap++) add_orbit(b, ap);
+  for (int b = 0; b < c; b++) {
+    // (b, c): no Mxy mirror, the My partner y.  Through the transpose, the (c, b)
+    // channel X and its Mx partner Y, whose terms at u* are conjugated
+    const int x = b * N + c, y = My(x), X = Tr(x), Y = Mx(Tr(x));
+    add_rep(x, 1);
+    add_row(make_short4(x, -1, y, -1), make_short4(X, -1, -1, Y), false);
+    add_row(make_short4(y, -1, x, -1), make_short4(Y, -1, -1, X), true);
   }
-  if (row != L.nrow || grp != L.ngrp) return fail(ctx, FLF_E_STATE, "internal: row table size");
+  if (row != L.nrowT) return fail(ctx, FLF_E_STATE, "internal: transposable row table size");
+  for (int b = 0; b < c; b++) add_orbit(b, b);
+  add_rep(c * N + c, 1);
+  add_row(make_short4(c * N + c, -1, -1, -1), none, false);
+  add_row(make_short4(-1, -1, c * N + c, -1), none, true);
+  if (row != L.nrow) return fail(ctx, FLF_E_STATE, "internal: row table size");
   const int nrepAll = (int)ctx->rep_ch.size();
   CUDA_TRY(ctx, cudaMalloc(&ctx->d_rowS, sizeof(short4) * rowS.size()));
   CUDA_TRY(ctx, cudaMemcpy(ctx->d_rowS, rowS.data(), sizeof(short4) * rowS.size(), cudaMemcpyHostToDevice));
-  CUDA_TRY(ctx, cudaMalloc(&ctx->d_rowF, sizeof(short) * rowF.size()));
-  CUDA_TRY(ctx, cudaMemcpy(ctx->d_rowF, rowF.data(), sizeof(short) * rowF.size(), cudaMemcpyHostToDevice));
-  CUDA_TRY(ctx, cudaMalloc(&ctx->d_oslots, sizeof(short4) * oslots.size()));
-  CUDA_TRY(ctx, cudaMemcpy(ctx->d_oslots, oslots.data(), sizeof(short4) * oslots.size(), cudaMemcpyHostToDevice));
-  CUDA_TRY(ctx, cudaMalloc(&ctx->d_slotcol, sizeof(short) * NN));
-  CUDA_TRY(ctx, cudaMemcpy(ctx->d_slotcol, slotcol.data(), sizeof(short) * NN, cudaMemcpyHostToDevice));
-  CUDA_TRY(ctx, cudaMalloc(&ctx->d_colslot, sizeof(short) * NN));
-  CUDA_TRY(ctx, cudaMemcpy(ctx->d_colslot, colslot.data(), sizeof(short) * NN, cudaMemcpyHostToDevice));
   CUDA_TRY(ctx, cudaMalloc(&ctx->d_rep_ch, sizeof(int) * nrepAll));
   CUDA_TRY(ctx, cudaMemcpy(ctx->d_rep_ch, ctx->rep_ch.data(), sizeof(int) * nrepAll, cudaMemcpyHostToDevice));
   CUDA_TRY(ctx, cudaMalloc(&ctx->d_rep_row, sizeof(int) * nrepAll));
@@ -450,8 +390,7 @@ int build_group(flf_ctx *ctx, Group &G, int fp64, int dir, cudaStream_t s) {
         pp.L = L; pp.f = f; pp.fh = fh; pp.fq = G.fq; pp.nkp = G.nkp;
         pp.spec = wspec.p; pp.rep0 = r0; pp.nrep_chunk = nr;
         pp.rep_row = ctx->d_rep_row; pp.rep_kind = ctx->d_rep_kind; pp.rep_ch = ctx->d_rep_ch;
-        pp.col_slot = ctx->d_colslot;
-        pp.P = G.P[dir] + plane_elems * sl;
+        pp.P = (float4 *)(G.P[dir] + plane_elems * sl);
         pp.scale = 1.0 / ((double)f * (double)f);
         pp.fp64 = fp64;
         e = launch_pack(pp, s);
@@ -788,6 +727,16 @@ void mac_shape(const flf_ctx *ctx, int dir, int &stages, int &chunk_rows, int &s
   while (split > 1 && 2 * split * ntp > 256) split--;   // at most 256 threads per block
 }
 
+// Shared-memory budget by which launch shapes are accepted (flf_set_option,
+// flf_set_tuned): that of a pipeline with an operand table of 256 B per mirror
+// orbit.  k_mac needs no more than this for one frame (mac_smem_bytes), so every
+// shape accepted here, saved ones included, fits.
+size_t mac_shape_bytes(const Layout &L, int stages, int chunk_rows, int split) {
+  const size_t comb = (size_t)2 * 4 * L.NN, red = (size_t)(2 * split - 1) * ((L.nthr + 31) / 32 * 32) * 8;
+  return sizeof(float2) * ((size_t)stages * chunk_rows * L.RS + std::max(comb, red)) + (size_t)268 * L.nthr +
+         2 * sizeof(unsigned long long) * stages + 16;
+}
+
 // Frames one multiply-accumulate pass takes: mac_max_frames(), or fewer where
 // the ring, the staged spectra and the operand tables of that many frames do
 // not fit shared memory with the current launch shape (Nnum 19 at 12 rows per
@@ -798,7 +747,7 @@ int frames_per_pass(const flf_ctx *ctx) {
     for (int d = 0; d < 2; d++) {
       int st, cr, sp;
       mac_shape(ctx, d, st, cr, sp);
-      if (mac_smem_bytes(ctx->L, tf, st, cr, sp, d == FLF_DIR_FORWARD) > kMacSmemMax) fits = false;
+      if (mac_smem_bytes(ctx->L, tf, st, cr, d == FLF_DIR_FORWARD) > kMacSmemMax) fits = false;
     }
     if (fits) return tf;
   }
@@ -808,8 +757,8 @@ int frames_per_pass(const flf_ctx *ctx) {
 MacParams mac_params(const flf_ctx *ctx, const Group &G, int dir, int nt) {
   MacParams mp{};
   mp.L = ctx->L; mp.f = G.f; mp.fh = G.fh; mp.fq = G.fq; mp.nkp = G.nkp; mp.nquads = G.nquads; mp.T = nt;
-  mp.P = G.P[dir];
-  mp.rowS = ctx->d_rowS; mp.rowF = ctx->d_rowF; mp.oslots = ctx->d_oslots; mp.slotcol = ctx->d_slotcol;
+  mp.P = (const float4 *)G.P[dir];
+  mp.rowS = ctx->d_rowS;
   mac_shape(ctx, dir, mp.stages, mp.chunk_rows, mp.split);
   mp.err = ctx->d_err;
   mp.wait_ns = (unsigned long long)ctx->opt_wait_us * 1000ull;
@@ -1089,8 +1038,7 @@ int flf_ctx_destroy(flf_ctx *ctx) {
   resolve_pending(ctx);
   for (cudaEvent_t e : ctx->evpool) cudaEventDestroy(e);
   free_all_geometries(ctx);
-  void *ptrs[] = {ctx->d_rowS, ctx->d_rowF, ctx->d_oslots, ctx->d_slotcol, ctx->d_colslot, ctx->d_rep_ch, ctx->d_rep_row,
-                  ctx->d_rep_kind, ctx->d_planes_all, ctx->d_planes_user, ctx->d_zero,
+  void *ptrs[] = {ctx->d_rowS, ctx->d_rep_ch, ctx->d_rep_row, ctx->d_rep_kind, ctx->d_planes_all, ctx->d_planes_user, ctx->d_zero,
                   ctx->wsS.p, ctx->wsO.p, ctx->wsCvol.p, ctx->wsCimg.p, ctx->wsCy.p};
   for (void *p : ptrs)
     if (p) cudaFree(p);
@@ -1659,7 +1607,7 @@ int flf_set_option(flf_ctx *ctx, const char *name, long long value) {
       return fail(ctx, FLF_E_ARG, "mac_split must be in [1, 4] with at most 256 threads per block "
                                   "(2 frequency pairs x split x %d orbit threads)", ntp);
     for (int cr : {crf, crb})
-      if (mac_smem_bytes(ctx->L, 1, st, cr, sp, true) > kMacSmemMax)
+      if (mac_shape_bytes(ctx->L, st, cr, sp) > kMacSmemMax)
         return fail(ctx, FLF_E_ARG, "pipeline of %d stages x %d rows exceeds shared memory", st, cr);
     ctx->opt_stages = st;
     ctx->opt_chunk_rows[FLF_DIR_FORWARD] = crf;
@@ -1715,7 +1663,8 @@ int flf_autotune(flf_ctx *ctx, int T, int Y, int X, int *out4, void *stream) {
       for (int b = 0; b < 2 && e == cudaSuccess; b++) {
         if (2 * split_c[b] * ntp > 256) continue;
         for (int ch : chunk_c) {
-          if (mac_smem_bytes(ctx->L, nt <= 1 ? 1 : (nt <= 2 ? 2 : 4), stages_c[a], ch, split_c[b], true) > kMacSmemMax)
+          if (mac_shape_bytes(ctx->L, stages_c[a], ch, split_c[b]) > kMacSmemMax ||   // flf_set_tuned takes it
+              mac_smem_bytes(ctx->L, nt, stages_c[a], ch, true) > kMacSmemMax)
             continue;
           e = mac_group_launch(ctx, gi, d, nt, ps, stages_c[a], ch, split_c[b], s);   // warm-up
           if (e == cudaSuccess) e = cudaEventRecord(e0, s);
@@ -1759,7 +1708,7 @@ int flf_set_tuned(flf_ctx *ctx, int Y, int X, const int *in4) {
     return fail(ctx, FLF_E_ARG, "invalid launch shape");
   for (int d = 1; d <= 2; d++)
     if (in4[d] < 2 || in4[d] > 64 || (in4[d] & 1) ||
-        mac_smem_bytes(ctx->L, 1, in4[0], in4[d], in4[3], true) > kMacSmemMax)
+        mac_shape_bytes(ctx->L, in4[0], in4[d], in4[3]) > kMacSmemMax)
       return fail(ctx, FLF_E_ARG, "invalid rows per chunk %d", in4[d]);
   for (int i = 0; i < 4; i++) Gm.tuned[i] = in4[i];
   return FLF_OK;

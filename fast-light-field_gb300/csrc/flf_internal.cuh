@@ -47,48 +47,48 @@ struct FftPlan {
 // uy)}, uy <= ux, ordered ux-major: quad k = ux(ux+1)/2 + uy.  Each quad holds
 // one half block per frequency pair (one for a diagonal quad uy = ux): half
 // blocks 2k - ux and 2k - ux + 1, so a plane has fq^2 half blocks in all.
-//   P[half block][row][slot], rows = (c+1)(c+2) per half block, slot stride RS.
+//   P[half block][row][pair] = (C, D): rows = (c+1)(c+2) per half block, NP =
+//   (NN+1)/2 pairs of output channels (j, j'), j = 0..NP-1, j' = Mxy j = NN-1-j
+//   (the last pair is the centre with itself), row stride RS = 2 NP complex.
+// A pair's two numbers are C = (A + B) / 2 and D = i (A - B) / 2 of A = T_xj and
+// B = conj T_xj'.  The mirror Mxy maps a frequency to itself, so the inputs x and
+// x' = Mxy x share the row: with w = s_x + conj s_x' and v = s_x - conj s_x',
+//   P = C Re w + D Im w,  M = C Im v - D Re v,  out_j = P + iM, out_j' = conj P + i conj M,
+// half the multiplications of the complex products T_xj s_x, T_x'j s_x'.  At u*
+// the same row is T of My x, to the channels (My j, Mx j).
 // Rows of a half block: the generic input orbits (b, a'), a' <= b < c, as their
-// rows i = (b, a') and Mx i = (b, N-1-a') at u (c(c+1) rows, the c(c-1) rows
-// of the orbits with a' < b first); then row pairs (u, u*) of the centre-cross
-// representatives (b, c), b < c, and of the centre.  Orbits with a' < b and the
-// (b, c) pairs also stand for their transposes (a', b) and (c, b), which have
-// no rows.  Slots: output channels of the mirror orbits, slot-major: the c^2
-// generic orbits [q, My q, Mx q, Mxy q] as four blocks of c^2, the c orbits
-// [q, My q] (alpha = c) and the c orbits [q, Mx q] (beta = c) as two blocks of
-// c each, then the centre.  The second half block of a quad keeps its columns
-// in transposed order (the slot of channel j holds channel Tr j); thread t of
-// the second frequency pair owns the transposed orbit of t, so both sides read
-// both half blocks at the slots of orbit t: consecutive for a warp.
+// rows x = (b, a') and Mx x = (b, N-1-a') at u; row pairs of the centre-cross
+// representatives x = (b, c), b < c, and of the centre: T_xj at u, then T at u*
+// with mirrored columns (My j, Mx j), which makes it a row like any other (of
+// My x at u).  Orbits with a' < b and the (b, c) pairs also stand for their
+// transposes (a', b) and (c, b), which have no rows; they are stored first
+// (nrowT rows): orbits a' < b, row pairs (b, c), orbits a' = b, centre.
+// The second half block of a quad keeps its columns in transposed order (the
+// place of channel j holds channel Tr j), so both frequency pairs of a quad read
+// both half blocks at the same places; a lane's pair stands for (Tr j, Tr j') there.
 struct Layout {
   int N, NN, c, nh;
-  int nrowG;      // c(c+1) generic rows per half block
-  int nrowGT;     // c(c-1) of them (stored first) stand for their transposes too
-  int nrep;       // c+1 row pairs per half block
+  int NP;         // (NN+1)/2 pairs of output channels
+  int nrowT;      // c(c+1) rows (stored first) stand for their transposes too
   int nrow;       // (c+1)(c+2) rows per half block
-  int ngrp;       // (c+1)^2 row groups (generic rows and row pairs) per half block
-  int RS;         // row stride in complex elements
-  int nthr;       // nh^2: output orbits (threads per row share)
+  int RS;         // row stride in complex elements (2 NP)
+  int nthr;       // nh^2 mirror orbits: the unit of the accepted launch shapes (mac_split)
 };
 
 inline Layout make_layout(int N) {
   Layout L;
   L.N = N; L.NN = N * N; L.c = N / 2; L.nh = L.c + 1;
-  L.nrowG = L.c * (L.c + 1);
-  L.nrowGT = L.c * (L.c - 1);
-  L.nrep = L.c + 1;
-  L.nrow = L.nrowG + 2 * L.nrep;
-  L.ngrp = L.nrowG + L.nrep;
-  L.RS = (L.NN + 1) & ~1;
+  L.NP = (L.NN + 1) / 2;
+  L.nrowT = L.c * (L.c + 1);
+  L.nrow = (L.c + 1) * (L.c + 2);
+  L.RS = 2 * L.NP;
   L.nthr = L.nh * L.nh;
   return L;
 }
 
-// Row-group flags (MacParams::rowF): bits 0-3 conjugate operand j, bits 4-7
-// zero operand j when the receiving frequency pair is self-paired (u = u*),
-// bits 8-11 operand j always zero, bit 12 the group also feeds the other
-// frequency pair of its quad through the transpose.
-constexpr int kRowTransposable = 1 << 12;
+// Row flag (third part of MacParams::rowS, .x): a row that repeats its
+// predecessor where the frequency is self-paired (u = u*).
+constexpr short kRowSecond = 1;
 
 // ----------------------------------------------------------------------------
 // Runtime division by an invariant divisor d (1 <= d < 2^16) for n < 2^16:
@@ -196,7 +196,7 @@ struct MacParams {
   int f, fh, fq, nkp;       // transform size, f/2+1, f/2+1, fq*fq half blocks per plane
   int nquads;               // fq(fq+1)/2 frequency quads (grid.x)
   int T;                    // frames in this launch (<= template TF)
-  const float2 *P;          // packed matrices [plane][half block][nrow][RS]
+  const float4 *P;          // packed matrices [plane][half block][nrow][NP]
   const int *planes;        // plane id per z index
   int nz;                   // planes in the list
   int zgroup;               // forward: planes per CTA group
@@ -205,14 +205,13 @@ struct MacParams {
   float2 *O;                // output spectra
   int nzo;                  // forward: number of z groups (output sets); backward: nz
   int nzo_grid;             // grid.y: number of z groups of this launch
-  const short4 *rowS;       // [2][ngrp]: operand channels of each row group for its own frequency
-                            // pair (use 0) and through the transpose (use 1); + NN: at u*
-  const short *rowF;        // [2][ngrp]: operand flags (kRowTransposable, conj / zero bits)
-  const short4 *oslots;     // [2][nthr]: an orbit's four virtual slots, own and transposed
-  const short *slotcol;     // slot -> output channel
+  const short4 *rowS;       // [3][nrow]: operand channels of each row for its own frequency pair (0)
+                            // and through the transpose (1): sa, sb at u, sa, sb at u* (-1: none);
+                            // then the row flags (.x)
   int stages;               // shared-memory ring stages of the bulk-copy pipeline
   int chunk_rows;           // stored rows per stage (even)
-  int split;                // threads sharing one orbit's rows (1..4)
+  int split;                // threads per quad in units of about 128 (1..4)
+  int shares;               // row shares (set by the launcher)
   int *err;                 // set nonzero when a bounded wait gives up
   unsigned long long wait_ns;   // limit of each wait for a ring slot (1 s)
   int drop_chunk;           // test of the bounded waits: chunk the first CTA never issues (-1: none)
@@ -235,8 +234,7 @@ struct PackParams {
   const int *rep_row;       // packed row of representative (first row)
   const int *rep_kind;      // 0 generic row, otherwise a row pair (u, u*)
   const int *rep_ch;
-  const short *col_slot;    // channel -> slot
-  float2 *P;                // this plane's packed blocks [fq * fq][nrow][RS]
+  float4 *P;                // this plane's packed blocks [fq * fq][nrow][NP]
   double scale;             // 1/f^2
   int fp64;
 };
@@ -358,6 +356,8 @@ size_t rfft2_smem_bytes(int f, int imgs, int fp64);
 int mac_max_frames();
 // Shared memory one CTA may opt in to (sm_100 family).
 constexpr size_t kMacSmemMax = 227 * 1024;
-size_t mac_smem_bytes(const Layout &L, int TF, int stages, int chunk_rows, int split, bool fwd);
+size_t mac_smem_bytes(const Layout &L, int TF, int stages, int chunk_rows, bool fwd);
+struct MacThreads { int ppt, cw, shares; };   // channel pairs per lane, warps side by side, row shares
+MacThreads mac_threads(const Layout &L, int split);
 
 }  // namespace flf

@@ -5,6 +5,7 @@
 #include "flf_internal.cuh"
 #include "flf_fft.cuh"
 
+#include <algorithm>
 #include <cstdio>
 
 namespace flf {
@@ -25,21 +26,6 @@ template <typename C> __device__ __forceinline__ C cmul(C a, C b) {
   return cmk<C>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 template <typename C> __device__ __forceinline__ C cconj(C a) { return cmk<C>(a.x, -a.y); }
-
-// acc += a * b  (complex multiply-accumulate, 4 FMAs)
-__device__ __forceinline__ void cmac(float2 &acc, float2 a, float2 b) {
-  acc.x = fmaf(a.x, b.x, acc.x);
-  acc.x = fmaf(-a.y, b.y, acc.x);
-  acc.y = fmaf(a.x, b.y, acc.y);
-  acc.y = fmaf(a.y, b.x, acc.y);
-}
-// acc += conj(a) * b
-__device__ __forceinline__ void cmacc(float2 &acc, float2 a, float2 b) {
-  acc.x = fmaf(a.x, b.x, acc.x);
-  acc.x = fmaf(a.y, b.y, acc.x);
-  acc.y = fmaf(a.x, b.y, acc.y);
-  acc.y = fmaf(-a.y, b.x, acc.y);
-}
 
 // ----------------------------------------------------------------------------
 // Shared-memory Stockham FFT (mixed radix 2/3/4/5/7), batched over the images
@@ -191,16 +177,13 @@ __global__ void __launch_bounds__(256) k_rfft2(Rfft2Params p) {
 // ----------------------------------------------------------------------------
 // Fused spectral multiply-accumulate (the hot kernel).
 //
-// One CTA owns one frequency pair (u, u*) and, for forward projection, a group
-// of planes (accumulated in registers: the reference's plane sum moved into
-// Fourier space) or, for back projection, one plane.  Each thread owns one
-// mirror orbit of output channels (4, 2 or 1 channels) for both frequencies;
-// row groups split the stored rows and are reduced through shared memory at
-// the end.  Every stored matrix element is read once from HBM and feeds
-// 4 complex multiply-adds per frame.  This replaces the reference's
-// expandX + calculateRows{,Mirrored} launches (projector.py:395-459) and
-// CalculateRow/CalculateRowBoth (py_light_field.cpp:303-341), which read and
-// wrote the accumulator once per lenslet offset.
+// Forward projection accumulates a group of planes in registers (the
+// reference's plane sum moved into Fourier space), back projection writes one
+// plane after the other.  Every stored matrix element is read once from HBM.
+// This replaces the reference's expandX + calculateRows{,Mirrored} launches
+// (projector.py:395-459) and CalculateRow/CalculateRowBoth
+// (py_light_field.cpp:303-341), which read and wrote the accumulator once per
+// lenslet offset.
 // ----------------------------------------------------------------------------
 // ---------------------------------------------------------------------------
 // Bulk-copy pipeline primitives (sm_90+ PTX: mbarrier, cp.async.bulk).
@@ -263,141 +246,10 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 
 constexpr unsigned long long kWaitLimitNs = 1000000000ull;   // 1 s per wait
 
-// Loads the four virtual slots [q, My q, Mx q, Mxy q] of this thread's orbit
-// from one staged row at the thread's slot offsets.  Degenerate orbits repeat
-// their stored entries (alpha = c: [q, My q, q, My q]; beta = c:
-// [q, q, Mx q, Mx q]; centre: [q] x 4), so every thread runs the same 4-slot
-// update with no branch (the padded slots compute duplicates that are never
-// written).
-__device__ __forceinline__ void load_slots(const float2 *row, const int (&off)[4], float2 (&t)[4]) {
-#pragma unroll
-  for (int k = 0; k < 4; k++) t[k] = row[off[k]];
-}
-
-// Slot permutations of the orbit [q, My q, Mx q, Mxy q].
-__device__ __forceinline__ constexpr int sy(int k) { return k ^ 1; }
-__device__ __forceinline__ constexpr int sx(int k) { return k ^ 2; }
-__device__ __forceinline__ constexpr int sxy(int k) { return 3 - k; }
-
 // Packed two-lane FP32 arithmetic (sm_100+): __ffma2_rn performs two
 // independent IEEE fused multiply-adds in one instruction, halving the issue
-// slots of the complex multiply-accumulate.  f2x is the two-lane value.
-typedef float2 f2x;
-__device__ __forceinline__ f2x pk(float lo, float hi) { return make_float2(lo, hi); }
-__device__ __forceinline__ float2 unpk(f2x v) { return v; }
-__device__ __forceinline__ void ffma2(f2x &acc, f2x a, f2x b) { acc = __ffma2_rn(a, b, acc); }
-
-// Per row group, the input spectra enter as four packed operand pairs
-// (A_j, B_j), j = 0..3.  Each complex accumulator is kept as two lane pairs
-// P and Q with value (P.x - Q.y, P.y + Q.x), so that with t = (t.x, t.y)
-//   acc += t * s        is  P = fma2(t, (s.x, s.x)), Q = fma2(t, (s.y, s.y))
-//   acc += conj(t) * s  is  P = fma2(t, (s.x,-s.x)), Q = fma2(t, (s.y,-s.y))
-// and no lane swap of t is needed.  sv[tf][side][use][group][j] = float4(A_j, B_j)
-// for the threads of frequency pair `side` reading a group of their own half
-// block (use 0) or of the other half block through the transpose (use 1);
-// built from comb once per plane.  An operand is zero where its flags say so,
-// or where the receiving pair is self-paired (u = u*) and the term would be
-// counted twice.
-__device__ void build_sv(float4 *sv, const float2 *comb, const short4 *rowS, const short *rowF, const Layout &L,
-                         int TF, bool selfp0, bool selfp1) {
-  const int G = L.ngrp, NN2 = 2 * L.NN;
-  for (int idx = threadIdx.x; idx < TF * 4 * G * 4; idx += blockDim.x) {
-    const int j = idx & 3;
-    const int g = (idx >> 2) % G;
-    const int su = ((idx >> 2) / G) & 3;          // side * 2 + use
-    const int tf = (idx >> 2) / (4 * G);
-    const int side = su >> 1, use = su & 1;
-    const short4 si = rowS[use * G + g];
-    const int fl = rowF[use * G + g];
-    const int ci = (j == 0) ? si.x : (j == 1) ? si.y : (j == 2) ? si.z : si.w;
-    const bool conj = (fl >> j) & 1;
-    const bool zero = ((fl >> (8 + j)) & 1) || ((side ? selfp1 : selfp0) && ((fl >> (4 + j)) & 1));
-    const float2 sc = zero ? make_float2(0.f, 0.f) : comb[(tf * 2 + side) * NN2 + ci];
-    sv[idx] = conj ? make_float4(sc.x, -sc.x, sc.y, -sc.y) : make_float4(sc.x, sc.x, sc.y, sc.y);
-  }
-}
-
-// Split accumulators of one thread: U (frequency u) and V (u*) for the four
-// virtual slots of its orbit and each frame, as P / Q lane pairs.
-template <int TF> struct MacAcc {
-  f2x UP[TF][4], UQ[TF][4], VP[TF][4], VQ[TF][4];
-  __device__ __forceinline__ void zero() {
-#pragma unroll
-    for (int tf = 0; tf < TF; tf++)
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        UP[tf][k] = make_float2(0.f, 0.f); UQ[tf][k] = make_float2(0.f, 0.f);
-        VP[tf][k] = make_float2(0.f, 0.f); VQ[tf][k] = make_float2(0.f, 0.f);
-      }
-  }
-};
-__device__ __forceinline__ float2 pq_value(f2x P, f2x Q) { return make_float2(P.x - Q.y, P.y + Q.x); }
-
-// One generic stored row t (input channel i at u): feeds channel i at u,
-// Mxy i at u, My i at u*, Mx i at u*.
-// SW: the thread's virtual slots are those of a transposed orbit, [r, Mx r,
-// My r, Mxy r], so the My and Mx slot permutations trade places.
-template <int TF, bool SW>
-__device__ __forceinline__ void mac_generic_row(const float2 (&t)[4], const float4 *svr, int svstride,
-                                                MacAcc<TF> &a) {
-#pragma unroll
-  for (int tf = 0; tf < TF; tf++) {
-    const float4 q0 = svr[tf * svstride + 0], q1 = svr[tf * svstride + 1];
-    const float4 q2 = svr[tf * svstride + 2], q3 = svr[tf * svstride + 3];
-    const f2x A0 = pk(q0.x, q0.y), B0 = pk(q0.z, q0.w), A1 = pk(q1.x, q1.y), B1 = pk(q1.z, q1.w);
-    const f2x A2 = pk(q2.x, q2.y), B2 = pk(q2.z, q2.w), A3 = pk(q3.x, q3.y), B3 = pk(q3.z, q3.w);
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      ffma2(a.UP[tf][k], t[k], A0);
-      ffma2(a.UQ[tf][k], t[k], B0);
-      ffma2(a.UP[tf][k], t[sxy(k)], A1);
-      ffma2(a.UQ[tf][k], t[sxy(k)], B1);
-      ffma2(a.VP[tf][SW ? sx(k) : sy(k)], t[k], A2);
-      ffma2(a.VQ[tf][SW ? sx(k) : sy(k)], t[k], B2);
-      ffma2(a.VP[tf][SW ? sy(k) : sx(k)], t[k], A3);
-      ffma2(a.VQ[tf][SW ? sy(k) : sx(k)], t[k], B3);
-    }
-  }
-}
-
-// A centre-cross row pair (t at u, s at u*) of representative kind rk.
-template <int TF, bool SW>
-__device__ __forceinline__ void mac_pair_rows(const float2 (&t)[4], const float2 (&s)[4], int rk,
-                                              const float4 *svr, int svstride, MacAcc<TF> &a) {
-#pragma unroll
-  for (int tf = 0; tf < TF; tf++) {
-    const float4 q0 = svr[tf * svstride + 0], q1 = svr[tf * svstride + 1];
-    const f2x A0 = pk(q0.x, q0.y), B0 = pk(q0.z, q0.w), A1 = pk(q1.x, q1.y), B1 = pk(q1.z, q1.w);
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      ffma2(a.UP[tf][k], t[k], A0);
-      ffma2(a.UQ[tf][k], t[k], B0);
-      ffma2(a.VP[tf][k], s[k], A1);
-      ffma2(a.VQ[tf][k], s[k], B1);
-    }
-    if (rk != 3) {
-      const float4 q2 = svr[tf * svstride + 2], q3 = svr[tf * svstride + 3];
-      const f2x A2 = pk(q2.x, q2.y), B2 = pk(q2.z, q2.w), A3 = pk(q3.x, q3.y), B3 = pk(q3.z, q3.w);
-      if ((rk == 1) != SW) {   // My partner (rk 1) or Mx partner (rk 2), in this thread's slot order
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          ffma2(a.VP[tf][sy(k)], t[k], A2);
-          ffma2(a.VQ[tf][sy(k)], t[k], B2);
-          ffma2(a.UP[tf][sy(k)], s[k], A3);
-          ffma2(a.UQ[tf][sy(k)], s[k], B3);
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          ffma2(a.VP[tf][sx(k)], t[k], A2);
-          ffma2(a.VQ[tf][sx(k)], t[k], B2);
-          ffma2(a.UP[tf][sx(k)], s[k], A3);
-          ffma2(a.UQ[tf][sx(k)], s[k], B3);
-        }
-      }
-    }
-  }
-}
+// slots.  A complex accumulator gains element * real operand in one of them.
+__device__ __forceinline__ void fma_cr(float2 &acc, float2 e, float s) { acc = __ffma2_rn(e, make_float2(s, s), acc); }
 
 // Asynchronous 8-byte global -> shared copy (completes at cp.async.wait_all).
 __device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
@@ -408,7 +260,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 // Stage the input spectra of plane slot `zs` at the four frequencies of the
 // quad into shared memory: comb[t][side][i] = S_i[u_side], comb[t][side][NN + i]
-// = S_i[u_side*], with u_0 = (uy, ux), u_1 = (ux, uy) (rows py, ps; column px).
+// = S_i[u_side*], with u_0 = (uy, ux), u_1 = (ux, uy).
 __device__ __forceinline__ void stage_comb(float2 *comb, const MacParams &p, int TF, int zs, int uy, int ux) {
   const int us = uy ? p.f - uy : 0, vs = ux ? p.f - ux : 0;
   const int NN = p.L.NN, ffh = p.f * p.fh;
@@ -430,69 +282,154 @@ __device__ __forceinline__ void stage_comb(float2 *comb, const MacParams &p, int
   cp_async_commit();
 }
 
-// Shared memory of k_mac: ring | sv | scratch (comb staging, later the
-// share and side reduction) | rowS | rowF | mbarriers.
-__host__ __device__ inline size_t mac_scratch_elems(const Layout &L, int TF, int split, bool fwd) {
-  const size_t comb = (size_t)(fwd ? 2 : 1) * TF * 2 * 2 * L.NN;                    // float2
-  const size_t red = (size_t)(2 * split - 1) * ((L.nthr + 31) / 32 * 32) * 8 * TF;   // f2x = 8 B
-  return comb > red ? comb : red;
+// Operand table of one plane, built from comb:
+//   sv[t][half block][row][side][u / u*] = (p0, p1, m0, m1),
+// the real factors with which the row (C, D of every channel pair) enters the
+// accumulators of the receiving side,  P += C p0 + D p1,  M += C m0 + D m1.
+// With sa the spectrum that multiplies the row's channel directly and sb the
+// one that meets it through the Mxy mirror, w = sa + conj sb, v = sa - conj sb:
+// (p0, p1, m0, m1) = (Re w, Im w, Im v, -Re v).  rowS names sa and sb per use
+// (0: the half block's own side, 1: the other side, through the transpose);
+// a second row (kRowSecond) counts nothing where the receiving frequency pair
+// is self-paired (u = u*), since its first row says the same.
+template <int TF>
+__device__ void build_sv(float4 *sv, const float2 *comb, const short4 *rowS, const Layout &L, int nhalf, bool selfp0,
+                         bool selfp1) {
+  const int R = L.nrow, NN2 = 2 * L.NN;
+  const int per = R * 4;                               // entries of one half block
+  for (int idx = threadIdx.x; idx < TF * nhalf * per; idx += blockDim.x) {
+    const int uv = idx & 1, side = (idx >> 1) & 1;
+    const int tb = idx / per;                          // t * nhalf + half block
+    const int row = (idx - tb * per) >> 2;
+    const int t = tb / nhalf, bs = tb - t * nhalf;
+    const int use = side != bs;
+    if (use && row >= L.nrowT) continue;               // never read
+    const short4 si = rowS[use * R + row];
+    const int ia = uv ? si.z : si.x, ib = uv ? si.w : si.y;
+    const float2 *cb = comb + (t * 2 + side) * NN2 + uv * L.NN;
+    const bool zero = (rowS[2 * R + row].x & kRowSecond) && (side ? selfp1 : selfp0);
+    const float2 sa = ia >= 0 && !zero ? cb[ia] : make_float2(0.f, 0.f);
+    const float2 sb = ib >= 0 && !zero ? cb[ib] : make_float2(0.f, 0.f);
+    sv[((t * 2 + bs) * R + row) * 4 + side * 2 + uv] =
+        make_float4(sa.x + sb.x, sa.y - sb.y, sa.y + sb.y, sb.x - sa.x);
+  }
 }
 
-size_t mac_smem_bytes(const Layout &L, int TF, int stages, int chunk_rows, int split, bool fwd) {
-  return sizeof(float2) * ((size_t)stages * chunk_rows * L.RS + mac_scratch_elems(L, TF, split, fwd)) +
-         sizeof(float4) * (size_t)TF * 4 * L.ngrp * 4 + sizeof(short4) * 2 * L.ngrp + sizeof(short) * 2 * L.ngrp +
+// Shared memory of k_mac: ring | sv | scratch (comb staging, later the output
+// exchange) | rowS | mbarriers.
+__host__ __device__ inline size_t mac_scratch_elems(const Layout &L, int TF, bool fwd) {
+  return (size_t)(fwd ? 2 : 1) * TF * 2 * 2 * L.NN;                    // float2
+}
+__host__ __device__ inline size_t mac_scratch_pad(size_t e) { return (e + 1) & ~(size_t)1; }   // 16-byte multiple
+
+size_t mac_smem_bytes(const Layout &L, int TF, int stages, int chunk_rows, bool fwd) {
+  return sizeof(float2) * ((size_t)stages * chunk_rows * L.RS + mac_scratch_pad(mac_scratch_elems(L, TF, fwd))) +
+         sizeof(float4) * (size_t)TF * 2 * L.nrow * 4 + sizeof(short4) * 3 * L.nrow +
          2 * sizeof(unsigned long long) * stages + 16;
 }
 
-// Launch bounds: blocks of at most 128 threads (orbit groups of Nnum <= 15
-// with a row split of 2) or of at most 256, and the CTAs per SM the register
-// budget is sized for.
-template <int TF, bool WIDE> struct MacOcc {
-  static constexpr int threads = WIDE ? 256 : 128;
-  static constexpr int v = WIDE ? (TF == 1 ? 2 : 1) : (TF == 1 ? 4 : (TF == 2 ? 3 : 2));
+// Accumulators of one thread: per side, frame and channel pair the P and M sums at u and u*.
+template <int TF, int PPT> struct MacAcc {
+  float2 UP[2][TF][PPT], UM[2][TF][PPT], VP[2][TF][PPT], VM[2][TF][PPT];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int s = 0; s < 2; s++)
+#pragma unroll
+      for (int t = 0; t < TF; t++)
+#pragma unroll
+        for (int k = 0; k < PPT; k++)
+          UP[s][t][k] = UM[s][t][k] = VP[s][t][k] = VM[s][t][k] = make_float2(0.f, 0.f);
+  }
+};
+
+// One stored row into the accumulators of the sides S0 .. S1 - 1.
+template <int TF, int PPT, int S0, int S1>
+__device__ __forceinline__ void mac_row(const float4 *row, const int (&off)[PPT], const float4 *svr, int svt,
+                                        MacAcc<TF, PPT> &a) {
+  float2 C[PPT], D[PPT];
+#pragma unroll
+  for (int k = 0; k < PPT; k++) {
+    const float4 e = row[off[k]];
+    C[k] = make_float2(e.x, e.y);
+    D[k] = make_float2(e.z, e.w);
+  }
+#pragma unroll
+  for (int t = 0; t < TF; t++)
+#pragma unroll
+    for (int s = S0; s < S1; s++) {
+      const float4 u = svr[t * svt + s * 2], v = svr[t * svt + s * 2 + 1];
+#pragma unroll
+      for (int k = 0; k < PPT; k++) {
+        fma_cr(a.UP[s][t][k], C[k], u.x);
+        fma_cr(a.UM[s][t][k], C[k], u.z);
+        fma_cr(a.VP[s][t][k], C[k], v.x);
+        fma_cr(a.VM[s][t][k], C[k], v.z);
+      }
+#pragma unroll
+      for (int k = 0; k < PPT; k++) {
+        fma_cr(a.UP[s][t][k], D[k], u.y);
+        fma_cr(a.UM[s][t][k], D[k], u.w);
+        fma_cr(a.VP[s][t][k], D[k], v.y);
+        fma_cr(a.VM[s][t][k], D[k], v.w);
+      }
+    }
+}
+
+// Threads: `cw` warps side by side cover the channel pairs (PPT per lane), `H`
+// row shares of such warps take alternate rows of a chunk.
+template <int TF, int TH> struct MacOcc {
+  static constexpr int v = TH == 128 ? (TF == 1 ? 4 : (TF == 2 ? 3 : 2)) : (TF == 1 ? 2 : 1);
 };
 
 // One CTA = one frequency quad {(uy, ux), (ux, uy)} and a group of planes.
-// The threads form two sides, one per frequency pair of the quad; thread
-// (side, h, o) owns the mirror orbit o of output channels at its pair's
-// frequencies u and u* for the rows of its share h (rows are dealt round-robin
-// to the `split` threads of an orbit).  Every stored row of the quad's half
-// blocks streams through shared memory once and feeds both sides: the side it
-// belongs to through the thread's own orbit slots, and (for transposable
-// groups) the other side through the slots of the transposed orbit, since
-// T_{Tr i, Tr j}[(uy, ux)] = T_ij[(ux, uy)].  Shares (and, for a diagonal quad,
-// whose two sides are the same pair, the sides) are added through shared
-// memory when a plane's output is due, so there is no atomic and every output
-// is written by exactly one thread.
+// Every stored row of the quad's half blocks streams through shared memory
+// once and feeds both sides (frequency pairs) of the quad: its own side, and,
+// for the transposable rows (stored first), the other side through the
+// transpose T_{Tr i, Tr j}[(uy, ux)] = T_ij[(ux, uy)].  A lane owns PPT pairs
+// of output channels (j, Mxy j) on both sides: the pair (j, Mxy j) at u and the
+// pair (My j, Mx j) at u*, with Tr j for j on side 1.  The row shares' sums,
+// the two sides of a diagonal quad (one frequency pair) and the two sums of a
+// self-paired frequency are added through shared memory when a plane's output
+// is due, in a fixed order, so there is no atomic and every output has one
+// writer.
+//
+// What bounds it.  Real operands against C and D halve the multiplications of
+// the complex form (a stored complex number feeds 8 two-lane FMAs per frame, 16
+// before), which leaves the stream of the matrices as the bound at one frame:
+// per 1808-byte row (Nnum 15) an SM takes 77 cycles at the measured copy rate,
+// against 32 of FMA issue and 46 of shared memory (PPT = 2: two column warps
+// read the row once and 64 B of operands each; one pair per lane would read the
+// operands four times, four pairs would keep 64 accumulators a lane).  Measured
+// against the complex form (GB300, Nnum 15): back projection of 1005 x 1005 px,
+// 41 planes, one frame 2776 -> 1891 us (3.7 -> 5.4 TB/s), forward 3006 -> 2152 us;
+// three frames of 437 x 608 px, 31 planes, back 3202 -> 1242 us (the complex form
+// also ran three frames as four).
 // The stored rows stream through a ring of shared-memory stages filled by
 // bulk copies (crossing plane boundaries).  Forward projection accumulates the
 // planes of the group (the group sums are added by the inverse transform);
 // back projection writes each plane's spectra when the plane is done.  The
 // spectra of the next plane are staged with cp.async while the current plane
 // streams.
-template <int TF, bool FWD, bool WIDE>
-__global__ void __launch_bounds__(MacOcc<TF, WIDE>::threads, MacOcc<TF, WIDE>::v) k_mac(MacParams p) {
+template <int TF, bool FWD, int PPT, int TH>
+__global__ void __launch_bounds__(TH, MacOcc<TF, TH>::v) k_mac(MacParams p) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ int s_abort;
   __shared__ int s_issued;                      // chunks handed to the bulk-copy engine
   __shared__ int s_plane[kMacMaxZgroup];        // plane slots of this CTA's z range
   volatile int *abortf = &s_abort;
   const Layout &L = p.L;
-  const int NN = L.NN, NT = L.nthr, RS = L.RS, NN2 = 2 * L.NN, G = L.ngrp, c = L.c;
-  const int CH = p.chunk_rows, NST = p.stages, H = p.split;
-  const int NTP = (NT + 31) / 32 * 32;
-  float2 *ring = reinterpret_cast<float2 *>(smraw);                          // [NST][CH*RS]
-  float4 *sv = reinterpret_cast<float4 *>(ring + (size_t)NST * CH * RS);     // [TF][2][2][G][4]
-  float2 *scratch = reinterpret_cast<float2 *>(sv + TF * 4 * G * 4);        // comb [1|2][TF][2][2NN] / red
-  f2x *red = reinterpret_cast<f2x *>(scratch);                              // [2H-1][NTP][TF][8]
-  short4 *rowS = reinterpret_cast<short4 *>(scratch + mac_scratch_elems(L, TF, H, FWD));
-  short *rowF = reinterpret_cast<short *>(rowS + 2 * G);
-  unsigned long long *full = reinterpret_cast<unsigned long long *>(
-      (reinterpret_cast<uintptr_t>(rowF + 2 * G) + 7) & ~(uintptr_t)7);
+  const int NN = L.NN, N = L.N, NP = L.NP, R = L.nrow, nT = L.nrowT, NN2 = 2 * L.NN;
+  const int CH = p.chunk_rows, NST = p.stages, H = p.shares;
+  float4 *ring = reinterpret_cast<float4 *>(smraw);                          // [NST][CH][NP]
+  float4 *sv = ring + (size_t)NST * CH * NP;                                 // [TF][2][R][2][2]
+  float2 *scratch = reinterpret_cast<float2 *>(sv + TF * 2 * R * 4);         // comb [1|2][TF][2][2NN] / outs
+  float2 *outs = scratch;                                                    // [TF][side][u | u*][NN]
+  short4 *rowS = reinterpret_cast<short4 *>(scratch + mac_scratch_pad(mac_scratch_elems(L, TF, FWD)));
+  unsigned long long *full = reinterpret_cast<unsigned long long *>(rowS + 3 * R);
   int *released = reinterpret_cast<int *>(full + NST);   // [NST] warps done with each slot, ever
 
-  const int tid = threadIdx.x;
-  const int nwarps = (blockDim.x + 31) >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nwarps = blockDim.x >> 5;
   if (tid == 0) {
     for (int i = 0; i < NST; i++) {
       mbar_init(full + i, 1);
@@ -502,10 +439,7 @@ __global__ void __launch_bounds__(MacOcc<TF, WIDE>::threads, MacOcc<TF, WIDE>::v
     s_issued = 0;
     fence_mbar_init();
   }
-  for (int i = tid; i < 2 * G; i += blockDim.x) {
-    rowS[i] = p.rowS[i];
-    rowF[i] = p.rowF[i];
-  }
+  for (int i = tid; i < 3 * R; i += blockDim.x) rowS[i] = p.rowS[i];
   {
     const int zb = blockIdx.y * p.zgroup, nzl = min(p.zgroup, p.nz - zb);
     for (int i = tid; i < nzl; i += blockDim.x) s_plane[i] = p.planes[zb + i];
@@ -522,36 +456,29 @@ __global__ void __launch_bounds__(MacOcc<TF, WIDE>::threads, MacOcc<TF, WIDE>::v
   const int nhalf = diag ? 1 : 2;
   const bool selfp0 = (uy == 0) || (2 * uy == p.f), selfp1 = (ux == 0) || (2 * ux == p.f);
   const int ffh = p.f * p.fh;
-  const int HS = H * NTP;                        // threads per side
-  const int ts = tid / HS;                       // side of this thread
-  const int h = (tid - ts * HS) / NTP, o = tid - ts * HS - h * NTP;
-  const bool active = o < NT;
-  const int kind = (o < c * c) ? 0 : ((o < c * c + c) ? 1 : ((o < c * c + 2 * c) ? 2 : 3));
-  // virtual slots of orbit o: every half block is read at these (side 1 owns
-  // the transposed orbit, its half block is stored in transposed column order)
-  int off[4];
-  {
-    const short4 a = p.oslots[active ? o : 0];
-    off[0] = a.x; off[1] = a.y; off[2] = a.z; off[3] = a.w;
-  }
-  const int ns = (kind == 0) ? 4 : ((kind == 3) ? 1 : 2);
+  const int cw = nwarps / H;                     // column warps
+  const int h = warp / cw;                       // row share
+  const int p0 = (warp - h * cw) * 32 * PPT + lane;
+  int off[PPT];                                  // this lane's channel pairs (repeating the last one past the end)
+#pragma unroll
+  for (int k = 0; k < PPT; k++) off[k] = min(p0 + 32 * k, NP - 1);
   const int z0 = blockIdx.y * p.zgroup;
   const int z1 = min(z0 + p.zgroup, p.nz);
-  const int nrq = nhalf * L.nrow;                // stored rows of the quad per plane
+  const int nrq = nhalf * R;                     // stored rows of the quad per plane
   const int cpb = (nrq + CH - 1) / CH;           // chunks per (quad, plane)
   const int total = (z1 - z0) * cpb;
-  const size_t halfElems = (size_t)L.nrow * RS;
+  const size_t halfElems = (size_t)R * NP;       // float4
   const int combStride = TF * 2 * NN2;           // one plane's staged spectra (float2)
-  const int svs = 4 * G * 4;                     // sv stride between frames (float4)
+  const int svt = 2 * R * 4;                     // sv stride between frames (float4)
 
-  MacAcc<TF> acc;
+  MacAcc<TF, PPT> acc;
   acc.zero();
 
   stage_comb(scratch, p, TF, FWD ? z0 : 0, uy, ux);
   cp_async_wait_all();
   __syncthreads();   // barriers initialised, row tables and first spectra staged
-  build_sv(sv, scratch, rowS, rowF, L, TF, selfp0, selfp1);
-  __syncthreads();   // (back projection: the staging area is free for the reduction)
+  build_sv<TF>(sv, scratch, rowS, L, nhalf, selfp0, selfp1);
+  __syncthreads();   // (back projection: the staging area is free for the output exchange)
 
   // Chunk g goes to ring slot g % NST.  Thread 0 fills the whole ring; after
   // that, the warp that releases a slot last (each warp counts itself out
@@ -565,10 +492,10 @@ __global__ void __launch_bounds__(MacOcc<TF, WIDE>::threads, MacOcc<TF, WIDE>::v
     const int zl_n = gn / cpb, ch_n = gn - zl_n * cpb, sl = gn % NST;
     const int r0 = ch_n * CH;
     const int nr = min(CH, nrq - r0);
-    const float2 *src = p.P + ((long long)s_plane[zl_n] * p.nkp + hb0) * (long long)halfElems + (long long)r0 * RS;
-    const unsigned bytes = (unsigned)(nr * RS * sizeof(float2));
+    const float4 *src = p.P + ((long long)s_plane[zl_n] * p.nkp + hb0) * (long long)halfElems + (long long)r0 * NP;
+    const unsigned bytes = (unsigned)(nr * NP * sizeof(float4));
     mbar_arrive_expect_tx(full + sl, bytes);
-    bulk_g2s(ring + (size_t)sl * CH * RS, src, bytes, full + sl);
+    bulk_g2s(ring + (size_t)sl * CH * NP, src, bytes, full + sl);
   };
   if (tid == 0) {
     const int pre = min(NST, total);
@@ -585,7 +512,7 @@ __global__ void __launch_bounds__(MacOcc<TF, WIDE>::threads, MacOcc<TF, WIDE>::v
       if (zl > 0) {
         cp_async_wait_all();
         __syncthreads();   // spectra of plane zi staged; all threads done with plane zi-1
-        build_sv(sv, scratch + (zl & 1) * combStride, rowS, rowF, L, TF, selfp0, selfp1);
+        build_sv<TF>(sv, scratch + (zl & 1) * combStride, rowS, L, nhalf, selfp0, selfp1);
         __syncthreads();
       }
       if (zi + 1 < z1) stage_comb(scratch + ((zl + 1) & 1) * combStride, p, TF, zi + 1, uy, ux);
@@ -596,54 +523,29 @@ __global__ void __launch_bounds__(MacOcc<TF, WIDE>::threads, MacOcc<TF, WIDE>::v
       *abortf = 1;
       atomicExch(p.err, 2);
     }
-    if (!dead && active) {
+    if (!dead) {
       const int r0 = ch * CH;
       const int r1 = min(nrq, r0 + CH);
-      const float2 *stage = ring + (size_t)slot * CH * RS;
-      // the chunk's rows, one half block at a time
-      for (int bs = r0 / L.nrow; bs * L.nrow < r1; bs++) {
-        const int base = bs * L.nrow;
-        const int lo = max(r0, base) - base, hi = min(r1, base + L.nrow) - base;   // half-block rows
-        const int use = (bs == ts) ? 0 : 1;       // warp-uniform: a side is whole warps
-        const float4 *svb = sv + (ts * 2 + use) * G * 4;
-        const float2 *srow = stage + (base - r0) * RS;
-        // generic rows (through the transpose only the first nrowGT), then row pairs
-        const int rg = min(hi, use ? L.nrowGT : L.nrowG);
-        const int pr1 = min(hi, use ? L.nrowG + 2 * c : L.nrow);
-        const int pr0 = max(lo, L.nrowG);
-        if (ts == 0) {
+      const float4 *stage = ring + (size_t)slot * CH * NP;
+      // the chunk's rows, one half block at a time: the transposable ones feed
+      // both sides, the others the half block's own
+      for (int bs = r0 >= R ? 1 : 0; bs * R < r1; bs++) {
+        const int base = bs * R;
+        const int lo = max(r0, base) - base, hi = min(r1, base + R) - base;   // half-block rows
+        const float4 *svb = sv + (size_t)bs * R * 4;
+        const float4 *srow = stage + (base - r0) * NP;
+        const int rb = min(hi, nT);
 #pragma unroll 2
-          for (int r = lo + h; r < rg; r += H) {
-            float2 t[4];
-            load_slots(srow + (size_t)r * RS, off, t);
-            mac_generic_row<TF, false>(t, svb + r * 4, svs, acc);
-          }
-          for (int r = pr0 + 2 * h; r < pr1; r += 2 * H) {
-            const int k2 = (r - L.nrowG) >> 1;
-            float2 t[4], s2[4];
-            load_slots(srow + (size_t)r * RS, off, t);
-            load_slots(srow + (size_t)(r + 1) * RS, off, s2);
-            mac_pair_rows<TF, false>(t, s2, use ? 2 : ((k2 < c) ? 1 : 3), svb + (L.nrowG + k2) * 4, svs, acc);
-          }
+        for (int r = lo + h; r < rb; r += H) mac_row<TF, PPT, 0, 2>(srow + r * NP, off, svb + r * 4, svt, acc);
+        if (bs == 0) {
+          for (int r = max(lo, nT) + h; r < hi; r += H) mac_row<TF, PPT, 0, 1>(srow + r * NP, off, svb + r * 4, svt, acc);
         } else {
-#pragma unroll 2
-          for (int r = lo + h; r < rg; r += H) {
-            float2 t[4];
-            load_slots(srow + (size_t)r * RS, off, t);
-            mac_generic_row<TF, true>(t, svb + r * 4, svs, acc);
-          }
-          for (int r = pr0 + 2 * h; r < pr1; r += 2 * H) {
-            const int k2 = (r - L.nrowG) >> 1;
-            float2 t[4], s2[4];
-            load_slots(srow + (size_t)r * RS, off, t);
-            load_slots(srow + (size_t)(r + 1) * RS, off, s2);
-            mac_pair_rows<TF, true>(t, s2, use ? 2 : ((k2 < c) ? 1 : 3), svb + (L.nrowG + k2) * 4, svs, acc);
-          }
+          for (int r = max(lo, nT) + h; r < hi; r += H) mac_row<TF, PPT, 1, 2>(srow + r * NP, off, svb + r * 4, svt, acc);
         }
       }
     }
     __syncwarp();
-    if ((tid & 31) == 0 && !dead) {
+    if (lane == 0 && !dead) {
       __threadfence_block();                       // this warp's reads of the slot come first
       const int before = atomicAdd(released + slot, 1);
       if (before == round * nwarps + nwarps - 1 && g + NST < total && !*abortf) {
@@ -656,92 +558,71 @@ __global__ void __launch_bounds__(MacOcc<TF, WIDE>::threads, MacOcc<TF, WIDE>::v
 
     const bool out_due = (ch == cpb - 1) && (!FWD || zi + 1 == z1);
     if (out_due) {
-      f2x U[TF][4], V[TF][4];
-#pragma unroll
-      for (int tf = 0; tf < TF; tf++)
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          U[tf][k] = pq_value(acc.UP[tf][k], acc.UQ[tf][k]);
-          V[tf][k] = pq_value(acc.VP[tf][k], acc.VQ[tf][k]);
-        }
-      // writers: share 0 of each side, or of side 0 only for a diagonal quad
-      // (its two sides are the same frequency pair); the others add into them
-      const bool writer = (h == 0) && (!diag || ts == 0);
-      if (H > 1 || diag) {
-        if (FWD) cp_async_wait_all();   // the staging area doubles as reduction buffer
+      // the row shares add their channel values into outs in share order
+      if (FWD) {
+        cp_async_wait_all();   // the staging area doubles as the exchange buffer
         __syncthreads();
-        if (!writer && active) {
-          const int idx = diag ? ts * H + h - 1 : ts * (H - 1) + h - 1;
-          // in a diagonal quad, side 1's orbit is the transposed orbit T(o) of side 0,
-          // with its My and Mx slots swapped
-          int ot = o;
-          if (diag && ts) {
-            const int c2 = c * c;
-            ot = (o < c2) ? (o % c) * c + o / c : ((o < c2 + c) ? o + c : ((o < c2 + 2 * c) ? o - c : o));
-          }
-          f2x *rp = red + ((size_t)idx * NTP + ot) * TF * 8;
-#pragma unroll
-          for (int tf = 0; tf < TF; tf++)
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-              const int kk = (diag && ts) ? ((k == 1) ? 2 : ((k == 2) ? 1 : k)) : k;
-              rp[tf * 8 + kk] = U[tf][k];
-              rp[tf * 8 + 4 + kk] = V[tf][k];
-            }
-        }
-        __syncthreads();
-        if (writer && active) {
-          const int n0 = diag ? 0 : ts * (H - 1), n1 = diag ? 2 * H - 1 : n0 + H - 1;
-          for (int idx = n0; idx < n1; idx++) {
-            const f2x *rp = red + ((size_t)idx * NTP + o) * TF * 8;
-#pragma unroll
-            for (int tf = 0; tf < TF; tf++)
-#pragma unroll
-              for (int k = 0; k < 4; k++) {
-                const float2 a = unpk(U[tf][k]), b = unpk(rp[tf * 8 + k]);
-                const float2 cc2 = unpk(V[tf][k]), d = unpk(rp[tf * 8 + 4 + k]);
-                U[tf][k] = pk(a.x + b.x, a.y + b.y);
-                V[tf][k] = pk(cc2.x + d.x, cc2.y + d.y);
-              }
-          }
-        }
       }
-      if (writer && active && !dead) {
-        const int oy = ts ? ux : uy, ox = ts ? uy : ux;
-        const int osy = oy ? p.f - oy : 0;
-        const bool sp = ts ? selfp1 : selfp0;
+      for (int hh = 0; hh < H; hh++) {
+        if (h == hh) {
 #pragma unroll
-        for (int tf = 0; tf < TF; tf++) {
-          if (tf >= p.T) break;
-          const long long obase = FWD ? ((long long)(blockIdx.y * p.T + tf) * NN) * ffh
-                                      : ((long long)(tf * p.nzo + zi) * NN) * ffh;
+          for (int k = 0; k < PPT; k++) {
+            const int pr = p0 + 32 * k;
+            if (pr < NP) {
+              const int b = pr / N, a = pr - b * N;             // channel j = pr of side 0
+              const int my = (N - 1 - b) * N + a, tr = a * N + b, mytr = (N - 1 - a) * N + b;
 #pragma unroll
-          for (int k = 0; k < 4; k++) {
-            const int vk = (kind == 2) ? ((k & 1) ? 2 : 0) : k;   // stored slot k -> virtual slot
-            if (k < ns) {
-              int sl = off[0];
+              for (int s = 0; s < 2; s++) {
+                const int j = s ? tr : pr, m = s ? mytr : my;    // first channels of the pair at u and at u*
 #pragma unroll
-              for (int m = 1; m < 4; m++)
-                if (m == vk) sl = off[m];
-              int q = p.slotcol[sl];
-              if (ts) q = (q % L.N) * L.N + q / L.N;   // side 1: the transposed channel
-              float2 *op = p.O + obase + (long long)q * ffh;
-              float2 u = unpk(U[tf][0]), v = unpk(V[tf][0]);
-#pragma unroll
-              for (int m = 1; m < 4; m++)
-                if (m == vk) { u = unpk(U[tf][m]); v = unpk(V[tf][m]); }
-              if (sp) {
-                op[oy * p.fh + ox] = make_float2(u.x + v.x, u.y + v.y);
-              } else {
-                op[oy * p.fh + ox] = u;
-                op[osy * p.fh + ox] = v;
+                for (int t = 0; t < TF; t++) {
+                  float2 *ou = outs + (size_t)(t * 2 + s) * NN2, *ov = ou + NN;
+                  // first + conj(second) = 2 P, first - conj(second) = 2 i M (the halves are in C and D)
+                  auto put = [&](float2 *o, int c1, float2 P, float2 M) {
+                    float2 x = make_float2(P.x - M.y, P.y + M.x), y = make_float2(P.x + M.y, M.x - P.y);
+                    const int c2 = NN - 1 - c1;                  // equal for the centre, then x = y
+                    if (hh > 0) {
+                      const float2 ox = o[c1], oy = o[c2];
+                      x.x += ox.x; x.y += ox.y; y.x += oy.x; y.y += oy.y;
+                    }
+                    o[c1] = x;
+                    o[c2] = y;
+                  };
+                  put(ou, j, acc.UP[s][t][k], acc.UM[s][t][k]);
+                  put(ov, m, acc.VP[s][t][k], acc.VM[s][t][k]);
+                }
               }
             }
+          }
+        }
+        __syncthreads();
+      }
+      if (!dead) {
+        const int nside = diag ? 1 : 2;
+        const int nt = min(TF, p.T);
+        for (int idx = tid; idx < nt * nside * NN; idx += blockDim.x) {
+          const int q = idx % NN, ts = idx / NN;
+          const int t = ts / nside, s = ts - t * nside;
+          const float2 *o = outs + (size_t)(t * 2 + s) * NN2 + q;
+          float2 u = o[0], v = o[NN];
+          if (diag) {                                // the other side is the same frequency pair
+            const float2 u1 = o[NN2], v1 = o[NN2 + NN];
+            u.x += u1.x; u.y += u1.y; v.x += v1.x; v.y += v1.y;
+          }
+          const int oy = s ? ux : uy, ox = s ? uy : ux;
+          const long long obase = FWD ? ((long long)(blockIdx.y * p.T + t) * NN) * ffh
+                                      : ((long long)(t * p.nzo + zi) * NN) * ffh;
+          float2 *op = p.O + obase + (long long)q * ffh + ox;
+          if (s ? selfp1 : selfp0) {
+            op[oy * p.fh] = make_float2(u.x + v.x, u.y + v.y);
+          } else {
+            op[oy * p.fh] = u;
+            op[(p.f - oy) * p.fh] = v;
           }
         }
       }
       acc.zero();
-      if (H > 1 || diag) __syncthreads();   // the reduction buffer is free again
+      if (g + 1 < total) __syncthreads();   // the exchange buffer is free again
     }
     if (++ch == cpb) { ch = 0; zl++; }
     if (++slot == NST) { slot = 0; round++; }
@@ -793,18 +674,25 @@ __global__ void k_build_k(BuildKParams p) {
 }
 
 // Packed matrices of a chunk of representatives: the value of frequency pair
-// (py, px) goes to its half block (quad (py, px) side 0 when py <= px, quad
-// (px, py) side 1 otherwise); a row pair also stores the row at (f - py, px).
+// (fy, fx) goes to its half block (quad (fy, fx) side 0 when fy <= fx, quad
+// (fx, fy) side 1 otherwise) as C and D of every channel pair (see Layout); a
+// row pair also stores the row at (f - fy, fx), with its columns mirrored.
 template <typename R>
 __global__ void k_pack(PackParams p) {
   typedef typename CT<R>::T C;
   const Layout &L = p.L;
-  const int NN = L.NN, ffh = p.f * p.fh;
-  const long long total = (long long)p.nrep_chunk * NN * p.nkp;
+  const int N = L.N, NN = L.NN, NP = L.NP, ffh = p.f * p.fh;
+  const long long total = (long long)p.nrep_chunk * NP * p.nkp;
+  const R sc = (R)(0.5 * p.scale);
+  // C = (A + B) / 2, D = i (A - B) / 2 with A = first, B = conj second
+  auto cd = [&](C a, C s) {
+    return make_float4((float)((a.x + s.x) * sc), (float)((a.y - s.y) * sc), (float)(-(a.y + s.y) * sc),
+                       (float)((a.x - s.x) * sc));
+  };
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
-    const int q = (int)(idx % NN);
-    const long long r2 = idx / NN;
+    const int pr = (int)(idx % NP);
+    const long long r2 = idx / NP;
     const int rl = (int)(r2 % p.nrep_chunk);
     const int kp = (int)(r2 / p.nrep_chunk);
     const int fy = kp / p.fq, fx = kp % p.fq;       // frequency pair (fy, fx)
@@ -812,18 +700,19 @@ __global__ void k_pack(PackParams p) {
     const int hb = 2 * (hi * (hi + 1) / 2 + lo) - hi + (fy > fx ? 1 : 0);
     const int fs = fy ? p.f - fy : 0;
     const int rep = p.rep0 + rl;
-    const int kind = p.rep_kind[rep];
     const int row = p.rep_row[rep];
-    const C *sp = reinterpret_cast<const C *>(p.spec) + ((long long)rl * NN + q) * ffh;
-    // the second half block of a quad holds channel Tr q at the slot of q
-    const int slot = p.col_slot[fy > fx ? (q % L.N) * L.N + q / L.N : q];
-    float2 *dst = p.P + ((long long)hb * L.nrow + row) * L.RS + slot;
-    const R sc = (R)p.scale;
-    const C a = sp[fy * p.fh + fx];
-    dst[0] = make_float2((float)(a.x * sc), (float)(a.y * sc));
-    if (kind != 0) {
-      const C b = sp[fs * p.fh + fx];
-      dst[L.RS] = make_float2((float)(b.x * sc), (float)(b.y * sc));
+    const C *sp = reinterpret_cast<const C *>(p.spec) + (long long)rl * NN * ffh;
+    // the second half block of a quad holds channel Tr j at the place of j
+    const int b = pr / N, a = pr - b * N;
+    const int jb = fy > fx ? a : b, ja = fy > fx ? b : a;
+    const int j = jb * N + ja;
+    float4 *dst = p.P + ((long long)hb * L.nrow + row) * NP + pr;
+    const long long o = fy * p.fh + fx;
+    dst[0] = cd(sp[(long long)j * ffh + o], sp[(long long)(NN - 1 - j) * ffh + o]);
+    if (p.rep_kind[rep] != 0) {
+      const int my = (N - 1 - jb) * N + ja;
+      const long long os = fs * p.fh + fx;
+      dst[NP] = cd(sp[(long long)my * ffh + os], sp[(long long)(NN - 1 - my) * ffh + os]);
     }
   }
 }
@@ -1030,29 +919,37 @@ cudaError_t launch_irfft2(const Irfft2Params &p, cudaStream_t s) {
 
 int mac_max_frames() { return 4; }
 
-template <int TF>
-static cudaError_t launch_mac_tf(const MacParams &p, bool fwd, cudaStream_t s) {
-  const size_t sm = mac_smem_bytes(p.L, TF, p.stages, p.chunk_rows, p.split, fwd);
-  dim3 grid(p.nquads, p.nzo_grid);
-  const int block = 2 * p.split * (((p.L.nthr + 31) / 32) * 32);
-  const void *fn = block <= 128 ? (fwd ? (const void *)k_mac<TF, true, false> : (const void *)k_mac<TF, false, false>)
-                                : (fwd ? (const void *)k_mac<TF, true, true> : (const void *)k_mac<TF, false, true>);
-  cudaError_t e = set_smem(fn, sm);
+// Warps side by side over the channel pairs, and row shares: about 128 threads
+// per unit of p.split, at most 256.  Two pairs per lane from 33 pairs on.
+MacThreads mac_threads(const Layout &L, int split) {
+  MacThreads t;
+  t.ppt = L.NP > 32 ? 2 : 1;
+  t.cw = (L.NP + 32 * t.ppt - 1) / (32 * t.ppt);
+  t.shares = std::max(1, std::min(4 * split / t.cw, 8 / t.cw));
+  return t;
+}
+
+template <int TF, bool FWD>
+static cudaError_t launch_mac_tf(const MacParams &p0, cudaStream_t s) {
+  MacParams p = p0;
+  const MacThreads th = mac_threads(p.L, p.split);
+  p.shares = th.shares;
+  const size_t sm = mac_smem_bytes(p.L, TF, p.stages, p.chunk_rows, FWD);
+  const dim3 grid(p.nquads, p.nzo_grid);
+  const int block = 32 * th.cw * th.shares;
+  void (*fn)(MacParams) = block <= 128 ? (th.ppt == 2 ? k_mac<TF, FWD, 2, 128> : k_mac<TF, FWD, 1, 128>)
+                                       : (th.ppt == 2 ? k_mac<TF, FWD, 2, 256> : k_mac<TF, FWD, 1, 256>);
+  cudaError_t e = set_smem((const void *)fn, sm);
   if (e != cudaSuccess) return e;
-  if (block <= 128) {
-    if (fwd) k_mac<TF, true, false><<<grid, block, sm, s>>>(p);
-    else k_mac<TF, false, false><<<grid, block, sm, s>>>(p);
-  } else {
-    if (fwd) k_mac<TF, true, true><<<grid, block, sm, s>>>(p);
-    else k_mac<TF, false, true><<<grid, block, sm, s>>>(p);
-  }
+  fn<<<grid, block, sm, s>>>(p);
   return cudaGetLastError();
 }
 
 cudaError_t launch_mac(const MacParams &p, bool forward, cudaStream_t s) {
-  if (p.T <= 1) return launch_mac_tf<1>(p, forward, s);
-  if (p.T <= 2) return launch_mac_tf<2>(p, forward, s);
-  return launch_mac_tf<4>(p, forward, s);
+  if (p.T <= 1) return forward ? launch_mac_tf<1, true>(p, s) : launch_mac_tf<1, false>(p, s);
+  if (p.T == 2) return forward ? launch_mac_tf<2, true>(p, s) : launch_mac_tf<2, false>(p, s);
+  if (p.T == 3) return forward ? launch_mac_tf<3, true>(p, s) : launch_mac_tf<3, false>(p, s);
+  return forward ? launch_mac_tf<4, true>(p, s) : launch_mac_tf<4, false>(p, s);
 }
 
 cudaError_t launch_build_k(const BuildKParams &p, int nimg, cudaStream_t s) {
@@ -1063,7 +960,7 @@ cudaError_t launch_build_k(const BuildKParams &p, int nimg, cudaStream_t s) {
 }
 
 cudaError_t launch_pack(const PackParams &p, cudaStream_t s) {
-  const long long total = (long long)p.nrep_chunk * p.L.NN * p.nkp;
+  const long long total = (long long)p.nrep_chunk * p.L.NP * p.nkp;
   if (total == 0) return cudaSuccess;
   long long blocks = (total + 255) / 256;
   if (blocks > 65535LL * 16) blocks = 65535LL * 16;
