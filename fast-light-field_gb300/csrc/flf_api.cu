@@ -82,7 +82,7 @@ struct flf_ctx {
   int num_sms = 0;
   int req_f = 0, req_fp64 = 0;   // transform size / precision asked for by flf_prepare
   int opt_stages = 2;            // tunable: MAC shared-memory pipeline stages
-  int opt_chunk_rows[2] = {12, 12};   // tunable: stored rows per pipeline stage (forward, backward)
+  int opt_chunk_rows[2] = {0, 0};   // tunable: stored rows per pipeline stage (forward, backward); 0: auto_chunk_rows
   int opt_split = 1;             // tunable: threads sharing one orbit's rows
   int opt_ctas_per_sm = 16;      // tunable: multiply-accumulate CTAs per SM the plane grouping aims at
   int opt_plane_sizes = 1;       // 1: transform size per plane (grouped); 0: one size for all
@@ -716,12 +716,34 @@ int join_streams(flf_ctx *ctx, cudaStream_t s) {
   return FLF_OK;
 }
 
-// Launch shape of the multiply-accumulate in direction dir: the image shape's
-// tuned shape where one was set, else the options.
-void mac_shape(const flf_ctx *ctx, int dir, int &stages, int &chunk_rows, int &split) {
+// Stored rows per ring stage where none were asked for: the even number whose
+// chunks cost least (a chunk costs about four rows' time in barriers and copies
+// beside its own rows) among those that leave room for `want` CTAs per SM, as
+// many as the registers of nt frames allow.  Nnum 15, two stages, one frame: 12
+// rows forward, 16 back (three CTAs; full field 1864 us with 12 rows against 1992
+// with 10 and 2038 with 16 in two CTAs).
+int auto_chunk_rows(const Layout &L, int nt, int stages, bool fwd) {
+  const size_t sm_bytes = 228 * 1024, cta_reserve = 1024 + 512;   // of the SM; system and static use of a CTA
+  for (int want = nt <= 2 ? 3 : 2; want >= 1; want--) {
+    int best = 0, cost = 1 << 30;
+    for (int ch = want > 1 ? 6 : 2; ch <= 16; ch += 2) {
+      const size_t b = mac_smem_bytes(L, nt, stages, ch, fwd);
+      if (b > kMacSmemMax || want * (b + cta_reserve) > sm_bytes) break;
+      const int c = (2 * L.nrow + ch - 1) / ch * (ch + 4);
+      if (c <= cost) { cost = c; best = ch; }
+    }
+    if (best) return best;
+  }
+  return 2;
+}
+
+// Launch shape of the multiply-accumulate of nt frames in direction dir: the
+// image shape's tuned shape where one was set, else the options.
+void mac_shape(const flf_ctx *ctx, int dir, int nt, int &stages, int &chunk_rows, int &split) {
   const int *tn = ctx->geo.tuned;
   stages = tn[0] ? tn[0] : ctx->opt_stages;
   chunk_rows = tn[1 + dir] ? tn[1 + dir] : ctx->opt_chunk_rows[dir];
+  if (!chunk_rows) chunk_rows = auto_chunk_rows(ctx->L, nt, stages, dir == FLF_DIR_FORWARD);
   split = tn[3] ? tn[3] : ctx->opt_split;
   const int ntp = (ctx->L.nthr + 31) / 32 * 32;
   while (split > 1 && 2 * split * ntp > 256) split--;   // at most 256 threads per block
@@ -742,11 +764,11 @@ size_t mac_shape_bytes(const Layout &L, int stages, int chunk_rows, int split) {
 // not fit shared memory with the current launch shape (Nnum 19 at 12 rows per
 // stage: 2 frames).
 int frames_per_pass(const flf_ctx *ctx) {
-  for (int tf = mac_max_frames(); tf > 1; tf /= 2) {
+  for (int tf = mac_max_frames(); tf > 1; tf--) {
     bool fits = true;
     for (int d = 0; d < 2; d++) {
       int st, cr, sp;
-      mac_shape(ctx, d, st, cr, sp);
+      mac_shape(ctx, d, tf, st, cr, sp);
       if (mac_smem_bytes(ctx->L, tf, st, cr, d == FLF_DIR_FORWARD) > kMacSmemMax) fits = false;
     }
     if (fits) return tf;
@@ -759,7 +781,7 @@ MacParams mac_params(const flf_ctx *ctx, const Group &G, int dir, int nt) {
   mp.L = ctx->L; mp.f = G.f; mp.fh = G.fh; mp.fq = G.fq; mp.nkp = G.nkp; mp.nquads = G.nquads; mp.T = nt;
   mp.P = (const float4 *)G.P[dir];
   mp.rowS = ctx->d_rowS;
-  mac_shape(ctx, dir, mp.stages, mp.chunk_rows, mp.split);
+  mac_shape(ctx, dir, nt, mp.stages, mp.chunk_rows, mp.split);
   mp.err = ctx->d_err;
   mp.wait_ns = (unsigned long long)ctx->opt_wait_us * 1000ull;
   mp.drop_chunk = ctx->opt_drop_chunk;
@@ -1596,8 +1618,9 @@ int flf_set_option(flf_ctx *ctx, const char *name, long long value) {
   const bool cr_fwd = !strcmp(name, "mac_chunk_rows_forward"), cr_bwd = !strcmp(name, "mac_chunk_rows_backward");
   if (!strcmp(name, "mac_stages") || cr_all || cr_fwd || cr_bwd || !strcmp(name, "mac_split")) {
     const int st = !strcmp(name, "mac_stages") ? (int)value : ctx->opt_stages;
-    const int crf = (cr_all || cr_fwd) ? (int)value : ctx->opt_chunk_rows[FLF_DIR_FORWARD];
-    const int crb = (cr_all || cr_bwd) ? (int)value : ctx->opt_chunk_rows[FLF_DIR_BACKWARD];
+    // (rows chosen per launch fit every ring; shapes are accepted as with 12 rows)
+    const int crf = (cr_all || cr_fwd) ? (int)value : ctx->opt_chunk_rows[FLF_DIR_FORWARD] ? ctx->opt_chunk_rows[FLF_DIR_FORWARD] : 12;
+    const int crb = (cr_all || cr_bwd) ? (int)value : ctx->opt_chunk_rows[FLF_DIR_BACKWARD] ? ctx->opt_chunk_rows[FLF_DIR_BACKWARD] : 12;
     const int sp = !strcmp(name, "mac_split") ? (int)value : ctx->opt_split;
     if (st < 2 || st > 16) return fail(ctx, FLF_E_ARG, "mac_stages must be in [2, 16]");
     for (int cr : {crf, crb})
@@ -1610,8 +1633,8 @@ int flf_set_option(flf_ctx *ctx, const char *name, long long value) {
       if (mac_shape_bytes(ctx->L, st, cr, sp) > kMacSmemMax)
         return fail(ctx, FLF_E_ARG, "pipeline of %d stages x %d rows exceeds shared memory", st, cr);
     ctx->opt_stages = st;
-    ctx->opt_chunk_rows[FLF_DIR_FORWARD] = crf;
-    ctx->opt_chunk_rows[FLF_DIR_BACKWARD] = crb;
+    if (cr_all || cr_fwd) ctx->opt_chunk_rows[FLF_DIR_FORWARD] = crf;
+    if (cr_all || cr_bwd) ctx->opt_chunk_rows[FLF_DIR_BACKWARD] = crb;
     ctx->opt_split = sp;
     return FLF_OK;
   }

@@ -246,91 +246,77 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 
 constexpr unsigned long long kWaitLimitNs = 1000000000ull;   // 1 s per wait
 
-// Packed two-lane FP32 arithmetic (sm_100+): __ffma2_rn performs two
-// independent IEEE fused multiply-adds in one instruction, halving the issue
-// slots.  A complex accumulator gains element * real operand in one of them.
-__device__ __forceinline__ void fma_cr(float2 &acc, float2 e, float s) { acc = __ffma2_rn(e, make_float2(s, s), acc); }
+// Barrier of the first n threads of the block (the helper warp stays out).
+__device__ __forceinline__ void bar_sync(int n) { asm volatile("bar.sync 1, %0;\n" ::"r"(n) : "memory"); }
 
-// Asynchronous 8-byte global -> shared copy (completes at cp.async.wait_all).
-__device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
-// Stage the input spectra of plane slot `zs` at the four frequencies of the
-// quad into shared memory: comb[t][side][i] = S_i[u_side], comb[t][side][NN + i]
-// = S_i[u_side*], with u_0 = (uy, ux), u_1 = (ux, uy).
-__device__ __forceinline__ void stage_comb(float2 *comb, const MacParams &p, int TF, int zs, int uy, int ux) {
-  const int us = uy ? p.f - uy : 0, vs = ux ? p.f - ux : 0;
-  const int NN = p.L.NN, ffh = p.f * p.fh;
-  for (int idx = threadIdx.x; idx < TF * 2 * NN; idx += blockDim.x) {
-    const int i = idx % NN;
-    const int side = (idx / NN) & 1;
-    const int t = idx / (2 * NN);
-    float2 *dst = comb + (t * 2 + side) * 2 * NN;
-    if (t < p.T) {
-      const float2 *sb = p.S + ((long long)(t * p.nzS + zs) * NN + i) * ffh;
-      const int fy = side ? ux : uy, fys = side ? vs : us, fx = side ? uy : ux;
-      cp_async8(dst + i, sb + fy * p.fh + fx);
-      cp_async8(dst + NN + i, sb + fys * p.fh + fx);
-    } else {
-      dst[i] = make_float2(0.f, 0.f);
-      dst[NN + i] = make_float2(0.f, 0.f);
-    }
-  }
-  cp_async_commit();
-}
-
-// Operand table of one plane, built from comb:
-//   sv[t][half block][row][side][u / u*] = (p0, p1, m0, m1),
+// Operand table of one plane, straight from the input spectra:
+//   sv[t][half block][row][side][u / u*] = (p0, m0, p1, m1),
 // the real factors with which the row (C, D of every channel pair) enters the
 // accumulators of the receiving side,  P += C p0 + D p1,  M += C m0 + D m1.
 // With sa the spectrum that multiplies the row's channel directly and sb the
 // one that meets it through the Mxy mirror, w = sa + conj sb, v = sa - conj sb:
-// (p0, p1, m0, m1) = (Re w, Im w, Im v, -Re v).  rowS names sa and sb per use
+// (p0, m0, p1, m1) = (Re w, Im v, Im w, -Re v).  rowS names sa and sb per use
 // (0: the half block's own side, 1: the other side, through the transpose);
 // a second row (kRowSecond) counts nothing where the receiving frequency pair
-// is self-paired (u = u*), since its first row says the same.
+// is self-paired (u = u*), since its first row says the same.  fo: offsets of
+// the frequencies u, u* of side 0 and of side 1 in a spectrum.  Each spectrum
+// value enters one or two entries, so staging the spectra first would cost
+// more than it saves.
 template <int TF>
-__device__ void build_sv(float4 *sv, const float2 *comb, const short4 *rowS, const Layout &L, int nhalf, bool selfp0,
-                         bool selfp1) {
-  const int R = L.nrow, NN2 = 2 * L.NN;
-  const int per = R * 4;                               // entries of one half block
-  for (int idx = threadIdx.x; idx < TF * nhalf * per; idx += blockDim.x) {
-    const int uv = idx & 1, side = (idx >> 1) & 1;
-    const int tb = idx / per;                          // t * nhalf + half block
-    const int row = (idx - tb * per) >> 2;
-    const int t = tb / nhalf, bs = tb - t * nhalf;
-    const int use = side != bs;
-    if (use && row >= L.nrowT) continue;               // never read
-    const short4 si = rowS[use * R + row];
-    const int ia = uv ? si.z : si.x, ib = uv ? si.w : si.y;
-    const float2 *cb = comb + (t * 2 + side) * NN2 + uv * L.NN;
-    const bool zero = (rowS[2 * R + row].x & kRowSecond) && (side ? selfp1 : selfp0);
-    const float2 sa = ia >= 0 && !zero ? cb[ia] : make_float2(0.f, 0.f);
-    const float2 sb = ib >= 0 && !zero ? cb[ib] : make_float2(0.f, 0.f);
-    sv[((t * 2 + bs) * R + row) * 4 + side * 2 + uv] =
-        make_float4(sa.x + sb.x, sa.y - sb.y, sa.y + sb.y, sb.x - sa.x);
+__device__ void build_sv(float4 *sv, const MacParams &p, int zs, const short4 *rowS, int nhalf, bool selfp0,
+                         bool selfp1, const int (&fo)[4], int first, int step) {
+  constexpr int U = 4;                                 // entries per round, loads first
+  const int R = p.L.nrow, NN = p.L.NN, nT = p.L.nrowT;
+  const int ffh = p.f * p.fh;
+  const int n = min(TF, p.T) * nhalf * R * 4;
+  for (int i0 = first; i0 < n; i0 += U * step) {
+    float2 sa[U], sb[U];
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const int idx = i0 + k * step;
+      sa[k] = sb[k] = make_float2(0.f, 0.f);
+      if (idx >= n) continue;
+      const int e = idx & 3, side = e >> 1, rest = idx >> 2;
+      const int tb = rest / R, row = rest - tb * R;    // t * nhalf + half block
+      const int t = tb / nhalf, use = side != tb - t * nhalf;
+      if (use && row >= nT) continue;                  // never read
+      if ((rowS[2 * R + row].x & kRowSecond) && (side ? selfp1 : selfp0)) continue;
+      const short4 si = rowS[use * R + row];
+      const int ia = (e & 1) ? si.z : si.x, ib = (e & 1) ? si.w : si.y;
+      const float2 *src = p.S + (long long)(t * p.nzS + zs) * NN * ffh + (side ? ((e & 1) ? fo[3] : fo[2]) : ((e & 1) ? fo[1] : fo[0]));
+      if (ia >= 0) sa[k] = __ldg(src + ia * ffh);
+      if (ib >= 0) sb[k] = __ldg(src + ib * ffh);
+    }
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const int idx = i0 + k * step;
+      if (idx >= n) continue;
+      const int rest = idx >> 2, tb = rest / R, row = rest - tb * R;
+      const int t = tb / nhalf, bs = tb - t * nhalf;
+      sv[((t * 2 + bs) * R + row) * 4 + (idx & 3)] =
+          make_float4(sa[k].x + sb[k].x, sa[k].y + sb[k].y, sa[k].y - sb[k].y, sb[k].x - sa[k].x);
+    }
   }
 }
 
-// Shared memory of k_mac: ring | sv | scratch (comb staging, later the output
-// exchange) | rowS | mbarriers.
-__host__ __device__ inline size_t mac_scratch_elems(const Layout &L, int TF, bool fwd) {
-  return (size_t)(fwd ? 2 : 1) * TF * 2 * 2 * L.NN;                    // float2
-}
-__host__ __device__ inline size_t mac_scratch_pad(size_t e) { return (e + 1) & ~(size_t)1; }   // 16-byte multiple
-
+// Shared memory of k_mac: ring | operand tables (forward two, back projection
+// one) | back projection: output exchange | rowS | mbarriers.  (Forward, the
+// exchange uses the first operand table, which is the larger.)
 size_t mac_smem_bytes(const Layout &L, int TF, int stages, int chunk_rows, bool fwd) {
-  return sizeof(float2) * ((size_t)stages * chunk_rows * L.RS + mac_scratch_pad(mac_scratch_elems(L, TF, fwd))) +
-         sizeof(float4) * (size_t)TF * 2 * L.nrow * 4 + sizeof(short4) * 3 * L.nrow +
-         2 * sizeof(unsigned long long) * stages + 16;
+  return sizeof(float4) * ((size_t)stages * chunk_rows * L.NP + (size_t)(fwd && TF == 1 ? 2 : 1) * TF * 2 * L.nrow * 4) +
+         (fwd ? 0 : sizeof(float2) * (size_t)TF * 4 * L.NN) + sizeof(short4) * 3 * L.nrow +
+         2 * sizeof(unsigned long long) * (stages + 2) + 16;
 }
 
-// Accumulators of one thread: per side, frame and channel pair the P and M sums at u and u*.
+// Accumulators of one thread: per side, frame, channel pair and u / u* the lane
+// pairs X = (P.x, M.x) and Y = (P.y, M.y) for the packed two-lane FMA
+// (__ffma2_rn, two IEEE FMAs in one issue slot).  The operands come as lane pairs
+// from shared memory, only the streamed elements are doubled into both lanes
+// (four per channel pair and row, used on both sides and all frames); pairs of
+// (re, im) with doubled operands took 2 % longer at one frame and 5 % at four,
+// plain FMAs 3 % and 10 %.
 template <int TF, int PPT> struct MacAcc {
-  float2 UP[2][TF][PPT], UM[2][TF][PPT], VP[2][TF][PPT], VM[2][TF][PPT];
+  float2 X[2][TF][PPT][2], Y[2][TF][PPT][2];
   __device__ __forceinline__ void zero() {
 #pragma unroll
     for (int s = 0; s < 2; s++)
@@ -338,7 +324,8 @@ template <int TF, int PPT> struct MacAcc {
       for (int t = 0; t < TF; t++)
 #pragma unroll
         for (int k = 0; k < PPT; k++)
-          UP[s][t][k] = UM[s][t][k] = VP[s][t][k] = VM[s][t][k] = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int uv = 0; uv < 2; uv++) X[s][t][k][uv] = Y[s][t][k][uv] = make_float2(0.f, 0.f);
   }
 };
 
@@ -346,33 +333,28 @@ template <int TF, int PPT> struct MacAcc {
 template <int TF, int PPT, int S0, int S1>
 __device__ __forceinline__ void mac_row(const float4 *row, const int (&off)[PPT], const float4 *svr, int svt,
                                         MacAcc<TF, PPT> &a) {
-  float2 C[PPT], D[PPT];
+  float4 e[PPT];
 #pragma unroll
-  for (int k = 0; k < PPT; k++) {
-    const float4 e = row[off[k]];
-    C[k] = make_float2(e.x, e.y);
-    D[k] = make_float2(e.z, e.w);
-  }
+  for (int k = 0; k < PPT; k++) e[k] = row[off[k]];
 #pragma unroll
   for (int t = 0; t < TF; t++)
 #pragma unroll
-    for (int s = S0; s < S1; s++) {
-      const float4 u = svr[t * svt + s * 2], v = svr[t * svt + s * 2 + 1];
+    for (int s = S0; s < S1; s++)
 #pragma unroll
-      for (int k = 0; k < PPT; k++) {
-        fma_cr(a.UP[s][t][k], C[k], u.x);
-        fma_cr(a.UM[s][t][k], C[k], u.z);
-        fma_cr(a.VP[s][t][k], C[k], v.x);
-        fma_cr(a.VM[s][t][k], C[k], v.z);
-      }
+      for (int uv = 0; uv < 2; uv++) {
+        const float4 q = svr[t * svt + s * 2 + uv];   // p0, m0, p1, m1
+        const float2 q0 = make_float2(q.x, q.y), q1 = make_float2(q.z, q.w);
 #pragma unroll
-      for (int k = 0; k < PPT; k++) {
-        fma_cr(a.UP[s][t][k], D[k], u.y);
-        fma_cr(a.UM[s][t][k], D[k], u.w);
-        fma_cr(a.VP[s][t][k], D[k], v.y);
-        fma_cr(a.VM[s][t][k], D[k], v.w);
+        for (int k = 0; k < PPT; k++) {
+          a.X[s][t][k][uv] = __ffma2_rn(make_float2(e[k].x, e[k].x), q0, a.X[s][t][k][uv]);
+          a.Y[s][t][k][uv] = __ffma2_rn(make_float2(e[k].y, e[k].y), q0, a.Y[s][t][k][uv]);
+        }
+#pragma unroll
+        for (int k = 0; k < PPT; k++) {
+          a.X[s][t][k][uv] = __ffma2_rn(make_float2(e[k].z, e[k].z), q1, a.X[s][t][k][uv]);
+          a.Y[s][t][k][uv] = __ffma2_rn(make_float2(e[k].w, e[k].w), q1, a.Y[s][t][k][uv]);
+        }
       }
-    }
 }
 
 // Threads: `cw` warps side by side cover the channel pairs (PPT per lane), `H`
@@ -399,19 +381,23 @@ template <int TF, int TH> struct MacOcc {
 // per 1808-byte row (Nnum 15) an SM takes 77 cycles at the measured copy rate,
 // against 32 of FMA issue and 46 of shared memory (PPT = 2: two column warps
 // read the row once and 64 B of operands each; one pair per lane would read the
-// operands four times, four pairs would keep 64 accumulators a lane).  Measured
-// against the complex form (GB300, Nnum 15): back projection of 1005 x 1005 px,
-// 41 planes, one frame 2776 -> 1891 us (3.7 -> 5.4 TB/s), forward 3006 -> 2152 us;
-// three frames of 437 x 608 px, 31 planes, back 3202 -> 1242 us (the complex form
-// also ran three frames as four).
+// operands four times, four pairs would keep 64 accumulators a lane).  With three
+// and four frames the FMAs bound it (registers allow two CTAs per SM).
+// Measured (GB300, Nnum 15, sum of the launches of a projection; complex form
+// first): 1005 x 1005 px, 41 planes, one frame: back 2776 -> 1844 us (3.7 -> 5.6
+// TB/s), forward 3006 -> 1862 us (2152 with the operand tables built between
+// planes from staged spectra); 437 x 608 px, 31 planes, three frames: back
+// 3202 -> 1209 us; 450 x 450 px, 31 planes, four frames a launch: forward
+// 477 -> 207 us, back 462 -> 213 us a launch.
 // The stored rows stream through a ring of shared-memory stages filled by
 // bulk copies (crossing plane boundaries).  Forward projection accumulates the
-// planes of the group (the group sums are added by the inverse transform);
-// back projection writes each plane's spectra when the plane is done.  The
-// spectra of the next plane are staged with cp.async while the current plane
-// streams.
+// planes of the group (the group sums are added by the inverse transform), and
+// a helper warp (the last one) builds the next plane's operand table while the
+// current plane streams; back projection writes each plane's spectra when the
+// plane is done.
 template <int TF, bool FWD, int PPT, int TH>
-__global__ void __launch_bounds__(TH, MacOcc<TF, TH>::v) k_mac(MacParams p) {
+__global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>::v) k_mac(MacParams p) {
+  constexpr bool HELP = FWD && TF == 1;         // a helper warp builds the operand tables, two in turn
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ int s_abort;
   __shared__ int s_issued;                      // chunks handed to the bulk-copy engine
@@ -420,30 +406,19 @@ __global__ void __launch_bounds__(TH, MacOcc<TF, TH>::v) k_mac(MacParams p) {
   const Layout &L = p.L;
   const int NN = L.NN, N = L.N, NP = L.NP, R = L.nrow, nT = L.nrowT, NN2 = 2 * L.NN;
   const int CH = p.chunk_rows, NST = p.stages, H = p.shares;
+  const int svt = 2 * R * 4;                                                 // sv stride between frames (float4)
   float4 *ring = reinterpret_cast<float4 *>(smraw);                          // [NST][CH][NP]
-  float4 *sv = ring + (size_t)NST * CH * NP;                                 // [TF][2][R][2][2]
-  float2 *scratch = reinterpret_cast<float2 *>(sv + TF * 2 * R * 4);         // comb [1|2][TF][2][2NN] / outs
-  float2 *outs = scratch;                                                    // [TF][side][u | u*][NN]
-  short4 *rowS = reinterpret_cast<short4 *>(scratch + mac_scratch_pad(mac_scratch_elems(L, TF, FWD)));
+  float4 *sv0 = ring + (size_t)NST * CH * NP;                                // [1|2][TF][2][R][2][2]
+  float2 *outs = reinterpret_cast<float2 *>(FWD ? sv0 : sv0 + TF * svt);     // [TF][side][u | u*][NN]
+  short4 *rowS = reinterpret_cast<short4 *>(FWD ? reinterpret_cast<float2 *>(sv0 + (HELP ? 2 : 1) * TF * svt) : outs + TF * 4 * NN);
   unsigned long long *full = reinterpret_cast<unsigned long long *>(rowS + 3 * R);
-  int *released = reinterpret_cast<int *>(full + NST);   // [NST] warps done with each slot, ever
+  unsigned long long *svfull = full + NST;               // [2] operand table built (helper's lanes arrive)
+  unsigned long long *svfree = svfull + 2;               // [2] operand table read (a lane of each warp arrives)
+  int *released = reinterpret_cast<int *>(svfree + 2);   // [NST] warps done with each slot, ever
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nwarps = blockDim.x >> 5;
-  if (tid == 0) {
-    for (int i = 0; i < NST; i++) {
-      mbar_init(full + i, 1);
-      released[i] = 0;
-    }
-    *abortf = 0;
-    s_issued = 0;
-    fence_mbar_init();
-  }
-  for (int i = tid; i < 3 * R; i += blockDim.x) rowS[i] = p.rowS[i];
-  {
-    const int zb = blockIdx.y * p.zgroup, nzl = min(p.zgroup, p.nz - zb);
-    for (int i = tid; i < nzl; i += blockDim.x) s_plane[i] = p.planes[zb + i];
-  }
+  const int nwarps = (blockDim.x >> 5) - (HELP ? 1 : 0);  // streaming warps
+  const int nthreads = 32 * nwarps;
 
   // quad k = ux (ux + 1) / 2 + uy, uy <= ux
   const int kq = blockIdx.x;
@@ -456,69 +431,88 @@ __global__ void __launch_bounds__(TH, MacOcc<TF, TH>::v) k_mac(MacParams p) {
   const int nhalf = diag ? 1 : 2;
   const bool selfp0 = (uy == 0) || (2 * uy == p.f), selfp1 = (ux == 0) || (2 * ux == p.f);
   const int ffh = p.f * p.fh;
-  const int cw = nwarps / H;                     // column warps
-  const int h = warp / cw;                       // row share
-  const int p0 = (warp - h * cw) * 32 * PPT + lane;
-  int off[PPT];                                  // this lane's channel pairs (repeating the last one past the end)
-#pragma unroll
-  for (int k = 0; k < PPT; k++) off[k] = min(p0 + 32 * k, NP - 1);
   const int z0 = blockIdx.y * p.zgroup;
   const int z1 = min(z0 + p.zgroup, p.nz);
   const int nrq = nhalf * R;                     // stored rows of the quad per plane
   const int cpb = (nrq + CH - 1) / CH;           // chunks per (quad, plane)
   const int total = (z1 - z0) * cpb;
   const size_t halfElems = (size_t)R * NP;       // float4
-  const int combStride = TF * 2 * NN2;           // one plane's staged spectra (float2)
-  const int svt = 2 * R * 4;                     // sv stride between frames (float4)
 
-  MacAcc<TF, PPT> acc;
-  acc.zero();
-
-  stage_comb(scratch, p, TF, FWD ? z0 : 0, uy, ux);
-  cp_async_wait_all();
-  __syncthreads();   // barriers initialised, row tables and first spectra staged
-  build_sv<TF>(sv, scratch, rowS, L, nhalf, selfp0, selfp1);
-  __syncthreads();   // (back projection: the staging area is free for the output exchange)
-
-  // Chunk g goes to ring slot g % NST.  Thread 0 fills the whole ring; after
-  // that, the warp that releases a slot last (each warp counts itself out
-  // once it has finished its rows of the chunk) refills it at once with chunk
-  // g + NST, so no thread ever waits for a slot to drain.
+  // Chunk g goes to ring slot g % NST.  Thread 0 fills the whole ring before
+  // anything else; after that, the warp that releases a slot last (each warp
+  // counts itself out once it has finished its rows of the chunk) refills it at
+  // once with chunk g + NST, so no thread ever waits for a slot to drain.
   // p.drop_chunk >= 0 (a test of the bounded waits only): the first CTA never
   // issues that chunk, so the waits on its slot run out after p.wait_ns
   const int drop = blockIdx.x == 0 && blockIdx.y == 0 ? p.drop_chunk : -1;
-  auto issue = [&](int gn) {
+  auto issue = [&](int gn, const int *planes) {
     if (gn == drop) return;
     const int zl_n = gn / cpb, ch_n = gn - zl_n * cpb, sl = gn % NST;
     const int r0 = ch_n * CH;
     const int nr = min(CH, nrq - r0);
-    const float4 *src = p.P + ((long long)s_plane[zl_n] * p.nkp + hb0) * (long long)halfElems + (long long)r0 * NP;
+    const float4 *src = p.P + ((long long)planes[zl_n] * p.nkp + hb0) * (long long)halfElems + (long long)r0 * NP;
     const unsigned bytes = (unsigned)(nr * NP * sizeof(float4));
     mbar_arrive_expect_tx(full + sl, bytes);
     bulk_g2s(ring + (size_t)sl * CH * NP, src, bytes, full + sl);
   };
   if (tid == 0) {
+    for (int i = 0; i < NST; i++) {
+      mbar_init(full + i, 1);
+      released[i] = 0;
+    }
+    for (int i = 0; i < 2; i++) {
+      mbar_init(svfull + i, 32);
+      mbar_init(svfree + i, nwarps);
+    }
+    *abortf = 0;
+    fence_mbar_init();
     const int pre = min(NST, total);
-    for (int g = 0; g < pre; g++) issue(g);
+    for (int g = 0; g < pre; g++) issue(g, p.planes + z0);
     s_issued = pre;
   }
+  for (int i = tid; i < 3 * R; i += blockDim.x) rowS[i] = p.rowS[i];
+  for (int i = tid; i < z1 - z0; i += blockDim.x) s_plane[i] = p.planes[z0 + i];
+  const int fo[4] = {uy * p.fh + ux, (uy ? p.f - uy : 0) * p.fh + ux, ux * p.fh + uy, (ux ? p.f - ux : 0) * p.fh + uy};
+  __syncthreads();   // barriers initialised, row tables staged
+  build_sv<TF>(sv0, p, FWD ? z0 : 0, rowS, nhalf, selfp0, selfp1, fo, tid, blockDim.x);
+  __syncthreads();
+
+  if (HELP && warp == nwarps) {
+    // helper warp: operand tables of the planes after the first, two in turn
+    for (int zl = 1; zl < z1 - z0; zl++) {
+      const int b = zl & 1;
+      if (zl > 1 && !mbar_wait(svfree + b, ((zl >> 1) - 1) & 1, p.wait_ns)) break;   // the waiting warps report it
+      build_sv<TF>(sv0 + b * TF * svt, p, z0 + zl, rowS, nhalf, selfp0, selfp1, fo, lane, 32);
+      mbar_arrive(svfull + b);
+    }
+    __syncthreads();   // the streaming warps' last barrier
+    return;
+  }
+
+  const int cw = nwarps / H;                     // column warps
+  const int h = warp / cw;                       // row share
+  const int p0 = (warp - h * cw) * 32 * PPT + lane;
+  int off[PPT];                                  // this lane's channel pairs (repeating the last one past the end)
+#pragma unroll
+  for (int k = 0; k < PPT; k++) off[k] = min(p0 + 32 * k, NP - 1);
+
+  MacAcc<TF, PPT> acc;
+  acc.zero();
 
   bool dead = false;
   int zl = 0, ch = 0, slot = 0;
   int round = 0;
   for (int g = 0; g < total; g++) {
     const int zi = z0 + zl;
-    if (FWD && ch == 0) {
-      if (zl > 0) {
-        cp_async_wait_all();
-        __syncthreads();   // spectra of plane zi staged; all threads done with plane zi-1
-        build_sv<TF>(sv, scratch + (zl & 1) * combStride, rowS, L, nhalf, selfp0, selfp1);
-        __syncthreads();
-      }
-      if (zi + 1 < z1) stage_comb(scratch + ((zl + 1) & 1) * combStride, p, TF, zi + 1, uy, ux);
+    if (FWD && !HELP && ch == 0 && zl > 0) {
+      bar_sync(nthreads);   // every warp is done with plane zi - 1
+      build_sv<TF>(sv0, p, zi, rowS, nhalf, selfp0, selfp1, fo, tid, nthreads);
+      bar_sync(nthreads);
     }
     if (*abortf) dead = true;
-    if (!dead && !mbar_wait(full + slot, round & 1, p.wait_ns)) {
+    // table zl: the helper's fill number zl >> 1 of buffer zl & 1 (buffer 0's first one is not counted)
+    if (!dead && ((HELP && ch == 0 && zl > 0 && !mbar_wait(svfull + (zl & 1), ((zl - 1) >> 1) & 1, p.wait_ns)) ||
+                  !mbar_wait(full + slot, round & 1, p.wait_ns))) {
       dead = true;
       *abortf = 1;
       atomicExch(p.err, 2);
@@ -532,7 +526,7 @@ __global__ void __launch_bounds__(TH, MacOcc<TF, TH>::v) k_mac(MacParams p) {
       for (int bs = r0 >= R ? 1 : 0; bs * R < r1; bs++) {
         const int base = bs * R;
         const int lo = max(r0, base) - base, hi = min(r1, base + R) - base;   // half-block rows
-        const float4 *svb = sv + (size_t)bs * R * 4;
+        const float4 *svb = sv0 + (HELP ? (zl & 1) * TF * svt : 0) + (size_t)bs * R * 4;
         const float4 *srow = stage + (base - r0) * NP;
         const int rb = min(hi, nT);
 #pragma unroll 2
@@ -551,18 +545,16 @@ __global__ void __launch_bounds__(TH, MacOcc<TF, TH>::v) k_mac(MacParams p) {
       if (before == round * nwarps + nwarps - 1 && g + NST < total && !*abortf) {
         __threadfence_block();
         fence_proxy_async_smem();                  // ... before the bulk copy that overwrites it
-        issue(g + NST);
+        issue(g + NST, s_plane);
         atomicAdd(&s_issued, 1);
       }
+      if (HELP && ch == cpb - 1) mbar_arrive(svfree + (zl & 1));
     }
 
     const bool out_due = (ch == cpb - 1) && (!FWD || zi + 1 == z1);
     if (out_due) {
       // the row shares add their channel values into outs in share order
-      if (FWD) {
-        cp_async_wait_all();   // the staging area doubles as the exchange buffer
-        __syncthreads();
-      }
+      if (FWD) bar_sync(nthreads);   // every warp is done with the operand tables
       for (int hh = 0; hh < H; hh++) {
         if (h == hh) {
 #pragma unroll
@@ -578,8 +570,8 @@ __global__ void __launch_bounds__(TH, MacOcc<TF, TH>::v) k_mac(MacParams p) {
                 for (int t = 0; t < TF; t++) {
                   float2 *ou = outs + (size_t)(t * 2 + s) * NN2, *ov = ou + NN;
                   // first + conj(second) = 2 P, first - conj(second) = 2 i M (the halves are in C and D)
-                  auto put = [&](float2 *o, int c1, float2 P, float2 M) {
-                    float2 x = make_float2(P.x - M.y, P.y + M.x), y = make_float2(P.x + M.y, M.x - P.y);
+                  auto put = [&](float2 *o, int c1, float2 X, float2 Y) {   // X = (P.x, M.x), Y = (P.y, M.y)
+                    float2 x = make_float2(X.x - Y.y, Y.x + X.y), y = make_float2(X.x + Y.y, X.y - Y.x);
                     const int c2 = NN - 1 - c1;                  // equal for the centre, then x = y
                     if (hh > 0) {
                       const float2 ox = o[c1], oy = o[c2];
@@ -588,19 +580,19 @@ __global__ void __launch_bounds__(TH, MacOcc<TF, TH>::v) k_mac(MacParams p) {
                     o[c1] = x;
                     o[c2] = y;
                   };
-                  put(ou, j, acc.UP[s][t][k], acc.UM[s][t][k]);
-                  put(ov, m, acc.VP[s][t][k], acc.VM[s][t][k]);
+                  put(ou, j, acc.X[s][t][k][0], acc.Y[s][t][k][0]);
+                  put(ov, m, acc.X[s][t][k][1], acc.Y[s][t][k][1]);
                 }
               }
             }
           }
         }
-        __syncthreads();
+        bar_sync(nthreads);
       }
       if (!dead) {
         const int nside = diag ? 1 : 2;
         const int nt = min(TF, p.T);
-        for (int idx = tid; idx < nt * nside * NN; idx += blockDim.x) {
+        for (int idx = tid; idx < nt * nside * NN; idx += nthreads) {
           const int q = idx % NN, ts = idx / NN;
           const int t = ts / nside, s = ts - t * nside;
           const float2 *o = outs + (size_t)(t * 2 + s) * NN2 + q;
@@ -622,7 +614,7 @@ __global__ void __launch_bounds__(TH, MacOcc<TF, TH>::v) k_mac(MacParams p) {
         }
       }
       acc.zero();
-      if (g + 1 < total) __syncthreads();   // the exchange buffer is free again
+      if (g + 1 < total) bar_sync(nthreads);   // the exchange buffer is free again
     }
     if (++ch == cpb) { ch = 0; zl++; }
     if (++slot == NST) { slot = 0; round++; }
@@ -634,7 +626,6 @@ __global__ void __launch_bounds__(TH, MacOcc<TF, TH>::v) k_mac(MacParams p) {
     for (int g = max(0, issued - NST); g < issued; g++)
       if (g != drop) mbar_wait(full + (g % NST), (g / NST) & 1, kWaitLimitNs / 10);
   }
-  cp_async_wait_all();
 }
 
 // ----------------------------------------------------------------------------
@@ -936,8 +927,8 @@ static cudaError_t launch_mac_tf(const MacParams &p0, cudaStream_t s) {
   p.shares = th.shares;
   const size_t sm = mac_smem_bytes(p.L, TF, p.stages, p.chunk_rows, FWD);
   const dim3 grid(p.nquads, p.nzo_grid);
-  const int block = 32 * th.cw * th.shares;
-  void (*fn)(MacParams) = block <= 128 ? (th.ppt == 2 ? k_mac<TF, FWD, 2, 128> : k_mac<TF, FWD, 1, 128>)
+  const int threads = 32 * th.cw * th.shares, block = threads + (FWD && TF == 1 ? 32 : 0);   // and the helper warp
+  void (*fn)(MacParams) = threads <= 128 ? (th.ppt == 2 ? k_mac<TF, FWD, 2, 128> : k_mac<TF, FWD, 1, 128>)
                                        : (th.ppt == 2 ? k_mac<TF, FWD, 2, 256> : k_mac<TF, FWD, 1, 256>);
   cudaError_t e = set_smem((const void *)fn, sm);
   if (e != cudaSuccess) return e;
