@@ -299,8 +299,9 @@ struct WgradParams {         // dw[tap][ci][co] += sum_v x[v + tap][ci] dy[v][co
   const __nv_bfloat16 *dy;
   float *dw;
   int B, Z, Y, X, Ci, Co;
-  long long chunk;           // voxels per CTA (set by the launcher)
+  long long chunk;           // row blocks per CTA (set by the launcher)
   float *part;               // [chunks][27][Ci][Co] partial gradients, reduced in chunk order (or null)
+  int ny = 3;                // dy taps per CTA (set by the launcher): 3, or 1 without a workspace
 };
 cudaError_t launch_conv3d(ConvParams p, long long ws_elems, cudaStream_t s);
 cudaError_t launch_conv3d_pool(const ConvParams &p, cudaStream_t s);

@@ -27,10 +27,11 @@
 //                     slabs, packed weights streamed by bulk copies, persistent
 //                     CTAs with two TMEM accumulator buffers.
 //   k_conv3d_wgrad    weight gradient dW[tap][ci][co] = sum_v x[v+tap][ci]
-//                     dy[v][co]: per (voxel chunk, tap, channel tile) one CTA,
-//                     split-K over its 4 warps; each chunk writes a partial
-//                     sum and k_wgrad_reduce adds them in chunk order (no
-//                     atomics, so training repeats bit for bit).
+//                     dy[v][co]: per (chunk of rows, dz, channel tile) one
+//                     CTA, whose staged rows serve the nine taps of that dz;
+//                     each chunk writes a partial sum and k_wgrad_reduce adds
+//                     them in chunk order (no atomics, so training repeats bit
+//                     for bit).
 //   small kernels     bias gradient, 2x2x2 average pooling and its adjoint,
 //                     nearest 2x2x2 upsampling + skip and its adjoint with the
 //                     ReLU mask, MSE loss gradient, Adam, bead rendering.
@@ -1200,119 +1201,162 @@ __global__ void __launch_bounds__(352, 1)
   }
 }
 
-// Weight gradient.  CTA = (voxel chunk, tap) x (ci tile CM, co tile CN); the 4
-// warps take alternate k16 steps of its voxels (split-K) and are summed in
-// shared memory at the end.  The tile goes to its chunk's slice of p.part,
-// and k_wgrad_reduce adds the chunks to dW in chunk order, so the gradient is
-// the same bits on every run; with one chunk (p.part null) the CTA adds its
-// tile to dW itself (one writer per element).
-template <int CM, int CN>
-__global__ void __launch_bounds__(128) k_conv3d_wgrad(WgradParams p) {
-  constexpr int BK = 64, NS = 3, RA = CM / 8, RBc = CN / 8;
-  __shared__ __align__(128) bf16 Xs[NS][BK * CM];
-  __shared__ __align__(128) bf16 Ds[NS][BK * CN];
+// Weight gradient dW[tap][ci][co] = sum_v x[v + tap][ci] dy[v][co] on mma.sync.
+// CTA = (chunk of row blocks, dz) x (ci tile CM, co tile CN).  A row block is
+// four consecutive y rows of one (b, z, segment of TX voxels); the CTA marches
+// along y with the x rows (with one voxel of halo on either side) and the dy rows
+// of five blocks in shared memory, so a row is staged once for the nine taps of
+// its dz.  Warp (dy, row of the block) multiplies its whole row for the three dx
+// taps: per 16 voxels one fragment set of dy and three of x (the rows start one
+// voxel apart), accumulated in registers over the whole chunk.  The four rows'
+// sums are added in shared memory in row order; the tile goes to its chunk's
+// slice of p.part, and k_wgrad_reduce adds the chunks to dW in chunk order, so
+// the gradient is the same bits on every run; with one chunk (p.part null) the
+// CTA adds its tile to dW itself (one writer per element), and the nine (dz, dy)
+// have CTAs of their own (ny = 1), three warps sharing a row.
+// 16 -> 16 channels at 4 x 24 x 128 x 128, weight and bias gradient together: 1880
+// us with one CTA per tap (x and dy staged 27 times, an index division per 16
+// bytes) and one channel per thread in the bias sums, 161 us now.
+constexpr int kWgRows = 4, kWgSlots = 5, kWgWarps = 12;
+template <int CM, int CN, int TX>
+constexpr size_t wgrad_smem() {
+  const size_t ring = (size_t)kWgSlots * kWgRows * ((TX + 2) * CM + TX * CN) * sizeof(bf16);
+  const size_t red = (size_t)9 * CM * CN * sizeof(float);
+  return ring > red ? ring : red;
+}
+template <int CM, int CN, int TX>
+__global__ void __launch_bounds__(32 * kWgWarps, 1) k_conv3d_wgrad(WgradParams p) {
+  constexpr int RA = CM / 8, RB = CN / 8, XV = TX + 2, NT = 32 * kWgWarps;
+  extern __shared__ __align__(128) unsigned char wgsm[];
+  bf16 *Xs = reinterpret_cast<bf16 *>(wgsm);                               // [slot][row][XV][CM]
+  bf16 *Ds = Xs + (size_t)kWgSlots * kWgRows * XV * CM;                    // [slot][row][TX][CN]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const long long M = (long long)p.B * p.Z * p.Y * p.X;
-  const int tap = blockIdx.x % 27;
-  const long long chunk = blockIdx.x / 27;
+  const int parts = p.ny == 3 ? 3 : 9;                                     // (dz) or (dz, dy) per chunk
+  const int part = blockIdx.x % parts;
+  const long long chunk = blockIdx.x / parts;
+  const int dz = p.ny == 3 ? part : part / 3;                              // 0..2
+  const int wy = p.ny == 3 ? warp % 3 : part % 3;                          // this warp's dy, 0..2
+  const int wr = p.ny == 3 ? warp / 3 : warp & 3;                          // its row of the block
+  const int k0s = p.ny == 3 ? 0 : warp >> 2, kss = p.ny == 3 ? 1 : 3;      // its 16-voxel steps of the row
   const int ctiles = p.Co / CN;
   const int ci0 = (blockIdx.y / ctiles) * CM, co0 = (blockIdx.y % ctiles) * CN;
-  const long long v0 = chunk * p.chunk;
-  const long long v1 = v0 + p.chunk < M ? v0 + p.chunk : M;
-  const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-  const int KS = (int)((v1 - v0 + BK - 1) / BK);
+  const int nblk = (p.Y + kWgRows - 1) / kWgRows, nseg = (p.X + TX - 1) / TX;
+  const long long items = (long long)p.B * p.Z * nseg * nblk;
+  const long long i1 = min(items, (chunk + 1) * p.chunk);
 
-  auto load = [&](int ks, int st) {
-    for (int i = tid; i < BK * (RA + RBc); i += 128) {
-      const int row = i / (RA + RBc), c = i - row * (RA + RBc);
-      const long long vv = v0 + (long long)ks * BK + row;
-      const bool in = vv < v1;
-      if (c < RA) {
-        bool ok = false;
-        const bf16 *src = p.x;
-        if (in) {
-          const Vox q = decode(vv, p.Z, p.Y, p.X);
-          const int z = q.z + dz, y = q.y + dy, x = q.x + dx;
-          ok = z >= 0 && z < p.Z && y >= 0 && y < p.Y && x >= 0 && x < p.X;
-          if (ok) src = p.x + ((((long long)q.b * p.Z + z) * p.Y + y) * p.X + x) * p.Ci + ci0 + c * 8;
-        }
-        cp16(su32(&Xs[st][row * CM]) + ((c ^ swz<RA>(row)) << 4), src, ok);
-      } else {
-        const int cc = c - RA;
-        const bf16 *src = in ? p.dy + vv * p.Co + co0 + cc * 8 : p.dy;
-        cp16(su32(&Ds[st][row * CN]) + ((cc ^ swz<RBc>(row)) << 4), src, in);
-      }
-    }
-  };
-
-  float acc[CM / 16][CN / 8][4];
+  float acc[3][CM / 16][CN / 8][4];
 #pragma unroll
-  for (int i = 0; i < CM / 16; i++)
+  for (int d = 0; d < 3; d++)
 #pragma unroll
-    for (int j = 0; j < CN / 8; j++)
+    for (int i = 0; i < CM / 16; i++)
 #pragma unroll
-      for (int e = 0; e < 4; e++) acc[i][j][e] = 0.f;
-
+      for (int j = 0; j < CN / 8; j++)
 #pragma unroll
-  for (int s = 0; s < NS - 1; s++) {
-    if (s < KS) load(s, s);
-    cp_commit();
-  }
+        for (int e = 0; e < 4; e++) acc[d][i][j][e] = 0.f;
   const int mat = lane >> 3, r8 = lane & 7;
-  for (int ks = 0; ks < KS; ks++) {
-    cp_wait<NS - 2>();
-    __syncthreads();
-    const int st = ks % NS;
-    const int kr = warp * 16;   // this warp's 16 voxels of the stage
-    uint32_t a[CM / 16][4];
-#pragma unroll
-    for (int mt = 0; mt < CM / 16; mt++) {
-      // A[ci][k] from Xs[k][ci]: transposed 8x8 blocks (k rows, ci chunk)
-      const int row = kr + r8 + 8 * (mat >> 1);
-      const int c = mt * 2 + (mat & 1);
-      ldsm4t(su32(&Xs[st][row * CM]) + ((c ^ swz<RA>(row)) << 4), a[mt][0], a[mt][1], a[mt][2], a[mt][3]);
+
+  for (long long it = chunk * p.chunk; it < i1;) {
+    // a run: consecutive row blocks [kb, ke) of one (b, z, segment)
+    const int kb = (int)(it % nblk);
+    const int ke = (int)min((long long)nblk, kb + (i1 - it));
+    const long long col = it / nblk;
+    it += ke - kb;
+    const int seg = (int)(col % nseg);
+    const long long bz = col / nseg;
+    const int z = (int)(bz % p.Z), zx = z + dz - 1;
+    if (zx < 0 || zx >= p.Z) continue;
+    const int x0 = seg * TX, xw = min(TX, p.X - x0);
+    const int k16 = (xw + 15) >> 4;                                        // 16-voxel steps
+    const bf16 *xs = p.x + ((bz - z + zx) * p.Y * p.X + x0 - 1) * p.Ci + ci0;   // voxel x0 - 1 of row 0
+    const bf16 *ds = p.dy + (bz * p.Y * p.X + x0) * p.Co + co0;
+    // rows of block k into its slot; voxels outside the volume (and dy beyond the
+    // segment or the run) are zeros
+    auto load = [&](int k) {
+      const int slot = (k - kb + 1) % kWgSlots;
+      const int xu = (16 * k16 + 2) * RA, du = 16 * k16 * RB;
+      for (int i = tid; i < kWgRows * xu; i += NT) {
+        const int r = i / xu, e = i - r * xu, v = e / RA, c = e - v * RA;
+        const int y = kWgRows * k + r, x = x0 - 1 + v;
+        const bool ok = y >= 0 && y < p.Y && x >= 0 && x < p.X;
+        cp16(su32(Xs + ((size_t)(slot * kWgRows + r) * XV + v) * CM) + ((c ^ swz<RA>(v)) << 4),
+             ok ? xs + ((long long)y * p.X + v) * p.Ci + c * 8 : p.x, ok);
+      }
+      if (k >= kb && k < ke)
+        for (int i = tid; i < kWgRows * du; i += NT) {
+          const int r = i / du, e = i - r * du, v = e / RB, c = e - v * RB;
+          const int y = kWgRows * k + r;
+          const bool ok = y < p.Y && v < xw;
+          cp16(su32(Ds + ((size_t)(slot * kWgRows + r) * TX + v) * CN) + ((c ^ swz<RB>(v)) << 4),
+               ok ? ds + ((long long)y * p.X + v) * p.Co + c * 8 : p.dy, ok);
+        }
+    };
+    for (int k = kb - 1; k <= kb + 2; k++) {
+      if (k <= ke) load(k);
+      cp_commit();
     }
+    for (int k = kb; k < ke; k++) {
+      cp_wait<1>();        // blocks up to k + 1 have arrived
+      __syncthreads();     // for every warp, and block k - 2's slot is free
+      if (k + 3 <= ke) load(k + 3);
+      cp_commit();
+      if (kWgRows * k + wr < p.Y) {
+        const int j = wr + wy - 1;                                         // x row of the tap, relative to the block
+        const int xk = j < 0 ? k - 1 : j >= kWgRows ? k + 1 : k;
+        const bf16 *xr = Xs + (size_t)(((xk - kb + 1) % kWgSlots) * kWgRows + (j & (kWgRows - 1))) * XV * CM;
+        const bf16 *dr = Ds + (size_t)(((k - kb + 1) % kWgSlots) * kWgRows + wr) * TX * CN;
+        for (int ks = k0s; ks < k16; ks += kss) {
+          uint32_t bq[CN / 16][4];
 #pragma unroll
-    for (int n2 = 0; n2 < CN / 16; n2++) {
-      const int row = kr + r8 + 8 * (mat & 1);
-      const int c = n2 * 2 + (mat >> 1);
-      uint32_t b0, b1, b2, b3;
-      ldsm4t(su32(&Ds[st][row * CN]) + ((c ^ swz<RBc>(row)) << 4), b0, b1, b2, b3);
+          for (int n2 = 0; n2 < CN / 16; n2++) {
+            const int row = 16 * ks + r8 + 8 * (mat & 1), c = n2 * 2 + (mat >> 1);
+            ldsm4t(su32(dr + row * CN) + ((c ^ swz<RB>(row)) << 4), bq[n2][0], bq[n2][1], bq[n2][2], bq[n2][3]);
+          }
 #pragma unroll
-      for (int mt = 0; mt < CM / 16; mt++) {
-        mma_bf16(acc[mt][2 * n2], a[mt], b0, b1);
-        mma_bf16(acc[mt][2 * n2 + 1], a[mt], b2, b3);
+          for (int d = 0; d < 3; d++) {
+            // A[ci][voxel] from rows of ci: transposed 8x8 blocks, d voxels further
+#pragma unroll
+            for (int mt = 0; mt < CM / 16; mt++) {
+              const int row = 16 * ks + d + r8 + 8 * (mat >> 1), c = mt * 2 + (mat & 1);
+              uint32_t a[4];
+              ldsm4t(su32(xr + row * CM) + ((c ^ swz<RA>(row)) << 4), a[0], a[1], a[2], a[3]);
+#pragma unroll
+              for (int n2 = 0; n2 < CN / 16; n2++) {
+                mma_bf16(acc[d][mt][2 * n2], a, bq[n2][0], bq[n2][1]);
+                mma_bf16(acc[d][mt][2 * n2 + 1], a, bq[n2][2], bq[n2][3]);
+              }
+            }
+          }
+        }
       }
     }
-    const int nk = ks + NS - 1;
-    if (nk < KS) load(nk, nk % NS);
-    cp_commit();
+    cp_wait<0>();
+    __syncthreads();       // the next run's loads reuse the slots
   }
-  cp_wait<0>();
-  __syncthreads();
-  // sum the 4 warps' partial tiles in shared memory (reuses the ring)
-  float *red = reinterpret_cast<float *>(&Xs[0][0]);
-  static_assert(sizeof(Xs) >= sizeof(float) * CM * CN, "reduction buffer");
-  for (int i = tid; i < CM * CN; i += 128) red[i] = 0.f;
-  __syncthreads();
-  for (int w = 0; w < 4; w++) {
-    if (warp == w) {
+  // add the rows' (and steps') sums in a fixed order (reuses the ring)
+  float *red = reinterpret_cast<float *>(wgsm);                            // [dy][dx][CM][CN]
+  const int ny = p.ny, group = ny == 3 ? wr : warp, ngroups = kWgWarps / ny;
+  for (int g = 0; g < ngroups; g++) {
+    if (group == g) {
+      float *rw = red + (ny == 3 ? wy : 0) * 3 * CM * CN;
 #pragma unroll
-      for (int mt = 0; mt < CM / 16; mt++)
+      for (int d = 0; d < 3; d++)
 #pragma unroll
-        for (int nt = 0; nt < CN / 8; nt++)
+        for (int mt = 0; mt < CM / 16; mt++)
 #pragma unroll
-          for (int e = 0; e < 4; e++) {
-            const int ci = mt * 16 + (lane >> 2) + 8 * (e >> 1);
-            const int co = nt * 8 + 2 * (lane & 3) + (e & 1);
-            red[ci * CN + co] += acc[mt][nt][e];
-          }
+          for (int nt = 0; nt < CN / 8; nt++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+              const int ci = mt * 16 + (lane >> 2) + 8 * (e >> 1), co = nt * 8 + 2 * (lane & 3) + (e & 1);
+              float *o = rw + (d * CM + ci) * CN + co;
+              *o = g ? *o + acc[d][mt][nt][e] : acc[d][mt][nt][e];
+            }
     }
     __syncthreads();
   }
   const long long nw = 27LL * p.Ci * p.Co;
-  for (int i = tid; i < CM * CN; i += 128) {
-    const int ci = i / CN, co = i - ci * CN;
+  for (int i = tid; i < ny * 3 * CM * CN; i += NT) {
+    const int t = i / (CM * CN), e = i - t * CM * CN, ci = e / CN, co = e - ci * CN;
+    const int tap = dz * 9 + (ny == 3 ? t : (part % 3) * 3 + t);
     const long long o = ((long long)tap * p.Ci + ci0 + ci) * p.Co + co0 + co;
     if (p.part) p.part[chunk * nw + o] = red[i];
     else p.dw[o] += red[i];
@@ -1323,6 +1367,7 @@ __global__ void __launch_bounds__(128) k_conv3d_wgrad(WgradParams p) {
 __global__ void k_wgrad_reduce(const float *part, float *dw, long long n, int chunks) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     float s = 0.f;
+#pragma unroll 8
     for (int c = 0; c < chunks; c++) s += part[(long long)c * n + i];
     dw[i] += s;
   }
@@ -1341,23 +1386,64 @@ __global__ void k_conv3d_flip_weights(const bf16 *w, bf16 *w2, int Ci, int Co) {
 
 // Sums over rows of g[M][C], one row block per CTA: into part[block][c] (then
 // k_bias_reduce adds the blocks in order), or with a single block (part null)
-// straight into db[c].
-__global__ void k_bias_grad(const bf16 *g, float *db, float *part, long long M, int C, long long rows_per_block) {
-  const int c = threadIdx.x;
-  if (c >= C) return;
+// straight into db[c].  V8ROWS: 16 bytes (8 channels) a load, the rows dealt to
+// the threads and their sums added in thread order (C a multiple of 8, g
+// 16-byte aligned); else one channel per thread.
+template <bool V8ROWS>
+__global__ void __launch_bounds__(256) k_bias_grad(const bf16 *g, float *db, float *part, long long M, int C,
+                                                   long long rows_per_block) {
   const long long r0 = (long long)blockIdx.x * rows_per_block;
   const long long r1 = r0 + rows_per_block < M ? r0 + rows_per_block : M;
   float s = 0.f;
-  for (long long r = r0; r < r1; r++) s += __bfloat162float(g[r * C + c]);
+  const int c = threadIdx.x;
+  if constexpr (V8ROWS) {
+    __shared__ float sm[256 * 8];
+    const int G = C / 8, lanes = 256 / G;              // row lanes; threads past lanes * G idle
+    const int gi = threadIdx.x % G, rl = threadIdx.x / G;
+    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (rl < lanes) {
+#pragma unroll 4
+      for (long long r = r0 + rl; r < r1; r += lanes) {
+        const uint4 u = *reinterpret_cast<const uint4 *>(g + r * C + gi * 8);
+        const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&u);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const float2 f = __bfloat1622float2(h[k]);
+          v[2 * k] += f.x;
+          v[2 * k + 1] += f.y;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 8; k++) sm[rl * C + gi * 8 + k] = v[k];
+    }
+    __syncthreads();
+    if (c >= C) return;
+    for (int i = 0; i < lanes; i++) s += sm[i * C + c];
+  } else {
+    if (c >= C) return;
+    for (long long r = r0; r < r1; r++) s += __bfloat162float(g[r * C + c]);
+  }
   if (part) part[(long long)blockIdx.x * C + c] = s;
   else db[c] += s;
 }
 
-__global__ void k_bias_reduce(const float *part, float *db, int blocks, int C) {
-  const int c = threadIdx.x;
-  if (c >= C) return;
+// db[c] += sum over the blocks of part[block][c]: runs of consecutive blocks per
+// thread, the runs added in order.
+__global__ void __launch_bounds__(1024) k_bias_reduce(const float *part, float *db, int blocks, int C) {
+  __shared__ float sm[1024];
+  const int runs = 1024 / C, c = threadIdx.x % C, r = threadIdx.x / C;
+  const int len = (blocks + runs - 1) / runs;
   float s = 0.f;
-  for (int b = 0; b < blocks; b++) s += part[(long long)b * C + c];
+  if (r < runs) {
+    const int b1 = min(blocks, (r + 1) * len);
+#pragma unroll 8
+    for (int b = r * len; b < b1; b++) s += part[(long long)b * C + c];
+    sm[r * C + c] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x >= C) return;
+  s = 0.f;
+  for (int i = 0; i < runs; i++) s += sm[i * C + c];
   db[c] += s;
 }
 
@@ -2346,27 +2432,38 @@ cudaError_t launch_conv3d(ConvParams p, long long ws_elems, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+template <int CM, int CN, int TX>
+static cudaError_t launch_wgrad_t(const WgradParams &p, dim3 grid, cudaStream_t s) {
+  constexpr size_t sm = wgrad_smem<CM, CN, TX>();
+  cudaError_t e = cudaFuncSetAttribute((const void *)k_conv3d_wgrad<CM, CN, TX>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return e;
+  FLF_NET_LAUNCH(k_conv3d_wgrad<CM, CN, TX><<<grid, 32 * kWgWarps, sm, s>>>(p));
+  return cudaGetLastError();
+}
+
+// One CTA per SM (the ring takes most of the shared memory): as many chunks as
+// fill them, within the workspace's slices.
 cudaError_t launch_conv3d_wgrad(WgradParams p, long long ws_elems, cudaStream_t s, int num_sms) {
   const long long M = (long long)p.B * p.Z * p.Y * p.X;
   if (M == 0) return cudaSuccess;
-  const int CM = p.Ci >= 32 ? 32 : 16, CN = p.Co >= 64 ? 64 : p.Co;
+  const int CM = p.Ci % 32 == 0 ? 32 : 16, CN = p.Co % 32 == 0 ? 32 : 16, TX = CM + CN == 32 ? 128 : 64;
   const int tiles = (p.Ci / CM) * (p.Co / CN);
   const long long nw = 27LL * p.Ci * p.Co;
-  long long chunks = (4LL * num_sms + 27 * tiles - 1) / (27 * tiles);
+  const long long items = (long long)p.B * p.Z * ((p.X + TX - 1) / TX) * ((p.Y + kWgRows - 1) / kWgRows);
+  long long chunks = num_sms / (3LL * tiles);
+  if (chunks > items) chunks = items;
   if (!p.part) chunks = 1;                                         // no workspace: one writer per element
   else if (chunks > ws_elems / nw) chunks = ws_elems / nw;         // partial tiles must fit the workspace
   if (chunks < 1) chunks = 1;
-  long long per = (M + chunks - 1) / chunks;
-  per = (per + 63) / 64 * 64;
-  chunks = (M + per - 1) / per;
-  p.chunk = per;
+  p.chunk = (items + chunks - 1) / chunks;
+  chunks = (items + p.chunk - 1) / p.chunk;
   if (chunks == 1) p.part = nullptr;
-  dim3 grid((unsigned)(chunks * 27), (unsigned)tiles);
-#define FLF_WG(a, b) else if (CM == a && CN == b) FLF_NET_LAUNCH(k_conv3d_wgrad<a, b><<<grid, 128, 0, s>>>(p));
-  if (false) {
-  }
-  FLF_WG(16, 16) FLF_WG(16, 32) FLF_WG(16, 64) FLF_WG(32, 16) FLF_WG(32, 32) FLF_WG(32, 64)
-#undef FLF_WG
+  p.ny = p.part ? 3 : 1;
+  const dim3 grid((unsigned)(chunks * (p.ny == 3 ? 3 : 9)), (unsigned)tiles);
+  cudaError_t e = CM == 32 ? (CN == 32 ? launch_wgrad_t<32, 32, 64>(p, grid, s) : launch_wgrad_t<32, 16, 64>(p, grid, s))
+                           : (CN == 32 ? launch_wgrad_t<16, 32, 64>(p, grid, s) : launch_wgrad_t<16, 16, 128>(p, grid, s));
+  if (e != cudaSuccess) return e;
   if (p.part) FLF_NET_LAUNCH(k_wgrad_reduce<<<grid_for(nw, 256), 256, 0, s>>>(p.part, p.dw, nw, (int)chunks));
   return cudaGetLastError();
 }
@@ -2439,8 +2536,11 @@ cudaError_t launch_bias_grad(const void *g, float *db, float *ws, long long ws_e
   const long long rows = (M + blocks - 1) / blocks;
   blocks = (M + rows - 1) / rows;
   float *part = blocks > 1 ? ws : nullptr;
-  FLF_NET_LAUNCH(k_bias_grad<<<(unsigned)blocks, 128, 0, s>>>((const bf16 *)g, db, part, M, C, rows));
-  if (part) FLF_NET_LAUNCH(k_bias_reduce<<<1, 128, 0, s>>>(part, db, (int)blocks, C));
+  if (C % 8 == 0 && ((uintptr_t)g & 15) == 0)
+    FLF_NET_LAUNCH(k_bias_grad<true><<<(unsigned)blocks, 256, 0, s>>>((const bf16 *)g, db, part, M, C, rows));
+  else
+    FLF_NET_LAUNCH(k_bias_grad<false><<<(unsigned)blocks, 128, 0, s>>>((const bf16 *)g, db, part, M, C, rows));
+  if (part) FLF_NET_LAUNCH(k_bias_reduce<<<1, 1024, 0, s>>>(part, db, (int)blocks, C));
   return cudaGetLastError();
 }
 
