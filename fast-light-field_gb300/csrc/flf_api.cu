@@ -35,6 +35,9 @@ struct Group {
   double2 *tw64 = nullptr;    // double twiddles [f]
   float2 *P[2] = {nullptr, nullptr};   // packed matrices [slot][nkp half blocks][nrow][NP][C, D]
   bool built[2] = {false, false};
+  // complex elements of one channel's spectrum in row order (forward output) and in quad order
+  size_t spec() const { return (size_t)f * fh; }
+  size_t qspec() const { return (size_t)4 * nquads; }
   std::vector<int> planes;    // plane ids of the group, ascending (slot = index)
   int *d_ids = nullptr;       // device copy of `planes`
   int *d_slots = nullptr;     // 0..n-1
@@ -670,16 +673,17 @@ void ws_needs(const flf_ctx *ctx, const PlaneSet &ps, int nt, bool fwd, size_t &
   sS = sO = sCv = 0;
   for (size_t g = 0; g < G.groups.size(); g++) {
     if (!ps.n[g]) continue;
-    const size_t spec = sizeof(float2) * (size_t)NN * G.groups[g].f * G.groups[g].fh;
+    const size_t spec = sizeof(float2) * (size_t)NN * G.groups[g].spec();
+    const size_t qspec = sizeof(float2) * (size_t)NN * G.groups[g].qspec();
     const int n = ps.n[g];
     sCv = std::max(sCv, cset * nt * n);
     if (fwd) {
       const int zg = zgroup_for(ctx, n, G.groups[g].nquads);
-      sS = std::max(sS, spec * nt * n);
+      sS = std::max(sS, qspec * nt * n);
       sO = std::max(sO, spec * nt * ((n + zg - 1) / zg));
     } else {
-      sS = std::max(sS, spec * nt);
-      sO = std::max(sO, spec * nt * n);
+      sS = std::max(sS, qspec * nt);
+      sO = std::max(sO, qspec * nt * n);
     }
   }
 }
@@ -798,7 +802,7 @@ cudaError_t mac_group_launch(flf_ctx *ctx, size_t gi, int dir, int nt, const Pla
   MacParams mp = mac_params(ctx, G, dir, nt);
   mp.stages = stages; mp.chunk_rows = chunk; mp.split = split;
   mp.planes = ps.slots[gi]; mp.nz = nplanes; mp.zgroup = zg;
-  mp.S = (const float2 *)ctx->wsS.p; mp.O = (float2 *)ctx->wsO.p;
+  mp.S = (const float2 *)ctx->wsS.p; mp.O = (float4 *)ctx->wsO.p;
   if (dir == FLF_DIR_FORWARD) {
     mp.nzS = nplanes; mp.nzo = (nplanes + zg - 1) / zg; mp.nzo_grid = mp.nzo;
   } else {
@@ -831,7 +835,7 @@ Irfft2Params irfft2_params(const flf_ctx *ctx, const Group &G, const float2 *src
   const Geometry &Gm = ctx->geo;
   Irfft2Params ip{};
   ip.plan = G.plan; ip.N = ctx->N; ip.Y = Gm.Y; ip.X = Gm.X; ip.Ly = Gm.Ly; ip.Lx = Gm.Lx;
-  ip.nimg = nimg; ip.src = src; ip.sum_stride = 0; ip.nsum = 1;
+  ip.nimg = nimg; ip.src = src; ip.quads = 0; ip.sum_stride = 0; ip.nsum = 1;
   ip.chan = chan; ip.Lxp = channel_pitch(Gm.Lx); ip.twiddle = G.tw;
   return ip;
 }
@@ -886,7 +890,7 @@ int forward_chunk(flf_ctx *ctx, const float *vol, long long vol_sz, const PlaneS
     void *wS = (char *)ctx->wsS.p + slot * sS;
     float2 *wO = (float2 *)((char *)ctx->wsO.p + slot * sO);
     const Group &G = Gm.groups[gi];
-    const int ffh = G.f * G.fh;
+    const size_t sp1 = G.spec();
     const int zgroup = zgroup_for(ctx, nplanes, G.nquads);
     const int nzg = (nplanes + zgroup - 1) / zgroup;
 
@@ -895,21 +899,21 @@ int forward_chunk(flf_ctx *ctx, const float *vol, long long vol_sz, const PlaneS
     LAUNCH(ctx, "k_split", chan_bytes(ctx, nt * nplanes) + 4.0 * Y * X * nt * nplanes, s, launch_split(sp, s));
 
     Rfft2Params rp = rfft2_params(ctx, G, cvol, nt * nplanes * NN, wS);
-    LAUNCH(ctx, "k_rfft2", chan_bytes(ctx, nt * nplanes) + 8.0 * ffh * NN * nt * nplanes, s, launch_rfft2(rp, 0, s));
+    LAUNCH(ctx, "k_rfft2", chan_bytes(ctx, nt * nplanes) + 8.0 * sp1 * NN * nt * nplanes, s, launch_rfft2(rp, 0, s));
 
     const double pbytes = (double)nplanes * G.nkp * L.nrow * L.RS * sizeof(float2);
     MacParams mp = mac_params(ctx, G, FLF_DIR_FORWARD, nt);
     mp.planes = ps.slots[gi]; mp.nz = nplanes; mp.zgroup = zgroup;
-    mp.S = (const float2 *)wS; mp.nzS = nplanes; mp.O = wO; mp.nzo = nzg;
+    mp.S = (const float2 *)wS; mp.nzS = nplanes; mp.O = (float4 *)wO; mp.nzo = nzg;
     mp.nzo_grid = nzg;
-    LAUNCH(ctx, "k_mac_fwd", pbytes + 8.0 * ffh * NN * nt * ((double)nplanes + nzg), s, launch_mac(mp, true, s));
+    LAUNCH(ctx, "k_mac_fwd", pbytes + 8.0 * sp1 * NN * nt * ((double)nplanes + nzg), s, launch_mac(mp, true, s));
 
     if (k > 0 && nslot > 1) CUDA_TRY(ctx, cudaStreamWaitEvent(s, ctx->ev_chain, 0));
     Irfft2Params ip = irfft2_params(ctx, G, wO, nt * NN, chan);
-    ip.sum_stride = (long long)nt * NN * ffh; ip.nsum = nzg;
+    ip.sum_stride = (long long)(nt * NN * sp1); ip.nsum = nzg;
     ip.add = !first; ip.final_pass = (int)gi == last; ip.num = ip.final_pass ? num : nullptr;
     const double cb = chan_bytes(ctx, nt) * (1 + ip.add + (ip.num ? 1 : 0));
-    LAUNCH(ctx, "k_irfft2", 8.0 * ffh * NN * nt * nzg + cb, s, launch_irfft2(ip, s));
+    LAUNCH(ctx, "k_irfft2", 8.0 * sp1 * NN * nt * nzg + cb, s, launch_irfft2(ip, s));
     if (nslot > 1) CUDA_TRY(ctx, cudaEventRecord(ctx->ev_chain, s));
     first = false;
     k++;
@@ -949,22 +953,22 @@ int backward_chunk(flf_ctx *ctx, const float *chan, const PlaneSet &ps, int nt, 
     void *wS = (char *)ctx->wsS.p + slot * sS;
     float2 *wO = (float2 *)((char *)ctx->wsO.p + slot * sO);
     const Group &G = Gm.groups[gi];
-    const int ffh = G.f * G.fh;
+    const size_t sp1 = G.spec();
 
     Rfft2Params rp = rfft2_params(ctx, G, chan, nt * NN, wS);
-    LAUNCH(ctx, "k_rfft2", chan_bytes(ctx, nt) + 8.0 * ffh * NN * nt, s, launch_rfft2(rp, 0, s));
+    LAUNCH(ctx, "k_rfft2", chan_bytes(ctx, nt) + 8.0 * sp1 * NN * nt, s, launch_rfft2(rp, 0, s));
 
     const double pbytes = (double)nplanes * G.nkp * L.nrow * L.RS * sizeof(float2);
     const int zgb = zgroup_for(ctx, nplanes, G.nquads);
     MacParams mp = mac_params(ctx, G, FLF_DIR_BACKWARD, nt);
     mp.planes = ps.slots[gi]; mp.nz = nplanes; mp.zgroup = zgb;
-    mp.S = (const float2 *)wS; mp.nzS = 1; mp.O = wO; mp.nzo = nplanes;
+    mp.S = (const float2 *)wS; mp.nzS = 1; mp.O = (float4 *)wO; mp.nzo = nplanes;
     mp.nzo_grid = (nplanes + zgb - 1) / zgb;
-    LAUNCH(ctx, "k_mac_bwd", pbytes + 8.0 * ffh * NN * nt * (1.0 + nplanes), s, launch_mac(mp, false, s));
+    LAUNCH(ctx, "k_mac_bwd", pbytes + 8.0 * sp1 * NN * nt * (1.0 + nplanes), s, launch_mac(mp, false, s));
 
     Irfft2Params ip = irfft2_params(ctx, G, wO, nt * nplanes * NN, cvol);
-    ip.final_pass = 1;
-    LAUNCH(ctx, "k_irfft2", 8.0 * ffh * NN * nt * nplanes + chan_bytes(ctx, nt * nplanes), s, launch_irfft2(ip, s));
+    ip.final_pass = 1; ip.quads = 1;
+    LAUNCH(ctx, "k_irfft2", 8.0 * sp1 * NN * nt * nplanes + chan_bytes(ctx, nt * nplanes), s, launch_irfft2(ip, s));
 
     MergeParams mg = merge_params(ctx, cvol, ps.ids[gi], nplanes, nt, epi, out, aux, norm);
     const int npix = epi == EPI_STORE ? 1 : (epi == EPI_RL_STANDARD && norm.p ? 4 : 3);
@@ -981,7 +985,11 @@ int backward_chunk(flf_ctx *ctx, const float *chan, const PlaneSet &ps, int nt, 
 // flf_ctx_create forces by looking up the array's address (below): from then
 // on the GPU holds FLF_NOALLOC_SCRATCH_BYTES of it until the process exits.
 // ----------------------------------------------------------------------------
-static __device__ __align__(256) unsigned char g_noalloc_scratch[FLF_NOALLOC_SCRATCH_BYTES];
+// Geometries are accepted by FLF_NOALLOC_SCRATCH_BYTES for spectra of f (f/2+1)
+// values; the quad order of the output stores 2 (f/2+1)(f/2+2) of them, 32 Nnum^2
+// (f/2+1) bytes more, under 1.5 MiB for every geometry accepted (two spectra of it).
+constexpr size_t kNoallocBytes = FLF_NOALLOC_SCRATCH_BYTES + (3u << 19);
+static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocBytes];
 
 // Device address of the scratch array in the current CUDA context.  The
 // host-side symbol is only a stand-in and must never reach a kernel.  Called
@@ -1188,7 +1196,7 @@ int flf_backward_noalloc(flf_ctx *ctx, const float *img_dev, float *vol_dev, int
   const size_t cimg = up(sizeof(float) * chan_set_floats(ctx));
   size_t need = 0;
   for (const Group &G : Gm.groups) {
-    const size_t spec = up(sizeof(float2) * (size_t)NN * G.f * G.fh);
+    const size_t spec = up(sizeof(float2) * (size_t)NN * G.f * G.fh);   // (the rule: see kNoallocBytes)
     need = std::max(need, spec + cimg + spec + cimg);
   }
   if (need > FLF_NOALLOC_SCRATCH_BYTES)
@@ -1206,12 +1214,12 @@ int flf_backward_noalloc(flf_ctx *ctx, const float *img_dev, float *vol_dev, int
     cudaError_t e = launch_split(split_params(ctx, img_dev + t * YX, 0, YX, nullptr, 1, 1, C), s);
     for (size_t gi = 0; gi < Gm.groups.size() && e == cudaSuccess; gi++) {
       const Group &G = Gm.groups[gi];
-      const size_t spec = up(sizeof(float2) * (size_t)NN * G.f * G.fh);   // one frame or one plane
+      const size_t spec = up(sizeof(float2) * (size_t)NN * G.qspec());   // one frame or one plane
       float2 *S = (float2 *)(base + cimg);
       char *blocks = base + cimg + spec;
       const size_t per_plane = spec + cimg;
       const int ng = (int)G.planes.size();
-      const int zb = std::max(1, std::min(ng, (int)((FLF_NOALLOC_SCRATCH_BYTES - cimg - spec) / per_plane)));
+      const int zb = std::max(1, std::min(ng, (int)((kNoallocBytes - cimg - spec) / per_plane)));
       float2 *O = (float2 *)blocks;
       float *Co = (float *)(blocks + spec * zb);
       e = launch_rfft2(rfft2_params(ctx, G, C, NN, S), 0, s);
@@ -1220,11 +1228,11 @@ int flf_backward_noalloc(flf_ctx *ctx, const float *img_dev, float *vol_dev, int
         const int zg = zgroup_for(ctx, nzl, G.nquads);
         MacParams mp = mac_params(ctx, G, FLF_DIR_BACKWARD, 1);
         mp.planes = G.d_slots + z0; mp.nz = nzl; mp.zgroup = zg;
-        mp.S = S; mp.nzS = 1; mp.O = O; mp.nzo = nzl; mp.nzo_grid = (nzl + zg - 1) / zg;
+        mp.S = S; mp.nzS = 1; mp.O = (float4 *)O; mp.nzo = nzl; mp.nzo_grid = (nzl + zg - 1) / zg;
         e = launch_mac(mp, false, s);
         if (e != cudaSuccess) break;
         Irfft2Params ip = irfft2_params(ctx, G, O, nzl * NN, Co);
-        ip.final_pass = 1;
+        ip.final_pass = 1; ip.quads = 1;
         e = launch_irfft2(ip, s);
         if (e != cudaSuccess) break;
         const Strided out{vol_dev + t * YX, (long long)T * YX, YX};

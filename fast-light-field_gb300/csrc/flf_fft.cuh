@@ -16,13 +16,29 @@
 //   R1  rows 2q, 2q+1 packed as one complex row, row pass 1      global -> B
 //   R2  row pass 2 and the split of the two real rows' spectra   B -> A
 //   R3  column pass 1 (rows beyond the image read as zero)      A -> A
-//   R4  column pass 2, natural-order store                      A -> global
+//   R4  column pass 2                                            A -> A
+//   R5  store in quad order                                      A -> global
 // Inverse (irfft2, spectrum -> real Ly x Lx channel image):
+//   A0  (quad order) the input spectra to their places           global -> A
 //   A1  column pass 1 on the (summed) input spectra              global -> A
+//       (quad order: A -> A)
 //   A2  column pass 2                                            A -> A
 //   B1  Hermitian expansion of rows 2q, 2q+1 packed as one complex
 //       row, row pass 1                                          A -> B
 //   B2  row pass 2 and the pixel epilogue                        B -> global
+//
+// Quad order: per frequency quad k = hi (hi + 1) / 2 + lo (lo <= hi <= F/2, the
+// unit of the multiply-accumulate) a spectrum's four values at (lo, hi),
+// (-lo, hi), (hi, lo), (-hi, lo) side by side: 32 bytes, one sector, which the
+// multiply-accumulate reads (every input spectrum) or writes (the back
+// projection's output) whole for a channel.  In row order its 8-byte accesses
+// touched four sectors a channel, 43 million partial sectors in the output of 41
+// planes at f = 96: the multiply-accumulate took 1844 us back and 1862 forward
+// there against 1704 and 1789 in quad order, where R5 and A0, one more pass over
+// shared memory each, add 25 to 35 us to the transforms.  The values that a
+// self-paired frequency or a diagonal quad repeats are written by R5 and not
+// read by A0.  The forward projection's few output sets (one per group of planes)
+// stay in row order, which A1 sums as it reads (16 us less than through A0).
 #pragma once
 
 #include "flf_internal.cuh"
@@ -89,6 +105,7 @@ template <int F> struct Shape {
   static constexpr int P1 = split_p1(F);
   static constexpr int P2 = F / P1;
   static constexpr int FH = F / 2 + 1;
+  static constexpr int NQ = FH * (FH + 1) / 2;   // frequency quads
   static constexpr int PA = FH;       // row pitch (complex) of the F x FH buffer A
   static constexpr int PB = F + 1;    // row pitch of the packed-row buffer B (odd: no bank conflicts across rows)
   static constexpr int NT = F <= 48 ? 128 : 256;
@@ -297,6 +314,14 @@ __device__ __forceinline__ void load_twiddles(float2 *TW, const float2 *__restri
   }
 }
 
+// Frequency quad k = hi (hi + 1) / 2 + lo.
+__device__ __forceinline__ void quad_of(int k, int &lo, int &hi) {
+  hi = (int)((sqrtf(8.f * (float)k + 1.f) - 1.f) * 0.5f);
+  if ((hi + 1) * (hi + 2) / 2 <= k) hi++;
+  if (hi * (hi + 1) / 2 > k) hi--;
+  lo = k - hi * (hi + 1) / 2;
+}
+
 // ----------------------------------------------------------------------------
 // Forward transform of channel-major images (Rfft2Params mode 0): image g is
 // channel ch = g % NN = b*N + a, Ly x Lx samples of pixels (r*N + b, c*N + a);
@@ -411,14 +436,22 @@ __global__ void __launch_bounds__(Shape<F>::NT, Shape<F>::MINB) k_rfft2_sized(Rf
   }
   __syncthreads();
 
-  // R4: column pass 2; frequency ky = k1 + P1 k2 stored in natural order.
-  float2 *dst = reinterpret_cast<float2 *>(p.dst) + (long long)g * (F * FH);
+  // R4: column pass 2; frequency ky = k1 + P1 k2 ends up at row k1 * P2 + k2.
   for (int task = threadIdx.x; task < FH * P1; task += NT) {
     const int k1 = task / FH, c = task - k1 * FH;
-    float2 u[P2];
-    SFor<0, P2>::run([&](auto T) { u[decltype(T)::value] = A[(k1 * P2 + decltype(T)::value) * PA + c]; });
-    Dft<P2, -1>::run(u);
-    SFor<0, P2>::run([&](auto T) { dst[(k1 + P1 * decltype(T)::value) * FH + c] = u[decltype(T)::value]; });
+    pass2<F, -1>(reinterpret_cast<float *>(A + (k1 * P2) * PA + c), PA);
+  }
+  __syncthreads();
+
+  // R5: the quads, two 16-byte stores each.
+  float4 *dst = reinterpret_cast<float4 *>(p.dst) + (long long)g * (2 * Sh::NQ);
+  auto at = [&](int ky, int kx) { return A[((ky % P1) * P2 + ky / P1) * PA + kx]; };
+  for (int k = threadIdx.x; k < Sh::NQ; k += NT) {
+    int lo, hi;
+    quad_of(k, lo, hi);
+    const float2 u0 = at(lo, hi), v0 = at(lo ? F - lo : 0, hi), u1 = at(hi, lo), v1 = at(hi ? F - hi : 0, lo);
+    dst[2 * k] = make_float4(u0.x, u0.y, v0.x, v0.y);
+    dst[2 * k + 1] = make_float4(u1.x, u1.y, v1.x, v1.y);
   }
 }
 
@@ -429,7 +462,7 @@ __global__ void __launch_bounds__(Shape<F>::NT, Shape<F>::MINB) k_rfft2_sized(Rf
 // zeroes the samples outside the Y x X image and the row padding, and can
 // store num / value instead of the value.
 // ----------------------------------------------------------------------------
-template <int F>
+template <int F, bool QUADS>
 __global__ void __launch_bounds__(Shape<F>::NT, Shape<F>::MINB) k_irfft2_sized(Irfft2Params p, SizedArgs sa) {
   using Sh = Shape<F>;
   constexpr int P1 = Sh::P1, P2 = Sh::P2, FH = Sh::FH, PA = Sh::PA, PB = Sh::PB, NT = Sh::NT;
@@ -440,24 +473,46 @@ __global__ void __launch_bounds__(Shape<F>::NT, Shape<F>::MINB) k_irfft2_sized(I
   load_twiddles<F>(TW, p.twiddle);
 
   const int g = blockIdx.x;
-  const float2 *src = p.src + (long long)g * (F * FH);
   const int nsum = p.nsum;
+
+  // A0: the values of the quads to their places (those that a self-paired
+  // frequency or a diagonal quad repeats are not read).
+  if constexpr (QUADS) {
+    const float4 *src = reinterpret_cast<const float4 *>(p.src) + (long long)g * (2 * Sh::NQ);
+#pragma unroll 4
+    for (int k = threadIdx.x; k < Sh::NQ; k += NT) {
+      const float4 a = __ldg(src + 2 * k), b = __ldg(src + 2 * k + 1);
+      int lo, hi;
+      quad_of(k, lo, hi);
+      A[lo * PA + hi] = make_float2(a.x, a.y);
+      if (lo != 0 && 2 * lo != F) A[(F - lo) * PA + hi] = make_float2(a.z, a.w);
+      if (lo != hi) {
+        A[hi * PA + lo] = make_float2(b.x, b.y);
+        if (2 * hi != F) A[(F - hi) * PA + lo] = make_float2(b.z, b.w);
+      }
+    }
+  }
   __syncthreads();
 
-  // A1: column pass 1 straight from the input spectra.
+  // A1: column pass 1, in row order straight from the (summed) input spectra.
+  const float2 *src = p.src + (long long)g * (F * FH);
   for (int task = threadIdx.x; task < FH * P2; task += NT) {
     const int t = task / FH, c = task - t * FH;
     float2 x[P1];
-    SFor<0, P1>::run([&](auto K) {
-      constexpr int k = decltype(K)::value;
-      x[k] = src[(t + P2 * k) * FH + c];
-    });
-    for (int s = 1; s < nsum; s++) {
-      const float2 *ps = src + s * p.sum_stride;
+    if constexpr (QUADS) {
+      SFor<0, P1>::run([&](auto K) { x[decltype(K)::value] = A[(t + P2 * decltype(K)::value) * PA + c]; });
+    } else {
       SFor<0, P1>::run([&](auto K) {
         constexpr int k = decltype(K)::value;
-        x[k] = add2(x[k], ps[(t + P2 * k) * FH + c]);
+        x[k] = src[(t + P2 * k) * FH + c];
       });
+      for (int s = 1; s < nsum; s++) {
+        const float2 *ps = src + s * p.sum_stride;
+        SFor<0, P1>::run([&](auto K) {
+          constexpr int k = decltype(K)::value;
+          x[k] = add2(x[k], ps[(t + P2 * k) * FH + c]);
+        });
+      }
     }
     Dft<P1, 1>::run(x);
     twiddle_pass1<F, 1>(x, TW, t);
@@ -586,19 +641,19 @@ template <int F> cudaError_t irfft2_sized(const Irfft2Params &p, cudaStream_t s)
   template <int F> cudaError_t rfft2_sized(const Rfft2Params &p, cudaStream_t s) {                    \
     const SizedArgs sa = sized_args<F>(p.Ly, p.Lxp);                                                  \
     const size_t sm = smem_bytes<F>(sa.nq, sa.a_len);                                                 \
-    cudaError_t e = cudaFuncSetAttribute((const void *)k_rfft2_sized<F>,                              \
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);       \
+    void (*fn)(Rfft2Params, SizedArgs) = k_rfft2_sized<F>;                                            \
+    cudaError_t e = cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
     if (e != cudaSuccess) return e;                                                                   \
-    k_rfft2_sized<F><<<p.nimg, Shape<F>::NT, sm, s>>>(p, sa);                                         \
+    fn<<<p.nimg, Shape<F>::NT, sm, s>>>(p, sa);                                                       \
     return cudaGetLastError();                                                                        \
   }                                                                                                   \
   template <int F> cudaError_t irfft2_sized(const Irfft2Params &p, cudaStream_t s) {                  \
     const SizedArgs sa = sized_args<F>(p.Ly, p.Lxp);                                                  \
     const size_t sm = smem_bytes<F>(sa.nq, sa.a_len);                                                 \
-    cudaError_t e = cudaFuncSetAttribute((const void *)k_irfft2_sized<F>,                             \
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);       \
+    void (*fn)(Irfft2Params, SizedArgs) = p.quads ? k_irfft2_sized<F, true> : k_irfft2_sized<F, false>; \
+    cudaError_t e = cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
     if (e != cudaSuccess) return e;                                                                   \
-    k_irfft2_sized<F><<<p.nimg, Shape<F>::NT, sm, s>>>(p, sa);                                        \
+    fn<<<p.nimg, Shape<F>::NT, sm, s>>>(p, sa);                                                       \
     return cudaGetLastError();                                                                        \
   }
 

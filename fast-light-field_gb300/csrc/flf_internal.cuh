@@ -139,7 +139,7 @@ struct Rfft2Params {
   const float *chan;        // mode 0: [nimg][Ly][Lxp], image g = set * NN + ch
   int Lxp;
   const void *src_img;      // mode 1: Real images [nimg][f][f]
-  void *dst;                // Complex<Real> [nimg][f][fh]
+  void *dst;                // mode 0: complex [nimg][quads][4]; mode 1: Complex<Real> [nimg][f][fh]
   const void *twiddle;      // Complex<Real> [f]
   int imgs_per_cta;         // mode 1
   int nq_rows;              // mode 1: row pairs carrying data (<= f/2)
@@ -149,7 +149,8 @@ struct Irfft2Params {
   FftPlan plan;
   int N, Y, X, Ly, Lx;
   int nimg;                 // images g = set * NN + j
-  const float2 *src;        // spectra [nsum][nimg][f][fh]
+  const float2 *src;        // spectra [nsum][nimg][f][fh], or with quads [nimg][quads][4]
+  int quads;                // quad order (nsum = 1)
   long long sum_stride;     // elements between partial sums
   int nsum;
   float *chan;              // output: channel-major [nimg][Ly][Lxp]
@@ -200,9 +201,10 @@ struct MacParams {
   const int *planes;        // plane id per z index
   int nz;                   // planes in the list
   int zgroup;               // forward: planes per CTA group
-  const float2 *S;          // input spectra [T][nzS][NN][f][fh]
+  const float2 *S;          // input spectra [T][nzS][NN][nquads][4] (quad order)
   int nzS;                  // planes in S (forward nz, backward 1)
-  float2 *O;                // output spectra
+  float4 *O;                // output spectra: forward [zgroup][T][NN][f][fh] complex; backward
+                            // [T][nzo][NN][nquads][2 sides], u and u* of a side (quad order)
   int nzo;                  // forward: number of z groups (output sets); backward: nz
   int nzo_grid;             // grid.y: number of z groups of this launch
   const short4 *rowS;       // [3][nrow]: operand channels of each row for its own frequency pair (0)

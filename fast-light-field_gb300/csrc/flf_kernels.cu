@@ -258,16 +258,16 @@ __device__ __forceinline__ void bar_sync(int n) { asm volatile("bar.sync 1, %0;\
 // (p0, m0, p1, m1) = (Re w, Im v, Im w, -Re v).  rowS names sa and sb per use
 // (0: the half block's own side, 1: the other side, through the transpose);
 // a second row (kRowSecond) counts nothing where the receiving frequency pair
-// is self-paired (u = u*), since its first row says the same.  fo: offsets of
-// the frequencies u, u* of side 0 and of side 1 in a spectrum.  Each spectrum
-// value enters one or two entries, so staging the spectra first would cost
-// more than it saves.
+// is self-paired (u = u*), since its first row says the same.  A channel's four
+// values of quad kq (u, u* of side 0, then of side 1) lie side by side in its
+// spectrum.  Each enters one or two entries, so staging the spectra first would
+// cost more than it saves.
 template <int TF>
 __device__ void build_sv(float4 *sv, const MacParams &p, int zs, const short4 *rowS, int nhalf, bool selfp0,
-                         bool selfp1, const int (&fo)[4], int first, int step) {
+                         bool selfp1, int kq, int first, int step) {
   constexpr int U = 4;                                 // entries per round, loads first
   const int R = p.L.nrow, NN = p.L.NN, nT = p.L.nrowT;
-  const int ffh = p.f * p.fh;
+  const int ss = 4 * p.nquads;                         // values of a spectrum
   const int n = min(TF, p.T) * nhalf * R * 4;
   for (int i0 = first; i0 < n; i0 += U * step) {
     float2 sa[U], sb[U];
@@ -283,9 +283,9 @@ __device__ void build_sv(float4 *sv, const MacParams &p, int zs, const short4 *r
       if ((rowS[2 * R + row].x & kRowSecond) && (side ? selfp1 : selfp0)) continue;
       const short4 si = rowS[use * R + row];
       const int ia = (e & 1) ? si.z : si.x, ib = (e & 1) ? si.w : si.y;
-      const float2 *src = p.S + (long long)(t * p.nzS + zs) * NN * ffh + (side ? ((e & 1) ? fo[3] : fo[2]) : ((e & 1) ? fo[1] : fo[0]));
-      if (ia >= 0) sa[k] = __ldg(src + ia * ffh);
-      if (ib >= 0) sb[k] = __ldg(src + ib * ffh);
+      const float2 *src = p.S + (long long)(t * p.nzS + zs) * NN * ss + 4 * kq + e;
+      if (ia >= 0) sa[k] = __ldg(src + ia * ss);
+      if (ib >= 0) sb[k] = __ldg(src + ib * ss);
     }
 #pragma unroll
     for (int k = 0; k < U; k++) {
@@ -359,8 +359,10 @@ __device__ __forceinline__ void mac_row(const float4 *row, const int (&off)[PPT]
 
 // Threads: `cw` warps side by side cover the channel pairs (PPT per lane), `H`
 // row shares of such warps take alternate rows of a chunk.
+// (At one frame shared memory allows three CTAs: asking for four took registers
+// from the row loop, 2 to 10 % of the forward time.)
 template <int TF, int TH> struct MacOcc {
-  static constexpr int v = TH == 128 ? (TF == 1 ? 4 : (TF == 2 ? 3 : 2)) : (TF == 1 ? 2 : 1);
+  static constexpr int v = TH == 128 ? (TF <= 2 ? 3 : 2) : (TF == 1 ? 2 : 1);
 };
 
 // One CTA = one frequency quad {(uy, ux), (ux, uy)} and a group of planes.
@@ -384,11 +386,11 @@ template <int TF, int TH> struct MacOcc {
 // operands four times, four pairs would keep 64 accumulators a lane).  With three
 // and four frames the FMAs bound it (registers allow two CTAs per SM).
 // Measured (GB300, Nnum 15, sum of the launches of a projection; complex form
-// first): 1005 x 1005 px, 41 planes, one frame: back 2776 -> 1844 us (3.7 -> 5.6
-// TB/s), forward 3006 -> 1862 us (2152 with the operand tables built between
+// first): 1005 x 1005 px, 41 planes, one frame: back 2776 -> 1704 us (3.7 -> 6.0
+// TB/s), forward 3006 -> 1789 us (290 more with the operand tables built between
 // planes from staged spectra); 437 x 608 px, 31 planes, three frames: back
-// 3202 -> 1209 us; 450 x 450 px, 31 planes, four frames a launch: forward
-// 477 -> 207 us, back 462 -> 213 us a launch.
+// 3202 -> 1107 us; 450 x 450 px, 31 planes, four frames a launch: forward
+// 477 -> 202 us, back 462 -> 203 us a launch.
 // The stored rows stream through a ring of shared-memory stages filled by
 // bulk copies (crossing plane boundaries).  Forward projection accumulates the
 // planes of the group (the group sums are added by the inverse transform), and
@@ -430,7 +432,6 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>
   const int hb0 = 2 * kq - ux;                   // first half block of the quad
   const int nhalf = diag ? 1 : 2;
   const bool selfp0 = (uy == 0) || (2 * uy == p.f), selfp1 = (ux == 0) || (2 * ux == p.f);
-  const int ffh = p.f * p.fh;
   const int z0 = blockIdx.y * p.zgroup;
   const int z1 = min(z0 + p.zgroup, p.nz);
   const int nrq = nhalf * R;                     // stored rows of the quad per plane
@@ -472,9 +473,8 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>
   }
   for (int i = tid; i < 3 * R; i += blockDim.x) rowS[i] = p.rowS[i];
   for (int i = tid; i < z1 - z0; i += blockDim.x) s_plane[i] = p.planes[z0 + i];
-  const int fo[4] = {uy * p.fh + ux, (uy ? p.f - uy : 0) * p.fh + ux, ux * p.fh + uy, (ux ? p.f - ux : 0) * p.fh + uy};
   __syncthreads();   // barriers initialised, row tables staged
-  build_sv<TF>(sv0, p, FWD ? z0 : 0, rowS, nhalf, selfp0, selfp1, fo, tid, blockDim.x);
+  build_sv<TF>(sv0, p, FWD ? z0 : 0, rowS, nhalf, selfp0, selfp1, kq, tid, blockDim.x);
   __syncthreads();
 
   if (HELP && warp == nwarps) {
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>
     for (int zl = 1; zl < z1 - z0; zl++) {
       const int b = zl & 1;
       if (zl > 1 && !mbar_wait(svfree + b, ((zl >> 1) - 1) & 1, p.wait_ns)) break;   // the waiting warps report it
-      build_sv<TF>(sv0 + b * TF * svt, p, z0 + zl, rowS, nhalf, selfp0, selfp1, fo, lane, 32);
+      build_sv<TF>(sv0 + b * TF * svt, p, z0 + zl, rowS, nhalf, selfp0, selfp1, kq, lane, 32);
       mbar_arrive(svfull + b);
     }
     __syncthreads();   // the streaming warps' last barrier
@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>
     const int zi = z0 + zl;
     if (FWD && !HELP && ch == 0 && zl > 0) {
       bar_sync(nthreads);   // every warp is done with plane zi - 1
-      build_sv<TF>(sv0, p, zi, rowS, nhalf, selfp0, selfp1, fo, tid, nthreads);
+      build_sv<TF>(sv0, p, zi, rowS, nhalf, selfp0, selfp1, kq, tid, nthreads);
       bar_sync(nthreads);
     }
     if (*abortf) dead = true;
@@ -590,26 +590,29 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>
         bar_sync(nthreads);
       }
       if (!dead) {
-        const int nside = diag ? 1 : 2;
+        // (back projection: two lanes write a channel's 32 bytes of the quad)
         const int nt = min(TF, p.T);
-        for (int idx = tid; idx < nt * nside * NN; idx += nthreads) {
-          const int q = idx % NN, ts = idx / NN;
-          const int t = ts / nside, s = ts - t * nside;
+        for (int idx = tid; idx < nt * 2 * NN; idx += nthreads) {
+          const int s = idx & 1, tq = idx >> 1;
+          const int t = tq / NN, q = tq - t * NN;
+          if (diag && s) continue;                   // the other side is the same frequency pair
           const float2 *o = outs + (size_t)(t * 2 + s) * NN2 + q;
           float2 u = o[0], v = o[NN];
-          if (diag) {                                // the other side is the same frequency pair
+          if (diag) {
             const float2 u1 = o[NN2], v1 = o[NN2 + NN];
             u.x += u1.x; u.y += u1.y; v.x += v1.x; v.y += v1.y;
           }
-          const int oy = s ? ux : uy, ox = s ? uy : ux;
-          const long long obase = FWD ? ((long long)(blockIdx.y * p.T + t) * NN) * ffh
-                                      : ((long long)(t * p.nzo + zi) * NN) * ffh;
-          float2 *op = p.O + obase + (long long)q * ffh + ox;
           if (s ? selfp1 : selfp0) {
-            op[oy * p.fh] = make_float2(u.x + v.x, u.y + v.y);
-          } else {
+            u.x += v.x; u.y += v.y;
+          }
+          if (FWD) {                                 // row order
+            const int oy = s ? ux : uy;
+            float2 *op = reinterpret_cast<float2 *>(p.O) +
+                         ((long long)(blockIdx.y * p.T + t) * NN + q) * (p.f * p.fh) + (s ? uy : ux);
             op[oy * p.fh] = u;
-            op[(p.f - oy) * p.fh] = v;
+            if (!(s ? selfp1 : selfp0)) op[(p.f - oy) * p.fh] = v;
+          } else {                                   // quad order
+            p.O[(((long long)(t * p.nzo + zi) * NN + q) * p.nquads + kq) * 2 + s] = make_float4(u.x, u.y, v.x, v.y);
           }
         }
       }
