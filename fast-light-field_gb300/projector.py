@@ -228,7 +228,10 @@ class Projector_gb300(Projector_base):
         img = self.asnative(projection)
         T, Y, X = img.shape
         self._prepare(ctx, Y, X, hMatrix)
-        vol = torch.zeros((hMatrix.numZ, T, Y, X), dtype=torch.float32, device=self._dev())
+        # the library writes every pixel of the listed planes; only the others need zeros
+        # (filling the whole volume took 9 of 46 us of the smallest call)
+        make = torch.empty if len(plist) == hMatrix.numZ else torch.zeros
+        vol = make((hMatrix.numZ, T, Y, X), dtype=torch.float32, device=self._dev())
         ctx.backward(img, vol, T, Y, X, None if len(plist) == hMatrix.numZ else plist,
                      stream=self._stream())
         if rlUpdateFunc is not None:
