@@ -726,13 +726,13 @@ __global__ void __launch_bounds__(128) k_conv3d_tc16(ConvParams p, int tiles_x, 
 // and out[z][y0+r][x] = sum over (dz, dy) of D[z-1+dz][r+dy][x][dz*3+dy], so a
 // slab of R+2 input rows costs 3 (R+2) MMAs for R output rows instead of 9 R.
 //   warp 0     producer: one thread issues the TMA loads;
-//   warps 1-2  MMA issuers: one thread each issues the 9 MMAs of half of the
-//              rows per slab, then commits to the slab's accumulator barrier
-//              and to its shared-memory slot; before a slab's MMAs it tests
-//              the next slab's barriers without blocking, so that test's
-//              latency overlaps the MMAs (a blocking wait follows only if a
-//              phase was not complete yet);
-//   warps 3-10 epilogue: warp w reads TMEM lane quarter w % 4 (tcgen05.ld)
+//   MMA issuers (up to four warps, one thread each): take the slabs in turn,
+//              issue all MMAs of a slab, then commit to the slab's accumulator
+//              barrier and to its shared-memory slot; before a slab's MMAs a
+//              thread tests its next slab's barriers without blocking, so that
+//              test's latency overlaps the MMAs (a blocking wait follows only
+//              if a phase was not complete yet);
+//   the last 8 warps: epilogue, warp w reads TMEM lane quarter w % 4 (tcgen05.ld)
 //              for 8 of the 16 output channels, sums the three z terms, then
 //              bias / ReLU / mask and BF16 stores, or with HEAD the clamped,
 //              scaled start volume from output channel 0.  With POOL it also
@@ -749,6 +749,16 @@ struct Tma16Grid {   // work items: [B][zchunks][yblocks][xsegs] columns of R x 
 };
 
 constexpr int TMA16_NACC = 5;   // TMEM accumulator slots (R x 3 CO columns each)
+
+// MMA-issuing threads for a ring of S slabs.  The slabs are dealt to them in turn, so that one
+// thread's barrier waits (about 85 cycles even when the phase is complete) pass while the others
+// issue: 16 -> 16 at 24 x 456 x 456 takes 84.6 us with four, against 102 us with two threads that
+// shared every slab's rows (106 with two taking alternate slabs, 147 with one).  A barrier's phase is
+// told from the one two phases before it by its parity alone, so a thread may only wait for slab n
+// once slab n - S (the slab ring) and n - 2 NACC (the accumulator ring) are known complete: they
+// divide S, so that the same thread handled slab n - S, and there are at most NACC of them.
+__host__ __device__ constexpr int tma16_issuers(int S) { return S % 4 == 0 ? 4 : S % 3 == 0 ? 3 : S % 2 == 0 ? 2 : 1; }
+__host__ __device__ constexpr int tma16_threads(int S) { return 32 * (1 + tma16_issuers(S) + 8); }
 
 namespace {
 
@@ -830,7 +840,7 @@ __device__ __forceinline__ void head_rows(float (&o)[RH], const float (&v)[RH + 
 }
 
 template <int CI, int CO, int R, int S, bool HEAD, bool SW32, bool X1 = false, bool POOL = false>
-__global__ void __launch_bounds__(352, 1)
+__global__ void __launch_bounds__(tma16_threads(S), 1)
     k_conv3d_tma16(const __grid_constant__ CUtensorMap tx, ConvParams p, HeadOut h, Tma16Grid g) {
   extern __shared__ __align__(1024) unsigned char smem[];
   constexpr int PYH = R + 2, NACC = TMA16_NACC;
@@ -844,7 +854,8 @@ __global__ void __launch_bounds__(352, 1)
   static_assert(!(HEAD && X1), "the head is a full 3x3x3 convolution");
   static_assert(!POOL || (CO == 16 && R == 2 && !HEAD && !X1),
                 "the pooled output is for 16 output channels and two rows per item");
-  constexpr int NISS = (HEAD ? PYH : R) % 2 == 0 ? 2 : 1;   // MMA-issuing threads (warps 1 .. NISS)
+  constexpr int NISS = tma16_issuers(S);      // MMA-issuing threads (warps 1 .. NISS)
+  static_assert(S % NISS == 0 && NISS <= NACC, "see tma16_issuers");
   constexpr int CH = CO / 2;                  // output channels per epilogue warp
   static_assert((CI == 16 || CI == 32) && (CO == 16 || CO == 32), "16 or 32 channels in and out");
   static_assert(SW32 || CI == 16, "the unswizzled slab layout is for 16 input channels");
@@ -900,10 +911,10 @@ __global__ void __launch_bounds__(352, 1)
   if (tid == 0) {
     for (int k = 0; k < S; k++) {
       net_mbar_init(full(k), 1);
-      net_mbar_init(empty(k), NISS);
+      net_mbar_init(empty(k), 1);
     }
     for (int k = 0; k < NACC; k++) {
-      net_mbar_init(tfull(k), NISS);
+      net_mbar_init(tfull(k), 1);
       net_mbar_init(tempty(k), 256);
     }
     net_mbar_init(fin, NISS);
@@ -951,12 +962,11 @@ __global__ void __launch_bounds__(352, 1)
         }
       }
     }
-  } else if (warp <= 2) {
-    if (lane == 0 && warp <= NISS) {
-      // ---- MMA issuers: warp 1 + j takes rows j*RR/NISS .. (j+1)*RR/NISS - 1 (output rows, or for
-      // the head input rows) ----
-      constexpr int RI = (HEAD ? PYH : R) / NISS;
-      const int r0 = (warp - 1) * RI;
+  } else if (warp <= NISS) {
+    if (lane == 0) {
+      // ---- MMA issuers: warp 1 + j takes the slabs n = j, j + NISS, ... (output rows, or for the
+      // head input rows) ----
+      constexpr int RI = HEAD ? PYH : R;
       // instruction descriptor: F32 accumulate, BF16 A and B, both K-major, N = 3 CO, M = 128
       const uint32_t idesc =
           (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NN >> 3) << 17) | ((128u >> 4) << 24);
@@ -975,17 +985,18 @@ __global__ void __launch_bounds__(352, 1)
         int b, zlo, nz, y0, x0;
         decode(it, b, zlo, nz, y0, x0);
         for (int k = 0; k < nz + 2; k++, n++) {
+          if (n % NISS != (uint32_t)(warp - 1)) continue;
           const uint32_t acc = n % NACC;
           ok = (pre_full & pre_empty) ||
                (role_wait(full(n % S), (n / S) & 1, abort_s, 5) &&
                 (n < NACC || role_wait(tempty(acc), ((n / NACC) - 1) & 1, abort_s, 6)));
           if (!ok) break;
           {
-            // test slab n+1's barriers now, without blocking: the results are read at the next slab,
-            // so their latency overlaps this slab's MMAs (a blocking wait follows only if a phase
-            // was not yet complete).  A phase seen complete stays complete until this thread's own
-            // commits let the slot be refilled.
-            const uint32_t n1 = n + 1;
+            // test the barriers of this thread's next slab now, without blocking: the results are read
+            // there, so their latency overlaps this slab's MMAs (a blocking wait follows only if a
+            // phase was not yet complete).  A phase seen complete stays complete until this thread's
+            // own commits let the slot be refilled.
+            const uint32_t n1 = n + NISS;
             pre_full = mbar_test(full(n1 % S), (n1 / S) & 1);
             pre_empty = n1 < NACC ? 1u : mbar_test(tempty(n1 % NACC), ((n1 / NACC) - 1) & 1);
           }
@@ -1008,8 +1019,8 @@ __global__ void __launch_bounds__(352, 1)
                 for (int r = 0; r < RI; r++) {
                   const uint64_t ad = ((uint64_t)a_hi << 32) |
                                       (uint64_t)(al + kh * (PLANE >> 4) +
-                                                 (uint32_t)(((r0 + r + dy) * PXW + dx) * VOX));
-                  umma_f16(dcol + (r0 + r) * NN, ad, bd, idesc, (blk > 0 || kh > 0) ? 1u : 0u);
+                                                 (uint32_t)(((r + dy) * PXW + dx) * VOX));
+                  umma_f16(dcol + r * NN, ad, bd, idesc, (blk > 0 || kh > 0) ? 1u : 0u);
                 }
               }
             }
@@ -1020,8 +1031,8 @@ __global__ void __launch_bounds__(352, 1)
       }
     }
   } else {
-    // ---- epilogue: warps 3..10; warp w owns TMEM lane quarter w % 4 and output channels CH*hf .. ----
-    const int qd = warp & 3, hf = (warp - 3) >> 2;
+    // ---- epilogue: the last 8 warps; warp w owns TMEM lane quarter w % 4 and output channels CH*hf .. ----
+    const int qd = warp & 3, hf = (warp - 1 - NISS) >> 2;
     const uint32_t lane_base = (uint32_t)(qd * 32) << 16;
     float bias[CH];
 #pragma unroll
@@ -1034,11 +1045,13 @@ __global__ void __launch_bounds__(352, 1)
       const int x = x0 + qd * 32 + lane;
       float pacc[POOL ? CH : 1];   // POOL: the 2x2x2 average of the output, summed over a plane pair
       for (int i = 0; i < nz; i++) {
-        // output plane z = zlo + i reads slabs n+i (dz 0), n+i+1 (dz 1), n+i+2 (dz 2); each issuer's
-        // commits complete in order, so slab n+i+2's barrier covers the other two
-        const uint32_t m = n + i + 2;
+        // output plane z = zlo + i reads slabs n+i (dz 0), n+i+1 (dz 1), n+i+2 (dz 2); the issuers'
+        // commits complete in any order, so the first plane waits for all three
+        bool here = true;
+        for (uint32_t m = n + i + (i ? 2 : 0); m <= n + i + 2 && here; m++)
+          here = role_wait(tfull(m % NACC), (m / NACC) & 1, abort_s, 7);
         // tcgen05.ld is .sync.aligned: the whole warp takes one decision
-        if (!__all_sync(0xffffffffu, role_wait(tfull(m % NACC), (m / NACC) & 1, abort_s, 7) ? 1 : 0)) {
+        if (!__all_sync(0xffffffffu, here ? 1 : 0)) {
           ok = false;
           break;
         }
@@ -1857,7 +1870,7 @@ static cudaError_t launch_tma16(const ConvParams &p, const HeadOut &h, cudaStrea
   g.zchunks = (p.Z + g.zc - 1) / g.zc;
   g.items = (long long)p.B * g.zchunks * g.yblocks * g.xsegs;
   const unsigned grid = (unsigned)(g.items < sms ? g.items : sms);
-  FLF_NET_LAUNCH(k_conv3d_tma16<CI, CO, R, S, HEAD, SW32, X1, POOL><<<grid, 352, SMEM, s>>>(map, p, h, g));
+  FLF_NET_LAUNCH(k_conv3d_tma16<CI, CO, R, S, HEAD, SW32, X1, POOL><<<grid, tma16_threads(S), SMEM, s>>>(map, p, h, g));
   return cudaGetLastError();
 }
 
@@ -2400,7 +2413,7 @@ cudaError_t launch_conv3d(ConvParams p, long long ws_elems, cudaStream_t s) {
   if (p.Ci == 32 && p.Co == 16)
     return g_conv16_tc == 2 ? launch_tma16<32, 16, 2, 4, false, true>(p, HeadOut{}, s) : launch_tiled<32, 16>(p, s);
   if (p.Ci == 32 && p.Co == 32)
-    return g_conv16_tc == 2 ? launch_tma16<32, 32, 1, 5, false, true>(p, HeadOut{}, s) : launch_tiled<32, 32>(p, s);
+    return g_conv16_tc == 2 ? launch_tma16<32, 32, 1, 6, false, true>(p, HeadOut{}, s) : launch_tiled<32, 32>(p, s);
   if (p.wp && g_conv_wide_tc) {
     bool done = false;
     const cudaError_t e = launch_wide_tc(p, ws_elems, s, done);
