@@ -37,6 +37,7 @@
 //                     ReLU mask, MSE loss gradient, Adam, bead rendering.
 #include "flf_internal.cuh"
 
+#include <algorithm>
 #include <atomic>
 
 #include <cuda.h>
@@ -1895,10 +1896,15 @@ static cudaError_t launch_tma16(const ConvParams &p, const HeadOut &h, cudaStrea
 //           accumulator buffers (nM x CO <= 256 columns each); the issuing
 //           thread moves only the start-address words of the descriptors.
 //   warp 0      slab producer (one thread);
-//   warp 1      MMA issuer (one thread), TMEM allocation;
+//   warps 1, 3, 8, 9  MMA issuers (one thread and one M tile each); warp 1
+//               allocates TMEM;
 //   warp 2      B producer (one thread);
 //   warps 4-7   epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31 of every
 //               M tile, adds the bias, ReLU / mask, stores BF16.
+// One thread issues an MMA in 62 cycles at best, more with the waits between:
+// with one issuer for all M tiles a weight block took 270 to 320 cycles whatever
+// it fed; with one per M tile 64 -> 64 at 6 x 114 x 114 went from 41.4 to 27.2 us,
+// 128 -> 128 at 3 x 57 x 57 from 29.0 to 23.4.
 // Items are dealt round-robin to persistent CTAs (one per SM); the epilogue of
 // an item overlaps the MMAs of the next.  Every mbarrier wait is bounded; a
 // give-up sets g_net_err and a shared abort flag, and the CTA drains its copies
@@ -1916,9 +1922,11 @@ struct WideGrid {
 constexpr int WIDE_SB_MAX = 64;      // B block ring: barriers for at most this many blocks
 constexpr int WIDE_SB = 12;          // taps of B blocks in flight at most
 constexpr int WIDE_ACC_COLS = 256;   // columns of one TMEM accumulator buffer
+constexpr int WIDE_ISS = 4;          // MMA issuers, one M tile each (warps 1, 3, 8, 9)
+constexpr int WIDE_THREADS = 320;
 
 template <int CI, int CO>
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(WIDE_THREADS, 1)
     k_conv3d_wide(const __grid_constant__ CUtensorMap tx, ConvParams p, const bf16 *__restrict__ wp, WideGrid g) {
   extern __shared__ __align__(1024) unsigned char smem[];
   constexpr int KC = CI < 64 ? CI : 64;   // input channels of one chunk
@@ -1957,15 +1965,15 @@ __global__ void __launch_bounds__(256, 1)
   if (tid == 0) {
     for (int k = 0; k < 2; k++) {
       net_mbar_init(sfull(k), 1);
-      net_mbar_init(sempty(k), 1);
-      net_mbar_init(afull(k), 1);
+      net_mbar_init(sempty(k), WIDE_ISS);
+      net_mbar_init(afull(k), WIDE_ISS);
       net_mbar_init(aempty(k), 4);
     }
     for (uint32_t k = 0; k < SB; k++) {
       net_mbar_init(bfull(k), 1);
-      net_mbar_init(bempty(k), 1);
+      net_mbar_init(bempty(k), WIDE_ISS);
     }
-    net_mbar_init(fin, 1);
+    net_mbar_init(fin, WIDE_ISS);
     *abort_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");   // visible to TMA and the MMAs
   }
@@ -2000,6 +2008,7 @@ __global__ void __launch_bounds__(256, 1)
     return z + dz >= 0 && z + dz < p.Z && (dz1 == 2 || dz == dz1);
   };
 
+  const int iss = warp == 1 ? 0 : warp == 3 ? 1 : warp == 8 ? 2 : warp == 9 ? 3 : -1;
   uint32_t nslab = 0, nbb = 0;   // slab chunks / B blocks issued (producers)
   if (warp == 0) {
     if (lane == 0) {
@@ -2059,9 +2068,10 @@ __global__ void __launch_bounds__(256, 1)
         if (!ok) break;
       }
     }
-  } else if (warp == 1) {
+  } else if (iss >= 0) {
     if (lane == 0) {
-      // ---- MMA issuer ----
+      // ---- MMA issuers: M tile `iss` each (those past nM only pass the barriers on) ----
+      const int m0 = iss;
       // instruction descriptor: F32 accumulate, BF16 A and B, both K-major, N = CO, M = 128
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(CO >> 3) << 17) | ((128u >> 4) << 24);
       // operand descriptors: only the start-address field (low word, 16-byte units) moves.
@@ -2073,9 +2083,10 @@ __global__ void __launch_bounds__(256, 1)
       const uint32_t a_lo0 = (uint32_t)a0d, a_hi = (uint32_t)(a0d >> 32);
       const uint32_t b_lo0 = (uint32_t)b0d, b_hi = (uint32_t)(b0d >> 32);
       const uint32_t a_row = SW ? 8u : 1u, a_ks = SW ? 2u : 2u * (LBO >> 4), a_slot = SLOT >> 4;
+      const uint32_t a_dy = (uint32_t)(g.Xp - 3) * a_row;   // from past the last dx to the next dy
       const uint32_t a_m = 128u * a_row, b_ks = (2u * CO * 16u) >> 4, b_slot = SLOTB >> 4, b_tap = TB >> 4;
       const int nM = g.nM;
-      uint32_t ns = 0, nb = 0, li = 0;
+      uint32_t ns = 0, nb = 0, li = 0, pre = 0;
       bool ok = true;
       for (long long it = blockIdx.x; it < g.items && ok; it += gridDim.x, li++) {
         int b, z, y0, dz1;
@@ -2096,27 +2107,33 @@ __global__ void __launch_bounds__(256, 1)
               ok = false;
               break;
             }
-            const uint32_t a_c = a_lo0 + sl * a_slot;
+            uint32_t a_t = a_lo0 + sl * a_slot + m0 * a_m;   // this thread's tile at tap (dy, dx)
+            int dx = 0;
             for (int t9 = 0; t9 < 9; t9 += TPS) {
               const uint32_t bs = nb % SB;
-              if (!role_wait(bfull(bs), (nb / SB) & 1, abort_s, 25)) {
+              if (!pre && !role_wait(bfull(bs), (nb / SB) & 1, abort_s, 25)) {
                 ok = false;
                 break;
               }
+              // the next slot's barrier, tested without blocking while this slot's MMAs issue
+              pre = mbar_test(bfull((nb + 1) % SB), ((nb + 1) / SB) & 1);
               tc_fence_after();
+              uint32_t b_t = b_lo0 + bs * b_slot;
               for (int u = 0; u < TPS; u++) {
-                const int t = t9 + u;
-                const uint32_t a_t = a_c + (uint32_t)((t / 3) * g.Xp + (t % 3)) * a_row;
-                const uint32_t b_t = b_lo0 + bs * b_slot + u * b_tap;
+                if (m0 < nM) {
 #pragma unroll
-                for (int ks = 0; ks < KS; ks++) {
-                  const uint64_t bd = ((uint64_t)b_hi << 32) | (b_t + ks * b_ks);
-#pragma unroll
-                  for (int m = 0; m < 4; m++)
-                    if (m < nM)
-                      umma_f16(dcol + m * CO, ((uint64_t)a_hi << 32) | (a_t + ks * a_ks + m * a_m), bd, idesc, acc);
-                  acc = 1;
+                  for (int ks = 0; ks < KS; ks++) {
+                    umma_f16(dcol + m0 * CO, ((uint64_t)a_hi << 32) | (a_t + ks * a_ks),
+                             ((uint64_t)b_hi << 32) | (b_t + ks * b_ks), idesc, acc);
+                    acc = 1;
+                  }
                 }
+                a_t += a_row;
+                if (++dx == 3) {
+                  dx = 0;
+                  a_t += a_dy;
+                }
+                b_t += b_tap;
               }
               umma_commit(bempty(bs));   // the slot's B blocks are free once these MMAs complete
               nb++;
@@ -2130,8 +2147,8 @@ __global__ void __launch_bounds__(256, 1)
         umma_commit(afull(ab));
       }
     }
-  } else if (warp >= 4) {
-    // ---- epilogue ----
+  } else {
+    // ---- epilogue (warps 4-7) ----
     const int qd = warp & 3;
     const uint32_t lane_base = (uint32_t)(qd * 32) << 16;
     uint32_t li = 0;
@@ -2212,7 +2229,7 @@ __global__ void __launch_bounds__(256, 1)
         if (!net_mbar_wait(bfull(sl), (last / SB) & 1, 1000000000ULL)) atomicExch(&g_net_err, 28);
       }
   }
-  if (warp == 1 && lane == 0) {
+  if (iss >= 0 && lane == 0) {
     // every MMA issued has completed before the accumulators are released
     umma_commit(fin);
     if (!net_mbar_wait(fin, 0, 1000000000ULL)) atomicExch(&g_net_err, 29);
@@ -2299,32 +2316,43 @@ static cudaError_t launch_wide(ConvParams p, long long ws_elems, cudaStream_t s,
   const long long Mv = (long long)p.B * p.Z * p.Y * p.X;
   const bool can_split = p.ws && ws_elems >= 3 * Mv * CO;
   // work-unit shape: M tiles per item forced (modes 2..5) or chosen, and whether each item
-  // splits over its three input planes (FP32 partials in ws, summed by k_conv3d_finish): the
-  // least estimated time, ties to more M tiles.  Measured: a unit's time follows its weight
-  // blocks (~320 cycles each, whatever the number of M tiles they feed; ~15 % less with three
-  // taps per ring slot), plus a fixed cost per unit; a split also writes and reads three FP32
-  // partial sets (~3000 bytes per cycle) and launches the finish kernel.
+  // splits over its three input planes (FP32 partials in ws, summed by k_conv3d_finish).  The
+  // split changes the order of a sum, so it has a rule of its own, which a faster way to issue
+  // the MMAs does not move: the least of 320 cycles a weight block (272 with three taps per ring
+  // slot) and a fixed cost per unit, with three FP32 partial sets written and read (~3000 bytes per
+  // cycle) and the finish kernel's launch where split, ties to more M tiles.  The M tiles change no
+  // bits: among the shapes with that split the least estimated time.  Measured (64 -> 64, one to
+  // four M tiles with an issuer each): a weight block takes about 100 cycles and one MMA's time per
+  // M tile (the A and B operand reads, 32 + CO/4, or the math, CO/2), plus a fixed cost per unit.
   WideGrid g{};
   size_t smem = 0;
   bool found = false;
-  double best = 0;
-  for (int nM = 1; nM <= 4; nM++) {
-    if (g_conv_wide_tc >= 2 && nM != g_conv_wide_tc - 1) continue;
-    WideGrid c{};
-    size_t sm = 0;
-    if (!wide_shape(CI, CO, p.Y, p.X, nM, c, sm)) continue;
-    for (int sp = 1; sp <= (can_split ? 3 : 1); sp += 2) {
-      c.splits = sp;
-      c.items = (long long)p.B * p.Z * c.nyb * sp;
-      const double waves = (double)((c.items + sms - 1) / sms);
-      const double blocks = 27.0 * (CI / 16) / sp;
-      const double partials = sp > 1 ? 4000.0 + 2.0 * 3.0 * (double)Mv * CO * 4.0 / 3000.0 : 0.0;
-      const double cost = waves * (blocks * (c.tps == 3 ? 272.0 : 320.0) + 3000.0) + partials;
-      if (!found || cost <= best) {
-        found = true;
-        best = cost;
-        g = c;
-        smem = sm;
+  int split = 1;
+  for (int pass = 0; pass < 2; pass++) {
+    double best = -1;
+    for (int nM = 1; nM <= 4; nM++) {
+      if (g_conv_wide_tc >= 2 && nM != g_conv_wide_tc - 1) continue;
+      WideGrid c{};
+      size_t sm = 0;
+      if (!wide_shape(CI, CO, p.Y, p.X, nM, c, sm)) continue;
+      for (int sp = 1; sp <= (can_split ? 3 : 1); sp += 2) {
+        c.splits = sp;
+        c.items = (long long)p.B * p.Z * c.nyb * sp;
+        const double waves = (double)((c.items + sms - 1) / sms);
+        const double blocks = 27.0 * (CI / 16) / sp;
+        if (pass == 0) {
+          const double partials = sp > 1 ? 4000.0 + 2.0 * 3.0 * (double)Mv * CO * 4.0 / 3000.0 : 0.0;
+          const double cost = waves * (blocks * (c.tps == 3 ? 272.0 : 320.0) + 3000.0) + partials;
+          if (best < 0 || cost <= best) best = cost, split = sp;
+        } else if (sp == split) {
+          const double cost = waves * (blocks * (100.0 + std::max(32.0 + CO / 4.0, CO / 2.0) * c.nM) + 3000.0);
+          if (best < 0 || cost <= best) {
+            found = true;
+            best = cost;
+            g = c;
+            smem = sm;
+          }
+        }
       }
     }
   }
@@ -2356,7 +2384,7 @@ static cudaError_t launch_wide(ConvParams p, long long ws_elems, cudaStream_t s,
   }
   const unsigned grid = (unsigned)(g.items < sms ? g.items : sms);
   p.splits = g.splits;
-  FLF_NET_LAUNCH(k_conv3d_wide<CI, CO><<<grid, 256, sm_launch, s>>>(map, p, p.wp, g));
+  FLF_NET_LAUNCH(k_conv3d_wide<CI, CO><<<grid, WIDE_THREADS, sm_launch, s>>>(map, p, p.wp, g));
   if (g.splits > 1) FLF_NET_LAUNCH(k_conv3d_finish<<<grid_for(Mv * CO / 8, 256), 256, 0, s>>>(p, Mv));
   return cudaGetLastError();
 }
