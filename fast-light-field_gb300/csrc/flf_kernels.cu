@@ -914,12 +914,16 @@ cudaError_t launch_irfft2(const Irfft2Params &p, cudaStream_t s) {
 int mac_max_frames() { return 4; }
 
 // Warps side by side over the channel pairs, and row shares: about 128 threads
-// per unit of p.split, at most 256.  Two pairs per lane from 33 pairs on.
+// per unit of p.split, at most 256; a small Nnum's single column warp keeps a unit's
+// rows to itself, since a CTA then has few rows and its sums cost more to join than
+// to make (Nnum 5, 31 planes of 250 x 300 px, four frames: back 129 us a launch with
+// four shares, 76 with two, 58 with one; Nnum 7, 25 planes, one frame 44, 31, 31).
+// Two pairs per lane from 33 pairs on.
 MacThreads mac_threads(const Layout &L, int split) {
   MacThreads t;
   t.ppt = L.NP > 32 ? 2 : 1;
   t.cw = (L.NP + 32 * t.ppt - 1) / (32 * t.ppt);
-  t.shares = std::max(1, std::min(4 * split / t.cw, 8 / t.cw));
+  t.shares = t.cw == 1 ? split : std::max(1, std::min(4 * split / t.cw, 8 / t.cw));
   return t;
 }
 
