@@ -18,6 +18,8 @@ using namespace flf;
 
 namespace {
 
+constexpr int kFan = 4;   // streams the transforms of a merged projection run on
+
 thread_local std::string g_create_error;
 
 struct Workspace {
@@ -39,8 +41,8 @@ struct Group {
   size_t spec() const { return (size_t)f * fh; }
   size_t qspec() const { return (size_t)4 * nquads; }
   std::vector<int> planes;    // plane ids of the group, ascending (slot = index)
-  int *d_ids = nullptr;       // device copy of `planes`
-  int *d_slots = nullptr;     // 0..n-1
+  int *d_ids = nullptr;       // device copy of `planes` (in Geometry::d_lists)
+  int *d_slots = nullptr;     // 0..n-1 (likewise)
 };
 
 struct Geometry {
@@ -50,6 +52,7 @@ struct Geometry {
                                  // (stages, chunk rows forward, backward, split); 0: context options
   std::vector<Group> groups;
   std::vector<int> plane_group, plane_slot;
+  int *d_lists = nullptr;     // plane ids of all groups, one after the other, then their slots
   bool built(int dir) const {
     for (const Group &g : groups)
       if (!g.built[dir]) return false;
@@ -99,6 +102,8 @@ struct flf_ctx {
   bool psf_released = false;
   cudaStream_t s2 = nullptr;     // the second stream, and the events that fork / chain / join it
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_chain = nullptr;
+  cudaStream_t s_fan[kFan - 1] = {};   // streams of the transforms of a merged projection
+  cudaEvent_t ev_fan[kFan - 1] = {};
   void *noalloc_scratch = nullptr;   // device address of the fixed scratch of flf_backward_noalloc
   int *h_err = nullptr;          // host-mapped flag set by bounded device waits
   int *d_err = nullptr;
@@ -234,10 +239,11 @@ int ensure_ws(flf_ctx *ctx, Workspace &w, size_t bytes) {
 
 void free_geometry(Geometry &G) {
   for (Group &g : G.groups) {
-    void *ptrs[] = {g.tw, g.tw64, g.P[0], g.P[1], g.d_ids, g.d_slots};
+    void *ptrs[] = {g.tw, g.tw64, g.P[0], g.P[1]};
     for (void *p : ptrs)
       if (p) cudaFree(p);
   }
+  if (G.d_lists) cudaFree(G.d_lists);
   G = Geometry();
 }
 
@@ -549,16 +555,24 @@ int prepare(flf_ctx *ctx, int Y, int X, int fft_size, int fp64) {
       tw64[k] = make_double2(std::cos(ang), std::sin(ang));
       tw[k] = make_float2((float)tw64[k].x, (float)tw64[k].y);
     }
-    std::vector<int> slots(g.planes.size());
-    for (size_t i = 0; i < slots.size(); i++) slots[i] = (int)i;
     CUDA_TRY(ctx, cudaMalloc(&g.tw, sizeof(float2) * f));
     CUDA_TRY(ctx, cudaMemcpy(g.tw, tw.data(), sizeof(float2) * f, cudaMemcpyHostToDevice));
     CUDA_TRY(ctx, cudaMalloc(&g.tw64, sizeof(double2) * f));
     CUDA_TRY(ctx, cudaMemcpy(g.tw64, tw64.data(), sizeof(double2) * f, cudaMemcpyHostToDevice));
-    CUDA_TRY(ctx, cudaMalloc(&g.d_ids, sizeof(int) * g.planes.size()));
-    CUDA_TRY(ctx, cudaMemcpy(g.d_ids, g.planes.data(), sizeof(int) * g.planes.size(), cudaMemcpyHostToDevice));
-    CUDA_TRY(ctx, cudaMalloc(&g.d_slots, sizeof(int) * slots.size()));
-    CUDA_TRY(ctx, cudaMemcpy(g.d_slots, slots.data(), sizeof(int) * slots.size(), cudaMemcpyHostToDevice));
+  }
+  {
+    std::vector<int> lists(2 * nz);
+    CUDA_TRY(ctx, cudaMalloc(&G.d_lists, sizeof(int) * lists.size()));
+    int at = 0;
+    for (Group &g : G.groups) {
+      g.d_ids = G.d_lists + at;
+      g.d_slots = G.d_lists + nz + at;
+      for (size_t i = 0; i < g.planes.size(); i++, at++) {
+        lists[at] = g.planes[i];
+        lists[nz + at] = (int)i;
+      }
+    }
+    CUDA_TRY(ctx, cudaMemcpy(G.d_lists, lists.data(), sizeof(int) * lists.size(), cudaMemcpyHostToDevice));
   }
   G.valid = true;
   return FLF_OK;
@@ -566,10 +580,21 @@ int prepare(flf_ctx *ctx, int Y, int X, int fft_size, int fp64) {
 
 // The planes one projection call works on, split by transform group:
 // for group g, n[g] planes with ids ids[g] (volume addressing) and slots
-// slots[g] (rows of the group's packed matrices), both device arrays.
+// slots[g] (rows of the group's packed matrices), both device arrays; those of
+// the groups follow one another, so a launch over all planes takes the first's.
 struct PlaneSet {
   std::vector<int> n;
   std::vector<const int *> ids, slots;
+  int groups() const {   // those with planes
+    int k = 0;
+    for (int v : n) k += v > 0;
+    return k;
+  }
+  int planes() const {
+    int k = 0;
+    for (int v : n) k += v;
+    return k;
+  }
 };
 
 int check_planes_arg(flf_ctx *ctx, const int *planes, int nplanes) {
@@ -609,13 +634,13 @@ int make_plane_set(flf_ctx *ctx, const int *planes, int nplanes, cudaStream_t s,
     ids[g].push_back(z);
     slots[g].push_back(G.plane_slot[z]);
   }
-  std::vector<int> host;   // per group: ids then slots
+  std::vector<int> host;   // ids of all groups, then their slots
   std::vector<int> off(ng);
   for (int g = 0; g < ng; g++) {
     off[g] = (int)host.size();
     host.insert(host.end(), ids[g].begin(), ids[g].end());
-    host.insert(host.end(), slots[g].begin(), slots[g].end());
   }
+  for (int g = 0; g < ng; g++) host.insert(host.end(), slots[g].begin(), slots[g].end());
   if (ctx->planes_user_cap < (int)host.size()) {
     if (ctx->d_planes_user) cudaFree(ctx->d_planes_user);
     ctx->d_planes_user = nullptr;
@@ -628,7 +653,7 @@ int make_plane_set(flf_ctx *ctx, const int *planes, int nplanes, cudaStream_t s,
   for (int g = 0; g < ng; g++) {
     ps.n[g] = (int)ids[g].size();
     ps.ids[g] = ctx->d_planes_user + off[g];
-    ps.slots[g] = ctx->d_planes_user + off[g] + ps.n[g];
+    ps.slots[g] = ctx->d_planes_user + nplanes + off[g];
   }
   return FLF_OK;
 }
@@ -688,9 +713,80 @@ void ws_needs(const flf_ctx *ctx, const PlaneSet &ps, int nt, bool fwd, size_t &
   }
 }
 
+// Whether a projection of nt frames runs all its transform groups in one
+// multiply-accumulate launch (their transforms side by side on several streams)
+// rather than group by group on two streams: one frame of three groups or more,
+// where every group's launch loses some 16 us to its last CTAs and the waits between
+// kernels add up.  With more frames the transforms are large enough to be worth
+// hiding behind another group's multiply-accumulate, and with two groups there is
+// one end to save.  Measured, forward, group by group and merged (Nnum 15): 450 px,
+// 21 planes in 5 groups 347 and 303 us, 31 planes 478 and 429; 675 px, 31 planes in 7
+// groups 898 and 799; 1005 px, 41 planes in 6 groups 2081 and 1998 (back 1964 and
+// 1961); 450 px, 11 planes in 3 groups 167 and 163; 5 planes in 2 groups 83 and 89.
+bool merge_groups(const PlaneSet &ps, int nt) {
+  const int k = ps.groups();
+  return nt == 1 && k >= 3 && k <= kMacMaxGroups;
+}
+
+// Planes per CTA of such a launch: about opt_ctas_per_sm CTAs per SM in all.
+int merged_zgroup(const flf_ctx *ctx, const PlaneSet &ps) {
+  long long units = 0;
+  for (size_t g = 0; g < ctx->geo.groups.size(); g++) units += (long long)ps.n[g] * ctx->geo.groups[g].nquads;
+  const long long target = (long long)ctx->opt_ctas_per_sm * std::max(1, ctx->num_sms);
+  return (int)std::min<long long>(kMacMaxZgroup, std::max(1LL, (units + target - 1) / target));
+}
+
+size_t slot_bytes(size_t b) { return (b + 255) / 256 * 256; }
+
+// Bytes of every workspace for a projection of nt frames over ps: spectra in and
+// out, channel-major volume side and image side (a set per group where merged).
+struct WsSizes {
+  size_t S = 0, O = 0, Cvol = 0, Cimg = 0;
+  void grow(const WsSizes &o) {
+    S = std::max(S, o.S); O = std::max(O, o.O); Cvol = std::max(Cvol, o.Cvol); Cimg = std::max(Cimg, o.Cimg);
+  }
+};
+int ws_slots(const flf_ctx *ctx);
+WsSizes ws_sizes(const flf_ctx *ctx, const PlaneSet &ps, int nt, bool fwd) {
+  WsSizes w;
+  const size_t cset = sizeof(float) * chan_set_floats(ctx), NN = ctx->L.NN;
+  w.Cimg = cset * nt;
+  if (!merge_groups(ps, nt)) {
+    size_t a, b, c;
+    ws_needs(ctx, ps, nt, fwd, a, b, c);
+    w.S = ws_slots(ctx) * slot_bytes(a); w.O = ws_slots(ctx) * slot_bytes(b); w.Cvol = ws_slots(ctx) * slot_bytes(c);
+    return w;
+  }
+  const int zg = merged_zgroup(ctx, ps);
+  for (size_t g = 0; g < ctx->geo.groups.size(); g++) {
+    const int n = ps.n[g];
+    if (!n) continue;
+    const size_t spec = sizeof(float2) * NN * ctx->geo.groups[g].spec(), qspec = sizeof(float2) * NN * ctx->geo.groups[g].qspec();
+    w.S += slot_bytes(fwd ? qspec * n : qspec);
+    w.O += slot_bytes(fwd ? spec * ((n + zg - 1) / zg) : qspec * n);
+    w.Cvol += cset * n;
+  }
+  if (fwd) w.Cimg = cset * ps.groups();
+  return w;
+}
+
+// The workspaces of a run of T frames in passes of TF.
+int ensure_workspaces(flf_ctx *ctx, const PlaneSet &ps, int T, int TF, bool fwd, bool bwd) {
+  WsSizes w;
+  for (int nt : {std::min(T, TF), T % TF}) {
+    if (!nt) continue;
+    if (fwd) w.grow(ws_sizes(ctx, ps, nt, true));
+    if (bwd) w.grow(ws_sizes(ctx, ps, nt, false));
+  }
+  int rc = ensure_ws(ctx, ctx->wsS, w.S);
+  if (rc == FLF_OK) rc = ensure_ws(ctx, ctx->wsO, w.O);
+  if (rc == FLF_OK) rc = ensure_ws(ctx, ctx->wsCvol, w.Cvol);
+  if (rc == FLF_OK) rc = ensure_ws(ctx, ctx->wsCimg, w.Cimg);
+  return rc;
+}
+
 // Workspace slots: one per stream the transform groups alternate over.
 int ws_slots(const flf_ctx *ctx) { return ctx->opt_streams > 1 ? 2 : 1; }
-size_t slot_bytes(size_t b) { return (b + 255) / 256 * 256; }
 
 // The second stream and its events (created on first use).
 int ensure_streams(flf_ctx *ctx) {
@@ -699,6 +795,32 @@ int ensure_streams(flf_ctx *ctx) {
   CUDA_TRY(ctx, cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
   CUDA_TRY(ctx, cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
   CUDA_TRY(ctx, cudaEventCreateWithFlags(&ctx->ev_chain, cudaEventDisableTiming));
+  for (int i = 0; i < kFan - 1; i++) {
+    CUDA_TRY(ctx, cudaStreamCreateWithFlags(&ctx->s_fan[i], cudaStreamNonBlocking));
+    CUDA_TRY(ctx, cudaEventCreateWithFlags(&ctx->ev_fan[i], cudaEventDisableTiming));
+  }
+  return FLF_OK;
+}
+
+// n launches side by side: launch i goes to st[i % kFan], all after what s holds
+// now; fan_in makes s wait for them.
+int fan_out(flf_ctx *ctx, cudaStream_t s, int n, cudaStream_t st[kFan]) {
+  for (int i = 0; i < kFan; i++) st[i] = s;
+  if (ctx->opt_streams < 2) return FLF_OK;
+  if (int rc = ensure_streams(ctx)) return rc;
+  CUDA_TRY(ctx, cudaEventRecord(ctx->ev_fork, s));
+  for (int i = 1; i < std::min(n, kFan); i++) {
+    st[i] = ctx->s_fan[i - 1];
+    CUDA_TRY(ctx, cudaStreamWaitEvent(st[i], ctx->ev_fork, 0));
+  }
+  return FLF_OK;
+}
+int fan_in(flf_ctx *ctx, cudaStream_t s, int n) {
+  if (ctx->opt_streams < 2) return FLF_OK;
+  for (int i = 1; i < std::min(n, kFan); i++) {
+    CUDA_TRY(ctx, cudaEventRecord(ctx->ev_fan[i - 1], ctx->s_fan[i - 1]));
+    CUDA_TRY(ctx, cudaStreamWaitEvent(s, ctx->ev_fan[i - 1], 0));
+  }
   return FLF_OK;
 }
 
@@ -780,10 +902,9 @@ int frames_per_pass(const flf_ctx *ctx) {
   return 1;
 }
 
-MacParams mac_params(const flf_ctx *ctx, const Group &G, int dir, int nt) {
+MacParams mac_params(const flf_ctx *ctx, int dir, int nt) {
   MacParams mp{};
-  mp.L = ctx->L; mp.f = G.f; mp.fh = G.fh; mp.fq = G.fq; mp.nkp = G.nkp; mp.nquads = G.nquads; mp.T = nt;
-  mp.P = (const float4 *)G.P[dir];
+  mp.L = ctx->L; mp.T = nt;
   mp.rowS = ctx->d_rowS;
   mac_shape(ctx, dir, nt, mp.stages, mp.chunk_rows, mp.split);
   mp.err = ctx->d_err;
@@ -792,22 +913,25 @@ MacParams mac_params(const flf_ctx *ctx, const Group &G, int dir, int nt) {
   return mp;
 }
 
+// Adds n planes (slots `planes`) of group G in z groups of zgroup planes.
+void mac_add_group(MacParams &mp, const Group &G, int dir, const int *planes, int n, int zgroup, const void *S, void *O) {
+  MacGroup &g = mp.g[mp.ngroups++];
+  g.f = G.f; g.fh = G.fh; g.nkp = G.nkp; g.nquads = G.nquads;
+  g.nz = n; g.zgroup = zgroup;
+  g.nzS = dir == FLF_DIR_FORWARD ? n : 1;
+  g.nzo = dir == FLF_DIR_FORWARD ? (n + zgroup - 1) / zgroup : n;
+  g.P = (const float4 *)G.P[dir]; g.planes = planes;
+  g.S = (const float2 *)S; g.O = (float4 *)O;
+}
+
 // One multiply-accumulate launch of group gi over all its planes for nt
 // frames, on the workspaces (flf_autotune's timing unit).
 cudaError_t mac_group_launch(flf_ctx *ctx, size_t gi, int dir, int nt, const PlaneSet &ps, int stages, int chunk,
                              int split, cudaStream_t s) {
   const Group &G = ctx->geo.groups[gi];
-  const int nplanes = ps.n[gi];
-  const int zg = zgroup_for(ctx, nplanes, G.nquads);
-  MacParams mp = mac_params(ctx, G, dir, nt);
+  MacParams mp = mac_params(ctx, dir, nt);
   mp.stages = stages; mp.chunk_rows = chunk; mp.split = split;
-  mp.planes = ps.slots[gi]; mp.nz = nplanes; mp.zgroup = zg;
-  mp.S = (const float2 *)ctx->wsS.p; mp.O = (float4 *)ctx->wsO.p;
-  if (dir == FLF_DIR_FORWARD) {
-    mp.nzS = nplanes; mp.nzo = (nplanes + zg - 1) / zg; mp.nzo_grid = mp.nzo;
-  } else {
-    mp.nzS = 1; mp.nzo = nplanes; mp.nzo_grid = (nplanes + zg - 1) / zg;
-  }
+  mac_add_group(mp, G, dir, ps.slots[gi], ps.n[gi], zgroup_for(ctx, ps.n[gi], G.nquads), ctx->wsS.p, ctx->wsO.p);
   return launch_mac(mp, dir == FLF_DIR_FORWARD, s);
 }
 
@@ -826,7 +950,7 @@ Rfft2Params rfft2_params(const flf_ctx *ctx, const Group &G, const float *chan, 
   const Geometry &Gm = ctx->geo;
   Rfft2Params rp{};
   rp.plan = G.plan; rp.N = ctx->N; rp.Y = Gm.Y; rp.X = Gm.X; rp.Ly = Gm.Ly; rp.Lx = Gm.Lx;
-  rp.nimg = nimg; rp.mode = 0; rp.chan = chan; rp.Lxp = channel_pitch(Gm.Lx);
+  rp.nimg = nimg; rp.mode = 0; rp.chan = chan; rp.nsum = 1; rp.Lxp = channel_pitch(Gm.Lx);
   rp.dst = dst; rp.twiddle = G.tw;
   return rp;
 }
@@ -844,7 +968,7 @@ MergeParams merge_params(const flf_ctx *ctx, const float *src, const int *planes
                          Strided out, Strided aux, Strided norm) {
   const Geometry &Gm = ctx->geo;
   MergeParams mg{};
-  mg.src = src; mg.nzo = nzo; mg.nsets = nzo * nt; mg.planes = planes;
+  mg.src = src; mg.nsum = 1; mg.nzo = nzo; mg.nsets = nzo * nt; mg.planes = planes;
   mg.N = ctx->N; mg.Y = Gm.Y; mg.X = Gm.X; mg.Ly = Gm.Ly; mg.Lx = Gm.Lx; mg.Lxp = channel_pitch(Gm.Lx);
   mg.epi = epi; mg.out = out; mg.aux = aux; mg.norm = norm;
   return mg;
@@ -853,13 +977,79 @@ MergeParams merge_params(const flf_ctx *ctx, const float *src, const int *planes
 // Bytes of nsets channel-major image sets.
 double chan_bytes(const flf_ctx *ctx, int nsets) { return 4.0 * chan_set_floats(ctx) * nsets; }
 
+// A channel-major image set [nt][NN][Ly][Lxp] as its consumers take it: the sum
+// of nsum sets `stride` floats apart, or num over that sum.
+struct ChanImg {
+  const float *p = nullptr;
+  int nsum = 1;
+  long long stride = 0;
+  const float *num = nullptr;
+};
+
+// Forward projection of frame t0 of vol, all groups in one multiply-accumulate
+// launch (merge_groups): their output sets side by side in `chan`, for the
+// consumer to add in group order.
+int forward_merged(flf_ctx *ctx, const float *vol, long long vol_sz, const PlaneSet &ps, int t0, float *chan,
+                   const float *num, ChanImg &out, cudaStream_t s) {
+  Geometry &Gm = ctx->geo;
+  const Layout &L = ctx->L;
+  const int NN = L.NN, Y = Gm.Y, X = Gm.X, nall = ps.planes(), ng = ps.groups();
+  const size_t cset = chan_set_floats(ctx);
+  float *cvol = (float *)ctx->wsCvol.p;
+  char *wS = (char *)ctx->wsS.p, *wO = (char *)ctx->wsO.p;
+  const int *ids = nullptr;
+  for (size_t gi = Gm.groups.size(); gi-- > 0;)
+    if (ps.n[gi]) ids = ps.ids[gi];
+  SplitParams sp = split_params(ctx, vol + (long long)t0 * Y * X, vol_sz, (long long)Y * X, ids, nall, 1, cvol);
+  LAUNCH(ctx, "k_split", chan_bytes(ctx, nall) + 4.0 * Y * X * nall, s, launch_split(sp, s));
+  MacParams mp = mac_params(ctx, FLF_DIR_FORWARD, 1);
+  const int zgroup = merged_zgroup(ctx, ps);
+  cudaStream_t st[kFan];
+  if (int rc = fan_out(ctx, s, ng, st)) return rc;
+  double bytes = 0;
+  int k = 0, at = 0;
+  for (size_t gi = 0; gi < Gm.groups.size(); gi++) {
+    const int n = ps.n[gi];
+    if (!n) continue;
+    const Group &G = Gm.groups[gi];
+    Rfft2Params rp = rfft2_params(ctx, G, cvol + at * cset, n * NN, wS);
+    const cudaStream_t sk = st[k % kFan];
+    LAUNCH(ctx, "k_rfft2", chan_bytes(ctx, n) + 8.0 * G.qspec() * NN * n, sk, launch_rfft2(rp, 0, sk));
+    mac_add_group(mp, G, FLF_DIR_FORWARD, ps.slots[gi], n, zgroup, wS, wO);
+    const int nzg = (n + zgroup - 1) / zgroup;
+    bytes += (double)n * G.nkp * L.nrow * L.RS * sizeof(float2) + 8.0 * NN * (G.qspec() * n + G.spec() * nzg);
+    wS += slot_bytes(sizeof(float2) * NN * G.qspec() * n);
+    wO += slot_bytes(sizeof(float2) * NN * G.spec() * nzg);
+    at += n;
+    k++;
+  }
+  if (int rc = fan_in(ctx, s, ng)) return rc;
+  LAUNCH(ctx, "k_mac_fwd", bytes, s, launch_mac(mp, true, s));
+  if (int rc = fan_out(ctx, s, ng, st)) return rc;
+  k = 0;
+  for (size_t gi = 0; gi < Gm.groups.size(); gi++) {
+    if (!ps.n[gi]) continue;
+    const Group &G = Gm.groups[gi];
+    Irfft2Params ip = irfft2_params(ctx, G, (const float2 *)mp.g[k].O, NN, chan + k * cset);
+    ip.sum_stride = (long long)(NN * G.spec()); ip.nsum = mp.g[k].nzo;
+    const cudaStream_t sk = st[k % kFan];
+    LAUNCH(ctx, "k_irfft2", 8.0 * G.spec() * NN * ip.nsum + chan_bytes(ctx, 1), sk, launch_irfft2(ip, sk));
+    k++;
+  }
+  out.p = chan; out.nsum = ng; out.stride = (long long)cset; out.num = num;
+  return fan_in(ctx, s, ng);
+}
+
 // Forward projection of frames [t0, t0+nt) of vol into the channel-major
 // image set `chan` ([nt][NN][Ly][Lxp]): each transform group is projected and
 // summed in Fourier space over its planes; the groups are added in the
 // channel-major domain.  The last group's pass zeroes the samples outside the
 // image and, with `num`, stores num / (H x) (the standard RL error image).
 int forward_chunk(flf_ctx *ctx, const float *vol, long long vol_sz, const PlaneSet &ps, int t0, int nt,
-                  float *chan, const float *num, cudaStream_t s) {
+                  float *chan, const float *num, ChanImg &out, cudaStream_t s) {
+  if (merge_groups(ps, nt)) return forward_merged(ctx, vol, vol_sz, ps, t0, chan, num, out, s);
+  out = ChanImg();
+  out.p = chan;
   Geometry &Gm = ctx->geo;
   const Layout &L = ctx->L;
   const int NN = L.NN, Y = Gm.Y, X = Gm.X;
@@ -867,10 +1057,7 @@ int forward_chunk(flf_ctx *ctx, const float *vol, long long vol_sz, const PlaneS
   ws_needs(ctx, ps, nt, true, sS, sO, sCv);
   sS = slot_bytes(sS), sO = slot_bytes(sO), sCv = slot_bytes(sCv);
   const int nslot = ws_slots(ctx);
-  int rc = ensure_ws(ctx, ctx->wsS, nslot * sS);
-  if (rc == FLF_OK) rc = ensure_ws(ctx, ctx->wsO, nslot * sO);
-  if (rc == FLF_OK) rc = ensure_ws(ctx, ctx->wsCvol, nslot * sCv);
-  if (rc != FLF_OK) return rc;
+  int rc = FLF_OK;
   int last = -1;
   for (size_t gi = 0; gi < Gm.groups.size(); gi++)
     if (ps.n[gi]) last = (int)gi;
@@ -902,10 +1089,8 @@ int forward_chunk(flf_ctx *ctx, const float *vol, long long vol_sz, const PlaneS
     LAUNCH(ctx, "k_rfft2", chan_bytes(ctx, nt * nplanes) + 8.0 * sp1 * NN * nt * nplanes, s, launch_rfft2(rp, 0, s));
 
     const double pbytes = (double)nplanes * G.nkp * L.nrow * L.RS * sizeof(float2);
-    MacParams mp = mac_params(ctx, G, FLF_DIR_FORWARD, nt);
-    mp.planes = ps.slots[gi]; mp.nz = nplanes; mp.zgroup = zgroup;
-    mp.S = (const float2 *)wS; mp.nzS = nplanes; mp.O = (float4 *)wO; mp.nzo = nzg;
-    mp.nzo_grid = nzg;
+    MacParams mp = mac_params(ctx, FLF_DIR_FORWARD, nt);
+    mac_add_group(mp, G, FLF_DIR_FORWARD, ps.slots[gi], nplanes, zgroup, wS, wO);
     LAUNCH(ctx, "k_mac_fwd", pbytes + 8.0 * sp1 * NN * nt * ((double)nplanes + nzg), s, launch_mac(mp, true, s));
 
     if (k > 0 && nslot > 1) CUDA_TRY(ctx, cudaStreamWaitEvent(s, ctx->ev_chain, 0));
@@ -921,11 +1106,69 @@ int forward_chunk(flf_ctx *ctx, const float *vol, long long vol_sz, const PlaneS
   return join_streams(ctx, s_caller);
 }
 
+// Back projection of one frame, all groups in one multiply-accumulate launch
+// (merge_groups) and all planes in one merge.
+int backward_merged(flf_ctx *ctx, const ChanImg &img, const PlaneSet &ps, Strided out, Strided aux, Strided norm,
+                    int epi, cudaStream_t s) {
+  Geometry &Gm = ctx->geo;
+  const Layout &L = ctx->L;
+  const int NN = L.NN, Y = Gm.Y, X = Gm.X, nall = ps.planes(), ng = ps.groups();
+  const size_t cset = chan_set_floats(ctx);
+  float *cvol = (float *)ctx->wsCvol.p;
+  char *wS = (char *)ctx->wsS.p, *wO = (char *)ctx->wsO.p;
+  MacParams mp = mac_params(ctx, FLF_DIR_BACKWARD, 1);
+  const int zgroup = merged_zgroup(ctx, ps);
+  cudaStream_t st[kFan];
+  if (int rc = fan_out(ctx, s, ng, st)) return rc;
+  double bytes = 0;
+  int k = 0;
+  for (size_t gi = 0; gi < Gm.groups.size(); gi++) {
+    const int n = ps.n[gi];
+    if (!n) continue;
+    const Group &G = Gm.groups[gi];
+    Rfft2Params rp = rfft2_params(ctx, G, img.p, NN, wS);
+    rp.nsum = img.nsum; rp.sum_stride = img.stride; rp.num = img.num;
+    const cudaStream_t sk = st[k % kFan];
+    LAUNCH(ctx, "k_rfft2", chan_bytes(ctx, img.nsum + (img.num ? 1 : 0)) + 8.0 * G.qspec() * NN, sk,
+           launch_rfft2(rp, 0, sk));
+    mac_add_group(mp, G, FLF_DIR_BACKWARD, ps.slots[gi], n, zgroup, wS, wO);
+    bytes += (double)n * G.nkp * L.nrow * L.RS * sizeof(float2) + 8.0 * NN * G.qspec() * (1.0 + n);
+    wS += slot_bytes(sizeof(float2) * NN * G.qspec());
+    wO += slot_bytes(sizeof(float2) * NN * G.qspec() * n);
+    k++;
+  }
+  if (int rc = fan_in(ctx, s, ng)) return rc;
+  LAUNCH(ctx, "k_mac_bwd", bytes, s, launch_mac(mp, false, s));
+  if (int rc = fan_out(ctx, s, ng, st)) return rc;
+  const int *ids = nullptr;
+  int at = 0;
+  k = 0;
+  for (size_t gi = 0; gi < Gm.groups.size(); gi++) {
+    const int n = ps.n[gi];
+    if (!n) continue;
+    const Group &G = Gm.groups[gi];
+    if (!ids) ids = ps.ids[gi];
+    Irfft2Params ip = irfft2_params(ctx, G, (const float2 *)mp.g[k].O, n * NN, cvol + at * cset);
+    ip.final_pass = 1; ip.quads = 1;
+    const cudaStream_t sk = st[k % kFan];
+    LAUNCH(ctx, "k_irfft2", 8.0 * G.qspec() * NN * n + chan_bytes(ctx, n), sk, launch_irfft2(ip, sk));
+    at += n;
+    k++;
+  }
+  if (int rc = fan_in(ctx, s, ng)) return rc;
+  MergeParams mg = merge_params(ctx, cvol, ids, nall, 1, epi, out, aux, norm);
+  const int npix = epi == EPI_STORE ? 1 : (epi == EPI_RL_STANDARD && norm.p ? 4 : 3);
+  LAUNCH(ctx, "k_merge", chan_bytes(ctx, nall) + 4.0 * npix * Y * X * nall, s, launch_merge(mg, s));
+  return FLF_OK;
+}
+
 // Back projection of frames [t0, t0+nt) of the channel-major image set
-// `chan` into the volume `out` (planes of ps) with the epilogue `epi`
+// `img` into the volume `out` (planes of ps) with the epilogue `epi`
 // (aux / norm address volumes).
-int backward_chunk(flf_ctx *ctx, const float *chan, const PlaneSet &ps, int nt, Strided out, Strided aux,
+int backward_chunk(flf_ctx *ctx, const ChanImg &img, const PlaneSet &ps, int nt, Strided out, Strided aux,
                    Strided norm, int epi, cudaStream_t s) {
+  if (merge_groups(ps, nt)) return backward_merged(ctx, img, ps, out, aux, norm, epi, s);
+  const float *chan = img.p;
   Geometry &Gm = ctx->geo;
   const Layout &L = ctx->L;
   const int NN = L.NN, Y = Gm.Y, X = Gm.X;
@@ -933,10 +1176,7 @@ int backward_chunk(flf_ctx *ctx, const float *chan, const PlaneSet &ps, int nt, 
   ws_needs(ctx, ps, nt, false, sS, sO, sCv);
   sS = slot_bytes(sS), sO = slot_bytes(sO), sCv = slot_bytes(sCv);
   const int nslot = ws_slots(ctx);
-  int rc = ensure_ws(ctx, ctx->wsS, nslot * sS);
-  if (rc == FLF_OK) rc = ensure_ws(ctx, ctx->wsO, nslot * sO);
-  if (rc == FLF_OK) rc = ensure_ws(ctx, ctx->wsCvol, nslot * sCv);
-  if (rc != FLF_OK) return rc;
+  int rc = FLF_OK;
   // groups alternate over two streams with their own workspace slots (their
   // planes, and so their outputs, are disjoint)
   cudaStream_t st[2];
@@ -960,10 +1200,8 @@ int backward_chunk(flf_ctx *ctx, const float *chan, const PlaneSet &ps, int nt, 
 
     const double pbytes = (double)nplanes * G.nkp * L.nrow * L.RS * sizeof(float2);
     const int zgb = zgroup_for(ctx, nplanes, G.nquads);
-    MacParams mp = mac_params(ctx, G, FLF_DIR_BACKWARD, nt);
-    mp.planes = ps.slots[gi]; mp.nz = nplanes; mp.zgroup = zgb;
-    mp.S = (const float2 *)wS; mp.nzS = 1; mp.O = (float4 *)wO; mp.nzo = nplanes;
-    mp.nzo_grid = (nplanes + zgb - 1) / zgb;
+    MacParams mp = mac_params(ctx, FLF_DIR_BACKWARD, nt);
+    mac_add_group(mp, G, FLF_DIR_BACKWARD, ps.slots[gi], nplanes, zgb, wS, wO);
     LAUNCH(ctx, "k_mac_bwd", pbytes + 8.0 * sp1 * NN * nt * (1.0 + nplanes), s, launch_mac(mp, false, s));
 
     Irfft2Params ip = irfft2_params(ctx, G, wO, nt * nplanes * NN, cvol);
@@ -1077,6 +1315,10 @@ int flf_ctx_destroy(flf_ctx *ctx) {
   for (cudaEvent_t e : evs)
     if (e) cudaEventDestroy(e);
   if (ctx->s2) cudaStreamDestroy(ctx->s2);
+  for (int i = 0; i < kFan - 1; i++) {
+    if (ctx->ev_fan[i]) cudaEventDestroy(ctx->ev_fan[i]);
+    if (ctx->s_fan[i]) cudaStreamDestroy(ctx->s_fan[i]);
+  }
   delete ctx;
   return FLF_OK;
 }
@@ -1145,16 +1387,18 @@ int flf_forward(flf_ctx *ctx, const float *vol_dev, float *img_dev, int T, int Y
   if (rc != FLF_OK) return rc;
   const int TF = frames_per_pass(ctx);
   const long long vol_sz = (long long)T * Y * X;
-  rc = ensure_ws(ctx, ctx->wsCimg, sizeof(float) * chan_set_floats(ctx) * std::min(T, TF));
+  rc = ensure_workspaces(ctx, ps, T, TF, true, false);
   float *cimg = (float *)ctx->wsCimg.p;
   for (int t0 = 0; t0 < T && rc == FLF_OK; t0 += TF) {
     const int nt = std::min(TF, T - t0);
-    rc = forward_chunk(ctx, vol_dev, vol_sz, ps, t0, nt, cimg, nullptr, s);
+    ChanImg hx;
+    rc = forward_chunk(ctx, vol_dev, vol_sz, ps, t0, nt, cimg, nullptr, hx, s);
     if (rc != FLF_OK) break;
     const Strided out{img_dev + (long long)t0 * Y * X, 0, (long long)Y * X};
     MergeParams mg = merge_params(ctx, cimg, nullptr, 1, nt, EPI_STORE, out, Strided{nullptr, 0, 0},
                                   Strided{nullptr, 0, 0});
-    LAUNCH(ctx, "k_merge", chan_bytes(ctx, nt) + 4.0 * Y * X * nt, s, launch_merge(mg, s));
+    mg.nsum = hx.nsum; mg.sum_stride = hx.stride;
+    LAUNCH(ctx, "k_merge", chan_bytes(ctx, nt * hx.nsum) + 4.0 * Y * X * nt, s, launch_merge(mg, s));
   }
   return rc;
 }
@@ -1171,7 +1415,7 @@ int flf_backward(flf_ctx *ctx, const float *img_dev, float *vol_dev, int T, int 
   PlaneSet ps;
   if (rc == FLF_OK) rc = make_plane_set(ctx, planes, nplanes, s, ps);
   if (rc != FLF_OK) return rc;
-  rc = ensure_ws(ctx, ctx->wsCimg, sizeof(float) * chan_set_floats(ctx) * std::min(T, frames_per_pass(ctx)));
+  rc = ensure_workspaces(ctx, ps, T, frames_per_pass(ctx), false, true);
   if (rc != FLF_OK) return rc;
   return backward_run(ctx, img_dev, vol_dev, T, Y, X, ps, s);
 }
@@ -1226,9 +1470,8 @@ int flf_backward_noalloc(flf_ctx *ctx, const float *img_dev, float *vol_dev, int
       for (int z0 = 0; z0 < ng && e == cudaSuccess; z0 += zb) {
         const int nzl = std::min(zb, ng - z0);
         const int zg = zgroup_for(ctx, nzl, G.nquads);
-        MacParams mp = mac_params(ctx, G, FLF_DIR_BACKWARD, 1);
-        mp.planes = G.d_slots + z0; mp.nz = nzl; mp.zgroup = zg;
-        mp.S = S; mp.nzS = 1; mp.O = (float4 *)O; mp.nzo = nzl; mp.nzo_grid = (nzl + zg - 1) / zg;
+        MacParams mp = mac_params(ctx, FLF_DIR_BACKWARD, 1);
+        mac_add_group(mp, G, FLF_DIR_BACKWARD, G.d_slots + z0, nzl, zg, S, O);
         e = launch_mac(mp, false, s);
         if (e != cudaSuccess) break;
         Irfft2Params ip = irfft2_params(ctx, G, O, nzl * NN, Co);
@@ -1263,17 +1506,9 @@ int rl_setup(flf_ctx *ctx, float *x_dev, const float *ref_dev, int variant, int 
   if (rc != FLF_OK) return rc;
   const int nt = std::min(T, frames_per_pass(ctx));
   const size_t cset = sizeof(float) * chan_set_floats(ctx) * nt;
-  rc = ensure_ws(ctx, ctx->wsCimg, cset);
-  if (rc == FLF_OK && variant == FLF_RL_STANDARD) rc = ensure_ws(ctx, ctx->wsCy, cset);
+  if (variant == FLF_RL_STANDARD) rc = ensure_ws(ctx, ctx->wsCy, cset);
   if (rc == FLF_OK) rc = make_plane_set(ctx, nullptr, ctx->nz, s, ps);
-  if (rc != FLF_OK) return rc;
-  size_t a, b, c, a2, b2, c2;
-  ws_needs(ctx, ps, nt, true, a, b, c);
-  ws_needs(ctx, ps, nt, false, a2, b2, c2);
-  const int nslot = ws_slots(ctx);
-  rc = ensure_ws(ctx, ctx->wsS, nslot * slot_bytes(std::max(a, a2)));
-  if (rc == FLF_OK) rc = ensure_ws(ctx, ctx->wsO, nslot * slot_bytes(std::max(b, b2)));
-  if (rc == FLF_OK) rc = ensure_ws(ctx, ctx->wsCvol, nslot * slot_bytes(std::max(c, c2)));
+  if (rc == FLF_OK) rc = ensure_workspaces(ctx, ps, T, frames_per_pass(ctx), true, true);
   if (rc == FLF_OK) rc = ensure_streams(ctx);
   return rc;
 }
@@ -1291,7 +1526,9 @@ int backward_run(flf_ctx *ctx, const float *img_dev, float *vol_dev, int T, int 
     SplitParams sp = split_params(ctx, img_dev + t0 * YX, 0, YX, nullptr, 1, nt, cimg);
     LAUNCH(ctx, "k_split", chan_bytes(ctx, nt) + 4.0 * YX * nt, s, launch_split(sp, s));
     const Strided out{vol_dev + t0 * YX, (long long)T * YX, YX};
-    rc = backward_chunk(ctx, cimg, ps, nt, out, Strided{nullptr, 0, 0}, Strided{nullptr, 0, 0}, EPI_STORE, s);
+    ChanImg img;
+    img.p = cimg;
+    rc = backward_chunk(ctx, img, ps, nt, out, Strided{nullptr, 0, 0}, Strided{nullptr, 0, 0}, EPI_STORE, s);
   }
   return rc;
 }
@@ -1314,15 +1551,16 @@ int rl_run(flf_ctx *ctx, float *x_dev, const float *ref_dev, const float *norm_d
     for (int it = 0; it < iters && rc == FLF_OK; it++) {
       // H x (Prevedel) or y / H x (standard) as channel-major images, then the
       // back projection with the update fused into its pixel epilogue
+      ChanImg hx;
       rc = forward_chunk(ctx, x_dev, (long long)T * YX, ps, t0, nt, cimg,
-                         variant == FLF_RL_STANDARD ? cy : nullptr, s);
+                         variant == FLF_RL_STANDARD ? cy : nullptr, hx, s);
       if (rc != FLF_OK) break;
       if (variant == FLF_RL_PREVEDEL) {
         const Strided htf{const_cast<float *>(ref_dev) + t0 * YX, (long long)T * YX, YX};
-        rc = backward_chunk(ctx, cimg, ps, nt, xs, htf, Strided{nullptr, 0, 0}, EPI_RL_PREVEDEL, s);
+        rc = backward_chunk(ctx, hx, ps, nt, xs, htf, Strided{nullptr, 0, 0}, EPI_RL_PREVEDEL, s);
       } else {
         const Strided nrm{const_cast<float *>(norm_dev), YX, 0};
-        rc = backward_chunk(ctx, cimg, ps, nt, xs, Strided{nullptr, 0, 0}, nrm, EPI_RL_STANDARD, s);
+        rc = backward_chunk(ctx, hx, ps, nt, xs, Strided{nullptr, 0, 0}, nrm, EPI_RL_STANDARD, s);
       }
     }
   }

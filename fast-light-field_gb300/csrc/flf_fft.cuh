@@ -344,12 +344,25 @@ __global__ void __launch_bounds__(Shape<F>::NT, Shape<F>::MINB) k_rfft2_sized(Rf
   const int b = ch / N, a = ch - b * N;
   const int nq = sa.nq, Ly = p.Ly, Lx = p.Lx, X = p.X, Y = p.Y, Lxp = p.Lxp;
 
-  // R0: the channel image into region A with 16-byte loads.
+  // R0: the channel image into region A with 16-byte loads: the sum of nsum sets, or num over it
+  // (the standard RL error image, lfdeconv.py:192; positions outside the image are not used).
   {
     const float4 *src = reinterpret_cast<const float4 *>(p.chan + (long long)g * Ly * Lxp);
+    const float4 *num = p.num ? reinterpret_cast<const float4 *>(p.num + (long long)g * Ly * Lxp) : nullptr;
     float4 *st = reinterpret_cast<float4 *>(A);
     const int n4 = Ly * Lxp / 4;
-    for (int i = threadIdx.x; i < n4; i += NT) st[i] = __ldg(src + i);
+    for (int i = threadIdx.x; i < n4; i += NT) {
+      float4 v = __ldg(src + i);
+      for (int k = 1; k < p.nsum; k++) {
+        const float4 w = __ldg(src + i + k * (p.sum_stride / 4));
+        v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
+      }
+      if (num) {
+        const float4 w = __ldg(num + i);
+        v = make_float4(__fdiv_rn(w.x, v.x), __fdiv_rn(w.y, v.y), __fdiv_rn(w.z, v.z), __fdiv_rn(w.w, v.w));
+      }
+      st[i] = v;
+    }
   }
   __syncthreads();
 

@@ -137,6 +137,9 @@ struct Rfft2Params {
   int nimg;                 // total images
   int mode;                 // 0: channel-major float images (chan); 1: contiguous f*f images
   const float *chan;        // mode 0: [nimg][Ly][Lxp], image g = set * NN + ch
+  int nsum;                 // mode 0: images to add, sum_stride floats apart (a multiple of 4)
+  long long sum_stride;
+  const float *num;         // mode 0, optional: transform num / sum (like chan)
   int Lxp;
   const void *src_img;      // mode 1: Real images [nimg][f][f]
   void *dst;                // mode 0: complex [nimg][quads][4]; mode 1: Complex<Real> [nimg][f][fh]
@@ -174,6 +177,8 @@ struct SplitParams {        // src + plane*src_sz + t*src_st: Y x X pixels
 
 struct MergeParams {
   const float *src;         // [nsets][NN][Ly][Lxp], set s = t * nzo + zo
+  int nsum;                 // sets to add, sum_stride floats apart
+  long long sum_stride;
   int nzo, nsets;
   const int *planes;        // plane id per zo (device); NULL -> zo
   int N, Y, X, Ly, Lx, Lxp;
@@ -192,21 +197,27 @@ struct ResampleParams {     // bilinear resample of img [H][W] at yq [ny] x xq [
   double *out;
 };
 
-struct MacParams {
-  Layout L;
-  int f, fh, fq, nkp;       // transform size, f/2+1, f/2+1, fq*fq half blocks per plane
-  int nquads;               // fq(fq+1)/2 frequency quads (grid.x)
-  int T;                    // frames in this launch (<= template TF)
-  const float4 *P;          // packed matrices [plane][half block][nrow][NP]
-  const int *planes;        // plane id per z index
+// Planes of one transform size in a multiply-accumulate launch.
+struct MacGroup {
+  int f, fh, nkp;           // transform size, f/2+1, (f/2+1)^2 half blocks per plane
+  int nquads;               // frequency quads of a plane
+  int cta0;                 // first CTA of the group: quad + nquads * (planes' z group)
   int nz;                   // planes in the list
-  int zgroup;               // forward: planes per CTA group
-  const float2 *S;          // input spectra [T][nzS][NN][nquads][4] (quad order)
+  int zgroup;               // planes per CTA
   int nzS;                  // planes in S (forward nz, backward 1)
+  int nzo;                  // forward: number of z groups (output sets); backward: nz
+  const float4 *P;          // packed matrices [plane][half block][nrow][NP]
+  const int *planes;        // plane slot per z index
+  const float2 *S;          // input spectra [T][nzS][NN][nquads][4] (quad order)
   float4 *O;                // output spectra: forward [zgroup][T][NN][f][fh] complex; backward
                             // [T][nzo][NN][nquads][2 sides], u and u* of a side (quad order)
-  int nzo;                  // forward: number of z groups (output sets); backward: nz
-  int nzo_grid;             // grid.y: number of z groups of this launch
+};
+constexpr int kMacMaxGroups = 8;
+struct MacParams {
+  Layout L;
+  int T;                    // frames in this launch (the template's)
+  int ngroups;
+  MacGroup g[kMacMaxGroups];
   const short4 *rowS;       // [3][nrow]: operand channels of each row for its own frequency pair (0)
                             // and through the transpose (1): sa, sb at u, sa, sb at u* (-1: none);
                             // then the row flags (.x)

@@ -263,11 +263,11 @@ __device__ __forceinline__ void bar_sync(int n) { asm volatile("bar.sync 1, %0;\
 // spectrum.  Each enters one or two entries, so staging the spectra first would
 // cost more than it saves.
 template <int TF>
-__device__ void build_sv(float4 *sv, const MacParams &p, int zs, const short4 *rowS, int nhalf, bool selfp0,
+__device__ void build_sv(float4 *sv, const MacParams &p, const MacGroup &G, int zs, const short4 *rowS, int nhalf, bool selfp0,
                          bool selfp1, int kq, int first, int step) {
   constexpr int U = 4;                                 // entries per round, loads first
   const int R = p.L.nrow, NN = p.L.NN, nT = p.L.nrowT;
-  const int ss = 4 * p.nquads;                         // values of a spectrum
+  const int ss = 4 * G.nquads;                         // values of a spectrum
   const int n = min(TF, p.T) * nhalf * R * 4;
   for (int i0 = first; i0 < n; i0 += U * step) {
     float2 sa[U], sb[U];
@@ -283,7 +283,7 @@ __device__ void build_sv(float4 *sv, const MacParams &p, int zs, const short4 *r
       if ((rowS[2 * R + row].x & kRowSecond) && (side ? selfp1 : selfp0)) continue;
       const short4 si = rowS[use * R + row];
       const int ia = (e & 1) ? si.z : si.x, ib = (e & 1) ? si.w : si.y;
-      const float2 *src = p.S + (long long)(t * p.nzS + zs) * NN * ss + 4 * kq + e;
+      const float2 *src = G.S + (long long)(t * G.nzS + zs) * NN * ss + 4 * kq + e;
       if (ia >= 0) sa[k] = __ldg(src + ia * ss);
       if (ib >= 0) sb[k] = __ldg(src + ib * ss);
     }
@@ -423,7 +423,11 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>
   const int nthreads = 32 * nwarps;
 
   // quad k = ux (ux + 1) / 2 + uy, uy <= ux
-  const int kq = blockIdx.x;
+  int gi = 0;
+  while (gi + 1 < p.ngroups && (int)blockIdx.x >= p.g[gi + 1].cta0) gi++;
+  const MacGroup &G = p.g[gi];
+  const int zgi = ((int)blockIdx.x - G.cta0) / G.nquads;      // z group
+  const int kq = (int)blockIdx.x - G.cta0 - zgi * G.nquads;
   int ux = (int)((sqrtf(8.f * (float)kq + 1.f) - 1.f) * 0.5f);
   while ((ux + 1) * (ux + 2) / 2 <= kq) ux++;
   while (ux * (ux + 1) / 2 > kq) ux--;
@@ -431,9 +435,9 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>
   const bool diag = (uy == ux);
   const int hb0 = 2 * kq - ux;                   // first half block of the quad
   const int nhalf = diag ? 1 : 2;
-  const bool selfp0 = (uy == 0) || (2 * uy == p.f), selfp1 = (ux == 0) || (2 * ux == p.f);
-  const int z0 = blockIdx.y * p.zgroup;
-  const int z1 = min(z0 + p.zgroup, p.nz);
+  const bool selfp0 = (uy == 0) || (2 * uy == G.f), selfp1 = (ux == 0) || (2 * ux == G.f);
+  const int z0 = zgi * G.zgroup;
+  const int z1 = min(z0 + G.zgroup, G.nz);
   const int nrq = nhalf * R;                     // stored rows of the quad per plane
   const int cpb = (nrq + CH - 1) / CH;           // chunks per (quad, plane)
   const int total = (z1 - z0) * cpb;
@@ -445,13 +449,13 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>
   // once with chunk g + NST, so no thread ever waits for a slot to drain.
   // p.drop_chunk >= 0 (a test of the bounded waits only): the first CTA never
   // issues that chunk, so the waits on its slot run out after p.wait_ns
-  const int drop = blockIdx.x == 0 && blockIdx.y == 0 ? p.drop_chunk : -1;
+  const int drop = blockIdx.x == 0 ? p.drop_chunk : -1;
   auto issue = [&](int gn, const int *planes) {
     if (gn == drop) return;
     const int zl_n = gn / cpb, ch_n = gn - zl_n * cpb, sl = gn % NST;
     const int r0 = ch_n * CH;
     const int nr = min(CH, nrq - r0);
-    const float4 *src = p.P + ((long long)planes[zl_n] * p.nkp + hb0) * (long long)halfElems + (long long)r0 * NP;
+    const float4 *src = G.P + ((long long)planes[zl_n] * G.nkp + hb0) * (long long)halfElems + (long long)r0 * NP;
     const unsigned bytes = (unsigned)(nr * NP * sizeof(float4));
     mbar_arrive_expect_tx(full + sl, bytes);
     bulk_g2s(ring + (size_t)sl * CH * NP, src, bytes, full + sl);
@@ -468,13 +472,13 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>
     *abortf = 0;
     fence_mbar_init();
     const int pre = min(NST, total);
-    for (int g = 0; g < pre; g++) issue(g, p.planes + z0);
+    for (int g = 0; g < pre; g++) issue(g, G.planes + z0);
     s_issued = pre;
   }
   for (int i = tid; i < 3 * R; i += blockDim.x) rowS[i] = p.rowS[i];
-  for (int i = tid; i < z1 - z0; i += blockDim.x) s_plane[i] = p.planes[z0 + i];
+  for (int i = tid; i < z1 - z0; i += blockDim.x) s_plane[i] = G.planes[z0 + i];
   __syncthreads();   // barriers initialised, row tables staged
-  build_sv<TF>(sv0, p, FWD ? z0 : 0, rowS, nhalf, selfp0, selfp1, kq, tid, blockDim.x);
+  build_sv<TF>(sv0, p, G, FWD ? z0 : 0, rowS, nhalf, selfp0, selfp1, kq, tid, blockDim.x);
   __syncthreads();
 
   if (HELP && warp == nwarps) {
@@ -482,7 +486,7 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>
     for (int zl = 1; zl < z1 - z0; zl++) {
       const int b = zl & 1;
       if (zl > 1 && !mbar_wait(svfree + b, ((zl >> 1) - 1) & 1, p.wait_ns)) break;   // the waiting warps report it
-      build_sv<TF>(sv0 + b * TF * svt, p, z0 + zl, rowS, nhalf, selfp0, selfp1, kq, lane, 32);
+      build_sv<TF>(sv0 + b * TF * svt, p, G, z0 + zl, rowS, nhalf, selfp0, selfp1, kq, lane, 32);
       mbar_arrive(svfull + b);
     }
     __syncthreads();   // the streaming warps' last barrier
@@ -506,7 +510,7 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>
     const int zi = z0 + zl;
     if (FWD && !HELP && ch == 0 && zl > 0) {
       bar_sync(nthreads);   // every warp is done with plane zi - 1
-      build_sv<TF>(sv0, p, zi, rowS, nhalf, selfp0, selfp1, kq, tid, nthreads);
+      build_sv<TF>(sv0, p, G, zi, rowS, nhalf, selfp0, selfp1, kq, tid, nthreads);
       bar_sync(nthreads);
     }
     if (*abortf) dead = true;
@@ -607,12 +611,12 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>
           }
           if (FWD) {                                 // row order
             const int oy = s ? ux : uy;
-            float2 *op = reinterpret_cast<float2 *>(p.O) +
-                         ((long long)(blockIdx.y * p.T + t) * NN + q) * (p.f * p.fh) + (s ? uy : ux);
-            op[oy * p.fh] = u;
-            if (!(s ? selfp1 : selfp0)) op[(p.f - oy) * p.fh] = v;
+            float2 *op = reinterpret_cast<float2 *>(G.O) +
+                         ((long long)(zgi * p.T + t) * NN + q) * (G.f * G.fh) + (s ? uy : ux);
+            op[oy * G.fh] = u;
+            if (!(s ? selfp1 : selfp0)) op[(G.f - oy) * G.fh] = v;
           } else {                                   // quad order
-            p.O[(((long long)(t * p.nzo + zi) * NN + q) * p.nquads + kq) * 2 + s] = make_float4(u.x, u.y, v.x, v.y);
+            G.O[(((long long)(t * G.nzo + zi) * NN + q) * G.nquads + kq) * 2 + s] = make_float4(u.x, u.y, v.x, v.y);
           }
         }
       }
@@ -768,7 +772,9 @@ __global__ void __launch_bounds__(256) k_merge(MergeParams p) {
   for (int i = threadIdx.x; i < N * Lx; i += blockDim.x) {
     const int a = (int)p.dlx.div(i);
     const int c = i - a * Lx;
-    sm[a * pitch + c] = __ldg(src + a * cstride + c);
+    float v = __ldg(src + a * cstride + c);
+    for (int k = 1; k < p.nsum; k++) v += __ldg(src + k * p.sum_stride + a * cstride + c);
+    sm[a * pitch + c] = v;
   }
   __syncthreads();
   const int plane = p.planes ? p.planes[zo] : zo;
@@ -933,7 +939,13 @@ static cudaError_t launch_mac_tf(const MacParams &p0, cudaStream_t s) {
   const MacThreads th = mac_threads(p.L, p.split);
   p.shares = th.shares;
   const size_t sm = mac_smem_bytes(p.L, TF, p.stages, p.chunk_rows, FWD);
-  const dim3 grid(p.nquads, p.nzo_grid);
+  int ctas = 0;
+  for (int i = 0; i < p.ngroups; i++) {
+    MacGroup &G = p.g[i];
+    G.cta0 = ctas;
+    ctas += G.nquads * ((G.nz + G.zgroup - 1) / G.zgroup);
+  }
+  const dim3 grid(ctas);
   const int threads = 32 * th.cw * th.shares, block = threads + (FWD && TF == 1 ? 32 : 0);   // and the helper warp
   void (*fn)(MacParams) = threads <= 128 ? (th.ppt == 2 ? k_mac<TF, FWD, 2, 128> : k_mac<TF, FWD, 1, 128>)
                                        : (th.ppt == 2 ? k_mac<TF, FWD, 2, 256> : k_mac<TF, FWD, 1, 256>);
