@@ -2324,39 +2324,38 @@ static cudaError_t launch_wide(ConvParams p, long long ws_elems, cudaStream_t s,
   // bits: among the shapes with that split the least estimated time.  Measured (64 -> 64, one to
   // four M tiles with an issuer each): a weight block takes about 100 cycles and one MMA's time per
   // M tile (the A and B operand reads, 32 + CO/4, or the math, CO/2), plus a fixed cost per unit.
-  WideGrid g{};
-  size_t smem = 0;
-  bool found = false;
-  int split = 1;
-  for (int pass = 0; pass < 2; pass++) {
-    double best = -1;
-    for (int nM = 1; nM <= 4; nM++) {
-      if (g_conv_wide_tc >= 2 && nM != g_conv_wide_tc - 1) continue;
-      WideGrid c{};
-      size_t sm = 0;
-      if (!wide_shape(CI, CO, p.Y, p.X, nM, c, sm)) continue;
-      for (int sp = 1; sp <= (can_split ? 3 : 1); sp += 2) {
-        c.splits = sp;
-        c.items = (long long)p.B * p.Z * c.nyb * sp;
-        const double waves = (double)((c.items + sms - 1) / sms);
-        const double blocks = 27.0 * (CI / 16) / sp;
-        if (pass == 0) {
-          const double partials = sp > 1 ? 4000.0 + 2.0 * 3.0 * (double)Mv * CO * 4.0 / 3000.0 : 0.0;
-          const double cost = waves * (blocks * (c.tps == 3 ? 272.0 : 320.0) + 3000.0) + partials;
-          if (best < 0 || cost <= best) best = cost, split = sp;
-        } else if (sp == split) {
-          const double cost = waves * (blocks * (100.0 + std::max(32.0 + CO / 4.0, CO / 2.0) * c.nM) + 3000.0);
-          if (best < 0 || cost <= best) {
-            found = true;
-            best = cost;
-            g = c;
-            smem = sm;
-          }
-        }
+  WideGrid best[2];             // unsplit, split
+  size_t best_smem[2] = {0, 0};
+  double best_cost[2] = {-1, -1}, rule = -1;
+  int pick = -1;
+  for (int nM = 1; nM <= 4; nM++) {
+    if (g_conv_wide_tc >= 2 && nM != g_conv_wide_tc - 1) continue;
+    WideGrid c{};
+    size_t sm = 0;
+    if (!wide_shape(CI, CO, p.Y, p.X, nM, c, sm)) continue;
+    for (int k = 0; k < (can_split ? 2 : 1); k++) {
+      const int sp = k ? 3 : 1;
+      c.splits = sp;
+      c.items = (long long)p.B * p.Z * c.nyb * sp;
+      const double waves = (double)((c.items + sms - 1) / sms);
+      const double blocks = 27.0 * (CI / 16) / sp;
+      const double partials = sp > 1 ? 4000.0 + 2.0 * 3.0 * (double)Mv * CO * 4.0 / 3000.0 : 0.0;
+      const double by_rule = waves * (blocks * (c.tps == 3 ? 272.0 : 320.0) + 3000.0) + partials;
+      const double cost = waves * (blocks * (100.0 + std::max(32.0 + CO / 4.0, CO / 2.0) * c.nM) + 3000.0);
+      if (rule < 0 || by_rule <= rule) {
+        rule = by_rule;
+        pick = k;
+      }
+      if (best_cost[k] < 0 || cost <= best_cost[k]) {
+        best_cost[k] = cost;
+        best[k] = c;
+        best_smem[k] = sm;
       }
     }
   }
-  if (!found) return cudaSuccess;   // the mma.sync kernel takes this shape
+  if (pick < 0) return cudaSuccess;   // the mma.sync kernel takes this shape
+  const WideGrid &g = best[pick];
+  const size_t smem = best_smem[pick];
   done = true;
   if (reinterpret_cast<uintptr_t>(p.x) % 16 || reinterpret_cast<uintptr_t>(p.wp) % 16) return cudaErrorMisalignedAddress;
   PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
