@@ -90,7 +90,7 @@ struct flf_ctx {
   int opt_stages = 2;            // tunable: MAC shared-memory pipeline stages
   int opt_chunk_rows[2] = {0, 0};   // tunable: stored rows per pipeline stage (forward, backward); 0: auto_chunk_rows
   int opt_split = 1;             // tunable: threads sharing one orbit's rows
-  int opt_ctas_per_sm = 16;      // tunable: multiply-accumulate CTAs per SM the plane grouping aims at
+  int opt_ctas_per_sm = 0;       // tunable: multiply-accumulate CTAs per SM the plane grouping aims at (0: by rule)
   int opt_plane_sizes = 1;       // 1: transform size per plane (grouped); 0: one size for all
   int opt_geometry_cache = 2;    // geometries of other image shapes kept resident (most recent first)
   std::vector<Geometry> parked;  // those geometries
@@ -676,10 +676,19 @@ int check_ready(flf_ctx *ctx, int T, int Y, int X, int dir, cudaStream_t s) {
   return rc;
 }
 
+// Multiply-accumulate CTAs per SM the plane grouping aims at where none were
+// asked for: 16; 8 in back projections of two frames and more, which fill an SM with
+// fewer CTAs and gain by the longer ones (us a projection with 16 and 8: Nnum 5, 31
+// planes of 250 px, four frames 143, 135; Nnum 11, 330 px 502, 469; Nnum 15, 450 px
+// 899, 877; Nnum 19, 760 px 3361, 3270; one frame 39, 46 | 138, 141 | 303, 307).
+int ctas_per_sm(const flf_ctx *ctx, int dir, int nt) {
+  return ctx->opt_ctas_per_sm ? ctx->opt_ctas_per_sm : dir == FLF_DIR_BACKWARD && nt >= 2 ? 8 : 16;
+}
+
 // Planes per multiply-accumulate CTA: enough plane groups to give about
-// opt_ctas_per_sm (16) CTAs per SM over the nquads frequency quads.
-int zgroup_for(const flf_ctx *ctx, int nz, int nquads) {
-  const int target = ctx->opt_ctas_per_sm * std::max(1, ctx->num_sms);
+// `per_sm` CTAs per SM over the nquads frequency quads.
+int zgroup_for(const flf_ctx *ctx, int nz, int nquads, int per_sm) {
+  const int target = per_sm * std::max(1, ctx->num_sms);
   const int nzg_needed = std::min(nz, std::max(1, (target + nquads - 1) / nquads));
   return std::min(kMacMaxZgroup, std::max(1, (nz + nzg_needed - 1) / nzg_needed));
 }
@@ -703,7 +712,7 @@ void ws_needs(const flf_ctx *ctx, const PlaneSet &ps, int nt, bool fwd, size_t &
     const int n = ps.n[g];
     sCv = std::max(sCv, cset * nt * n);
     if (fwd) {
-      const int zg = zgroup_for(ctx, n, G.groups[g].nquads);
+      const int zg = zgroup_for(ctx, n, G.groups[g].nquads, ctas_per_sm(ctx, FLF_DIR_FORWARD, nt));
       sS = std::max(sS, qspec * nt * n);
       sO = std::max(sO, spec * nt * ((n + zg - 1) / zg));
     } else {
@@ -728,11 +737,11 @@ bool merge_groups(const PlaneSet &ps, int nt) {
   return nt == 1 && k >= 3 && k <= kMacMaxGroups;
 }
 
-// Planes per CTA of such a launch: about opt_ctas_per_sm CTAs per SM in all.
+// Planes per CTA of such a launch (of one frame): about 16 CTAs per SM in all.
 int merged_zgroup(const flf_ctx *ctx, const PlaneSet &ps) {
   long long units = 0;
   for (size_t g = 0; g < ctx->geo.groups.size(); g++) units += (long long)ps.n[g] * ctx->geo.groups[g].nquads;
-  const long long target = (long long)ctx->opt_ctas_per_sm * std::max(1, ctx->num_sms);
+  const long long target = (long long)ctas_per_sm(ctx, FLF_DIR_FORWARD, 1) * std::max(1, ctx->num_sms);
   return (int)std::min<long long>(kMacMaxZgroup, std::max(1LL, (units + target - 1) / target));
 }
 
@@ -931,7 +940,8 @@ cudaError_t mac_group_launch(flf_ctx *ctx, size_t gi, int dir, int nt, const Pla
   const Group &G = ctx->geo.groups[gi];
   MacParams mp = mac_params(ctx, dir, nt);
   mp.stages = stages; mp.chunk_rows = chunk; mp.split = split;
-  mac_add_group(mp, G, dir, ps.slots[gi], ps.n[gi], zgroup_for(ctx, ps.n[gi], G.nquads), ctx->wsS.p, ctx->wsO.p);
+  mac_add_group(mp, G, dir, ps.slots[gi], ps.n[gi], zgroup_for(ctx, ps.n[gi], G.nquads, ctas_per_sm(ctx, dir, nt)),
+                ctx->wsS.p, ctx->wsO.p);
   return launch_mac(mp, dir == FLF_DIR_FORWARD, s);
 }
 
@@ -1078,7 +1088,7 @@ int forward_chunk(flf_ctx *ctx, const float *vol, long long vol_sz, const PlaneS
     float2 *wO = (float2 *)((char *)ctx->wsO.p + slot * sO);
     const Group &G = Gm.groups[gi];
     const size_t sp1 = G.spec();
-    const int zgroup = zgroup_for(ctx, nplanes, G.nquads);
+    const int zgroup = zgroup_for(ctx, nplanes, G.nquads, ctas_per_sm(ctx, FLF_DIR_FORWARD, nt));
     const int nzg = (nplanes + zgroup - 1) / zgroup;
 
     SplitParams sp = split_params(ctx, vol + (long long)t0 * Y * X, vol_sz, (long long)Y * X, ps.ids[gi],
@@ -1199,7 +1209,7 @@ int backward_chunk(flf_ctx *ctx, const ChanImg &img, const PlaneSet &ps, int nt,
     LAUNCH(ctx, "k_rfft2", chan_bytes(ctx, nt) + 8.0 * sp1 * NN * nt, s, launch_rfft2(rp, 0, s));
 
     const double pbytes = (double)nplanes * G.nkp * L.nrow * L.RS * sizeof(float2);
-    const int zgb = zgroup_for(ctx, nplanes, G.nquads);
+    const int zgb = zgroup_for(ctx, nplanes, G.nquads, ctas_per_sm(ctx, FLF_DIR_BACKWARD, nt));
     MacParams mp = mac_params(ctx, FLF_DIR_BACKWARD, nt);
     mac_add_group(mp, G, FLF_DIR_BACKWARD, ps.slots[gi], nplanes, zgb, wS, wO);
     LAUNCH(ctx, "k_mac_bwd", pbytes + 8.0 * sp1 * NN * nt * (1.0 + nplanes), s, launch_mac(mp, false, s));
@@ -1469,7 +1479,7 @@ int flf_backward_noalloc(flf_ctx *ctx, const float *img_dev, float *vol_dev, int
       e = launch_rfft2(rfft2_params(ctx, G, C, NN, S), 0, s);
       for (int z0 = 0; z0 < ng && e == cudaSuccess; z0 += zb) {
         const int nzl = std::min(zb, ng - z0);
-        const int zg = zgroup_for(ctx, nzl, G.nquads);
+        const int zg = zgroup_for(ctx, nzl, G.nquads, ctas_per_sm(ctx, FLF_DIR_BACKWARD, 1));
         MacParams mp = mac_params(ctx, FLF_DIR_BACKWARD, 1);
         mac_add_group(mp, G, FLF_DIR_BACKWARD, G.d_slots + z0, nzl, zg, S, O);
         e = launch_mac(mp, false, s);

@@ -371,7 +371,8 @@ int mac_max_frames();
 // Shared memory one CTA may opt in to (sm_100 family).
 constexpr size_t kMacSmemMax = 227 * 1024;
 size_t mac_smem_bytes(const Layout &L, int TF, int stages, int chunk_rows, bool fwd);
-struct MacThreads { int ppt, cw, shares; };   // channel pairs per lane, warps side by side, row shares
-MacThreads mac_threads(const Layout &L, int split);
+struct MacThreads { int ppt, cw, sides, shares; };   // channel pairs per lane, warps side by side,
+                                                     // sides per thread, row shares
+MacThreads mac_threads(const Layout &L, int split, int frames, bool fwd);
 
 }  // namespace flf

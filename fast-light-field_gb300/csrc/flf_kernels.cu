@@ -250,7 +250,7 @@ constexpr unsigned long long kWaitLimitNs = 1000000000ull;   // 1 s per wait
 __device__ __forceinline__ void bar_sync(int n) { asm volatile("bar.sync 1, %0;\n" ::"r"(n) : "memory"); }
 
 // Operand table of one plane, straight from the input spectra:
-//   sv[t][half block][row][side][u / u*] = (p0, m0, p1, m1),
+//   sv[half block][row][side][t][u / u*] = (p0, m0, p1, m1),
 // the real factors with which the row (C, D of every channel pair) enters the
 // accumulators of the receiving side,  P += C p0 + D p1,  M += C m0 + D m1.
 // With sa the spectrum that multiplies the row's channel directly and sb the
@@ -293,7 +293,7 @@ __device__ void build_sv(float4 *sv, const MacParams &p, const MacGroup &G, int 
       if (idx >= n) continue;
       const int rest = idx >> 2, tb = rest / R, row = rest - tb * R;
       const int t = tb / nhalf, bs = tb - t * nhalf;
-      sv[((t * 2 + bs) * R + row) * 4 + (idx & 3)] =
+      sv[((bs * R + row) * 2 + ((idx >> 1) & 1)) * 2 * TF + t * 2 + (idx & 1)] =
           make_float4(sa[k].x + sb[k].x, sa[k].y + sb[k].y, sa[k].y - sb[k].y, sb[k].x - sa[k].x);
     }
   }
@@ -315,11 +315,11 @@ size_t mac_smem_bytes(const Layout &L, int TF, int stages, int chunk_rows, bool 
 // (four per channel pair and row, used on both sides and all frames); pairs of
 // (re, im) with doubled operands took 2 % longer at one frame and 5 % at four,
 // plain FMAs 3 % and 10 %.
-template <int TF, int PPT> struct MacAcc {
-  float2 X[2][TF][PPT][2], Y[2][TF][PPT][2];
+template <int TF, int PPT, int SD> struct MacAcc {
+  float2 X[SD][TF][PPT][2], Y[SD][TF][PPT][2];
   __device__ __forceinline__ void zero() {
 #pragma unroll
-    for (int s = 0; s < 2; s++)
+    for (int s = 0; s < SD; s++)
 #pragma unroll
       for (int t = 0; t < TF; t++)
 #pragma unroll
@@ -329,20 +329,21 @@ template <int TF, int PPT> struct MacAcc {
   }
 };
 
-// One stored row into the accumulators of the sides S0 .. S1 - 1.
-template <int TF, int PPT, int S0, int S1>
-__device__ __forceinline__ void mac_row(const float4 *row, const int (&off)[PPT], const float4 *svr, int svt,
-                                        MacAcc<TF, PPT> &a) {
+// One stored row into the accumulators S0 .. S1 - 1 of a thread's sides (svr:
+// the row's operands of the thread's first side).
+template <int TF, int PPT, int SD, int S0, int S1>
+__device__ __forceinline__ void mac_row(const float4 *row, const int (&off)[PPT], const float4 *svr,
+                                        MacAcc<TF, PPT, SD> &a) {
   float4 e[PPT];
 #pragma unroll
   for (int k = 0; k < PPT; k++) e[k] = row[off[k]];
 #pragma unroll
-  for (int t = 0; t < TF; t++)
+  for (int s = S0; s < S1; s++)
 #pragma unroll
-    for (int s = S0; s < S1; s++)
+    for (int t = 0; t < TF; t++)
 #pragma unroll
       for (int uv = 0; uv < 2; uv++) {
-        const float4 q = svr[t * svt + s * 2 + uv];   // p0, m0, p1, m1
+        const float4 q = svr[(s * TF + t) * 2 + uv];   // p0, m0, p1, m1
         const float2 q0 = make_float2(q.x, q.y), q1 = make_float2(q.z, q.w);
 #pragma unroll
         for (int k = 0; k < PPT; k++) {
@@ -358,11 +359,15 @@ __device__ __forceinline__ void mac_row(const float4 *row, const int (&off)[PPT]
 }
 
 // Threads: `cw` warps side by side cover the channel pairs (PPT per lane), `H`
-// row shares of such warps take alternate rows of a chunk.
+// row shares of such warps take alternate rows of a chunk, with SD = 1 a warp
+// for each side of the quad.  CTAs per SM the registers are asked to allow.
 // (At one frame shared memory allows three CTAs: asking for four took registers
-// from the row loop, 2 to 10 % of the forward time.)
-template <int TF, int TH> struct MacOcc {
-  static constexpr int v = TH == 128 ? (TF <= 2 ? 3 : 2) : (TF == 1 ? 2 : 1);
+// from the row loop, 2 to 10 % of the forward time.  Side warps: three at two
+// frames forward, Nnum 19, 760 x 760 px, 31 planes 1885 -> 1745 us a projection,
+// Nnum 23 with two 719 -> 642; back projection, whose outputs need registers,
+// loses 3 to 5 % by the same.)
+template <int TF, int TH, int SD, bool FWD> struct MacOcc {
+  static constexpr int v = SD == 1 ? (TH == 256 ? (TF == 2 && FWD ? 3 : 2) : TF == 2 && FWD ? 2 : 1) : TH == 128 ? (TF <= 2 ? 3 : 2) : (TF == 1 ? 2 : 1);
 };
 
 // One CTA = one frequency quad {(uy, ux), (ux, uy)} and a group of planes.
@@ -397,8 +402,8 @@ template <int TF, int TH> struct MacOcc {
 // a helper warp (the last one) builds the next plane's operand table while the
 // current plane streams; back projection writes each plane's spectra when the
 // plane is done.
-template <int TF, bool FWD, int PPT, int TH>
-__global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>::v) k_mac(MacParams p) {
+template <int TF, bool FWD, int PPT, int TH, int SD>
+__global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH, SD, FWD>::v) k_mac(MacParams p) {
   constexpr bool HELP = FWD && TF == 1;         // a helper warp builds the operand tables, two in turn
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ int s_abort;
@@ -408,11 +413,11 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>
   const Layout &L = p.L;
   const int NN = L.NN, N = L.N, NP = L.NP, R = L.nrow, nT = L.nrowT, NN2 = 2 * L.NN;
   const int CH = p.chunk_rows, NST = p.stages, H = p.shares;
-  const int svt = 2 * R * 4;                                                 // sv stride between frames (float4)
+  const int svn = TF * 2 * R * 4;                                            // float4 of an operand table
   float4 *ring = reinterpret_cast<float4 *>(smraw);                          // [NST][CH][NP]
-  float4 *sv0 = ring + (size_t)NST * CH * NP;                                // [1|2][TF][2][R][2][2]
-  float2 *outs = reinterpret_cast<float2 *>(FWD ? sv0 : sv0 + TF * svt);     // [TF][side][u | u*][NN]
-  short4 *rowS = reinterpret_cast<short4 *>(FWD ? reinterpret_cast<float2 *>(sv0 + (HELP ? 2 : 1) * TF * svt) : outs + TF * 4 * NN);
+  float4 *sv0 = ring + (size_t)NST * CH * NP;                                // [1|2][2][R][2][TF][2]
+  float2 *outs = reinterpret_cast<float2 *>(FWD ? sv0 : sv0 + svn);     // [TF][side][u | u*][NN]
+  short4 *rowS = reinterpret_cast<short4 *>(FWD ? reinterpret_cast<float2 *>(sv0 + (HELP ? 2 : 1) * svn) : outs + TF * 4 * NN);
   unsigned long long *full = reinterpret_cast<unsigned long long *>(rowS + 3 * R);
   unsigned long long *svfull = full + NST;               // [2] operand table built (helper's lanes arrive)
   unsigned long long *svfree = svfull + 2;               // [2] operand table read (a lane of each warp arrives)
@@ -486,21 +491,23 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>
     for (int zl = 1; zl < z1 - z0; zl++) {
       const int b = zl & 1;
       if (zl > 1 && !mbar_wait(svfree + b, ((zl >> 1) - 1) & 1, p.wait_ns)) break;   // the waiting warps report it
-      build_sv<TF>(sv0 + b * TF * svt, p, G, z0 + zl, rowS, nhalf, selfp0, selfp1, kq, lane, 32);
+      build_sv<TF>(sv0 + b * svn, p, G, z0 + zl, rowS, nhalf, selfp0, selfp1, kq, lane, 32);
       mbar_arrive(svfull + b);
     }
     __syncthreads();   // the streaming warps' last barrier
     return;
   }
 
-  const int cw = nwarps / H;                     // column warps
-  const int h = warp / cw;                       // row share
-  const int p0 = (warp - h * cw) * 32 * PPT + lane;
+  const int cw = SD == 1 ? nwarps / (2 * H) : nwarps / H;   // column warps
+  const int hs = warp / cw;
+  const int h = SD == 1 ? hs >> 1 : hs;          // row share
+  const int side0 = SD == 1 ? hs & 1 : 0;        // first side of this thread
+  const int p0 = (warp - hs * cw) * 32 * PPT + lane;
   int off[PPT];                                  // this lane's channel pairs (repeating the last one past the end)
 #pragma unroll
   for (int k = 0; k < PPT; k++) off[k] = min(p0 + 32 * k, NP - 1);
 
-  MacAcc<TF, PPT> acc;
+  MacAcc<TF, PPT, SD> acc;
   acc.zero();
 
   bool dead = false;
@@ -526,19 +533,32 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>
       const int r1 = min(nrq, r0 + CH);
       const float4 *stage = ring + (size_t)slot * CH * NP;
       // the chunk's rows, one half block at a time: the transposable ones feed
-      // both sides, the others the half block's own
+      // both sides, the others the half block's own.  (One row per loop turn: the
+      // loops of two rows were slower throughout, the more code a row is - Nnum 15,
+      // 450 px, 31 planes: one frame 328 and 319 us a projection forward, four
+      // with side warps 951 and 916 - and rows read ahead by hand slower too, 996.)
       for (int bs = r0 >= R ? 1 : 0; bs * R < r1; bs++) {
         const int base = bs * R;
         const int lo = max(r0, base) - base, hi = min(r1, base + R) - base;   // half-block rows
-        const float4 *svb = sv0 + (HELP ? (zl & 1) * TF * svt : 0) + (size_t)bs * R * 4;
+        const float4 *svb = sv0 + (HELP ? (zl & 1) * svn : 0) + ((size_t)bs * R * 2 + side0) * 2 * TF;
         const float4 *srow = stage + (base - r0) * NP;
-        const int rb = min(hi, nT);
-#pragma unroll 2
-        for (int r = lo + h; r < rb; r += H) mac_row<TF, PPT, 0, 2>(srow + r * NP, off, svb + r * 4, svt, acc);
-        if (bs == 0) {
-          for (int r = max(lo, nT) + h; r < hi; r += H) mac_row<TF, PPT, 0, 1>(srow + r * NP, off, svb + r * 4, svt, acc);
+        if constexpr (SD == 1) {
+          const int re = bs == side0 ? hi : min(hi, nT);
+#pragma unroll 1
+          for (int r = lo + h; r < re; r += H) mac_row<TF, PPT, 1, 0, 1>(srow + r * NP, off, svb + r * 4 * TF, acc);
         } else {
-          for (int r = max(lo, nT) + h; r < hi; r += H) mac_row<TF, PPT, 1, 2>(srow + r * NP, off, svb + r * 4, svt, acc);
+          const int rb = min(hi, nT);
+#pragma unroll 1
+          for (int r = lo + h; r < rb; r += H) mac_row<TF, PPT, 2, 0, 2>(srow + r * NP, off, svb + r * 4 * TF, acc);
+          if (bs == 0) {
+#pragma unroll 1
+            for (int r = max(lo, nT) + h; r < hi; r += H)
+              mac_row<TF, PPT, 2, 0, 1>(srow + r * NP, off, svb + r * 4 * TF, acc);
+          } else {
+#pragma unroll 1
+            for (int r = max(lo, nT) + h; r < hi; r += H)
+              mac_row<TF, PPT, 2, 1, 2>(srow + r * NP, off, svb + r * 4 * TF, acc);
+          }
         }
       }
     }
@@ -568,7 +588,8 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>
               const int b = pr / N, a = pr - b * N;             // channel j = pr of side 0
               const int my = (N - 1 - b) * N + a, tr = a * N + b, mytr = (N - 1 - a) * N + b;
 #pragma unroll
-              for (int s = 0; s < 2; s++) {
+              for (int sd = 0; sd < SD; sd++) {
+                const int s = SD == 1 ? side0 : sd;
                 const int j = s ? tr : pr, m = s ? mytr : my;    // first channels of the pair at u and at u*
 #pragma unroll
                 for (int t = 0; t < TF; t++) {
@@ -584,8 +605,8 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH>
                     o[c1] = x;
                     o[c2] = y;
                   };
-                  put(ou, j, acc.X[s][t][k][0], acc.Y[s][t][k][0]);
-                  put(ov, m, acc.X[s][t][k][1], acc.Y[s][t][k][1]);
+                  put(ou, j, acc.X[sd][t][k][0], acc.Y[sd][t][k][0]);
+                  put(ov, m, acc.X[sd][t][k][1], acc.Y[sd][t][k][1]);
                 }
               }
             }
@@ -925,18 +946,34 @@ int mac_max_frames() { return 4; }
 // to make (Nnum 5, 31 planes of 250 x 300 px, four frames: back 129 us a launch with
 // four shares, 76 with two, 58 with one; Nnum 7, 25 planes, one frame 44, 31, 31).
 // Two pairs per lane from 33 pairs on.
-MacThreads mac_threads(const Layout &L, int split) {
+// A warp for each side halves a thread's accumulators and its loop's code and
+// doubles the warps, for twice the reads of the streamed rows from shared memory;
+// us a projection with sides together and apart, back | forward:
+//   Nnum  5, 250 px, 31 planes: 1 frame  39, 48 |  58, 60;  4 frames 175, 143 | 204, 161
+//   Nnum 11, 330 px, 31 planes: 1 frame 138, 122 | 147, 129; 4 frames 721, 502 | 626, 457
+//   Nnum 15, 450 px, 31 planes: 1 frame 303, 311 | 319, 357; 2 frames 561, 613 | 557, 613;
+//                               3 frames 765, 704 | 798, 742; 4 frames 956, 900 | 969, 916
+//   Nnum 19, 380 px, 21 planes: 1 frame 257, 246 | 282, 349; 2 frames 475, 408 | 499, 459;
+//                               4 frames 1025, 842 | 811, 711
+//   Nnum 23, 460 px, 15 planes: 1 frame 388, 377 | 425, 545; 2 frames 796, 634 | 706, 642;
+//                               4 frames 1397, 1122 | 1389, 1097
+// From seven column warps on a CTA has no room for more.
+MacThreads mac_threads(const Layout &L, int split, int frames, bool fwd) {
   MacThreads t;
   t.ppt = L.NP > 32 ? 2 : 1;
   t.cw = (L.NP + 32 * t.ppt - 1) / (32 * t.ppt);
-  t.shares = t.cw == 1 ? split : std::max(1, std::min(4 * split / t.cw, 8 / t.cw));
+  t.sides = t.cw == 1   ? (frames >= 2 || t.ppt == 2 ? 1 : 2)
+            : t.cw == 2 ? (frames >= 3 ? 1 : 2)
+            : t.cw <= 6 ? (frames >= 2 || !fwd ? 1 : 2)
+                        : 2;
+  t.shares = t.sides == 1 && t.cw > 1 ? std::max(1, 4 / t.cw) : t.cw == 1 ? split : std::max(1, std::min(4 * split / t.cw, 8 / t.cw));
   return t;
 }
 
 template <int TF, bool FWD>
 static cudaError_t launch_mac_tf(const MacParams &p0, cudaStream_t s) {
   MacParams p = p0;
-  const MacThreads th = mac_threads(p.L, p.split);
+  const MacThreads th = mac_threads(p.L, p.split, TF, FWD);
   p.shares = th.shares;
   const size_t sm = mac_smem_bytes(p.L, TF, p.stages, p.chunk_rows, FWD);
   int ctas = 0;
@@ -946,9 +983,15 @@ static cudaError_t launch_mac_tf(const MacParams &p0, cudaStream_t s) {
     ctas += G.nquads * ((G.nz + G.zgroup - 1) / G.zgroup);
   }
   const dim3 grid(ctas);
-  const int threads = 32 * th.cw * th.shares, block = threads + (FWD && TF == 1 ? 32 : 0);   // and the helper warp
-  void (*fn)(MacParams) = threads <= 128 ? (th.ppt == 2 ? k_mac<TF, FWD, 2, 128> : k_mac<TF, FWD, 1, 128>)
-                                       : (th.ppt == 2 ? k_mac<TF, FWD, 2, 256> : k_mac<TF, FWD, 1, 256>);
+  const int threads = 32 * th.cw * th.shares * (th.sides == 1 ? 2 : 1);
+  const int block = threads + (FWD && TF == 1 ? 32 : 0);   // and the helper warp
+  void (*fn)(MacParams);
+  if (th.sides == 1) {
+    fn = th.ppt == 1 ? k_mac<TF, FWD, 1, 256, 1> : threads <= 256 ? k_mac<TF, FWD, 2, 256, 1> : k_mac<TF, FWD, 2, 384, 1>;
+  } else {
+    fn = threads <= 128 ? (th.ppt == 2 ? k_mac<TF, FWD, 2, 128, 2> : k_mac<TF, FWD, 1, 128, 2>)
+                        : (th.ppt == 2 ? k_mac<TF, FWD, 2, 256, 2> : k_mac<TF, FWD, 1, 256, 2>);
+  }
   cudaError_t e = set_smem((const void *)fn, sm);
   if (e != cudaSuccess) return e;
   fn<<<grid, block, sm, s>>>(p);
