@@ -222,7 +222,8 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // Wait for phase `parity` of `bar`; false after `limit_ns` nanoseconds.
 __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned parity,
                                           unsigned long long limit_ns) {
-  if (mbar_try_wait(bar, parity)) return true;
+  for (int i = 0; i < 32; i++)   // (the timer is slow to read)
+    if (mbar_try_wait(bar, parity)) return true;
   const unsigned long long t0 = global_ns();
   while (!mbar_try_wait(bar, parity))
     if (global_ns() - t0 > limit_ns) return false;
@@ -399,12 +400,13 @@ template <int TF, int TH, int SD, bool FWD> struct MacOcc {
 // The stored rows stream through a ring of shared-memory stages filled by
 // bulk copies (crossing plane boundaries).  Forward projection accumulates the
 // planes of the group (the group sums are added by the inverse transform), and
-// a helper warp (the last one) builds the next plane's operand table while the
+// a helper warp (the last but one) builds the next plane's operand table while the
 // current plane streams; back projection writes each plane's spectra when the
 // plane is done.
 template <int TF, bool FWD, int PPT, int TH, int SD>
-__global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH, SD, FWD>::v) k_mac(MacParams p) {
-  constexpr bool HELP = FWD && TF == 1;         // a helper warp builds the operand tables, two in turn
+__global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 64 : 0), MacOcc<TF, TH, SD, FWD>::v) k_mac(MacParams p) {
+  constexpr bool HELP = FWD && TF == 1;         // a helper warp builds the operand tables, two in turn, and a copy
+                                                // warp refills the ring
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ int s_abort;
   __shared__ int s_issued;                      // chunks handed to the bulk-copy engine
@@ -421,10 +423,11 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH,
   unsigned long long *full = reinterpret_cast<unsigned long long *>(rowS + 3 * R);
   unsigned long long *svfull = full + NST;               // [2] operand table built (helper's lanes arrive)
   unsigned long long *svfree = svfull + 2;               // [2] operand table read (a lane of each warp arrives)
-  int *released = reinterpret_cast<int *>(svfree + 2);   // [NST] warps done with each slot, ever
+  unsigned long long *empty = svfree + 2;                // copy warp: [NST] chunk read (a lane of each warp arrives)
+  int *released = reinterpret_cast<int *>(empty);        // else: [NST] warps done with each slot, ever
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nwarps = (blockDim.x >> 5) - (HELP ? 1 : 0);  // streaming warps
+  const int nwarps = (blockDim.x >> 5) - (HELP ? 2 : 0);  // streaming warps
   const int nthreads = 32 * nwarps;
 
   // quad k = ux (ux + 1) / 2 + uy, uy <= ux
@@ -449,9 +452,13 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH,
   const size_t halfElems = (size_t)R * NP;       // float4
 
   // Chunk g goes to ring slot g % NST.  Thread 0 fills the whole ring before
-  // anything else; after that, the warp that releases a slot last (each warp
+  // anything else.  After that, the warp that releases a slot last (each warp
   // counts itself out once it has finished its rows of the chunk) refills it at
-  // once with chunk g + NST, so no thread ever waits for a slot to drain.
+  // once with chunk g + NST, so no thread ever waits for a slot to drain; forward at
+  // one frame, where the registers allow one warp more, a copy warp does so as soon
+  // as every streaming warp has arrived on the slot's `empty` barrier (Nnum 23, 460
+  // px, 15 planes 425 -> 383 us a projection, Nnum 19, 760 px, 31 planes 1143 -> 1104,
+  // Nnum 15, 450 px 317 -> 312; with more frames it spills or evens out).
   // p.drop_chunk >= 0 (a test of the bounded waits only): the first CTA never
   // issues that chunk, so the waits on its slot run out after p.wait_ns
   const int drop = blockIdx.x == 0 ? p.drop_chunk : -1;
@@ -468,7 +475,8 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH,
   if (tid == 0) {
     for (int i = 0; i < NST; i++) {
       mbar_init(full + i, 1);
-      released[i] = 0;
+      if (HELP) mbar_init(empty + i, nwarps);
+      else released[i] = 0;
     }
     for (int i = 0; i < 2; i++) {
       mbar_init(svfull + i, 32);
@@ -486,6 +494,25 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH,
   build_sv<TF>(sv0, p, G, FWD ? z0 : 0, rowS, nhalf, selfp0, selfp1, kq, tid, blockDim.x);
   __syncthreads();
 
+  if (HELP && warp == nwarps + 1) {
+    // copy warp
+    if (lane == 0) {
+      int sl = 0, par = 0;
+      for (int g = min(NST, total); g < total; g++) {
+        if (!mbar_wait(empty + sl, par, p.wait_ns)) {
+          *abortf = 1;
+          atomicExch(p.err, 2);
+          break;
+        }
+        fence_proxy_async_smem();   // the warps' reads come before the copy that overwrites them
+        issue(g, s_plane);
+        s_issued = g + 1;
+        if (++sl == NST) { sl = 0; par ^= 1; }
+      }
+    }
+    __syncthreads();   // the streaming warps' last barrier
+    return;
+  }
   if (HELP && warp == nwarps) {
     // helper warp: operand tables of the planes after the first, two in turn
     for (int zl = 1; zl < z1 - z0; zl++) {
@@ -564,15 +591,19 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 32 : 0), MacOcc<TF, TH,
     }
     __syncwarp();
     if (lane == 0 && !dead) {
-      __threadfence_block();                       // this warp's reads of the slot come first
-      const int before = atomicAdd(released + slot, 1);
-      if (before == round * nwarps + nwarps - 1 && g + NST < total && !*abortf) {
-        __threadfence_block();
-        fence_proxy_async_smem();                  // ... before the bulk copy that overwrites it
-        issue(g + NST, s_plane);
-        atomicAdd(&s_issued, 1);
+      if (HELP) {
+        mbar_arrive(empty + slot);
+        if (ch == cpb - 1) mbar_arrive(svfree + (zl & 1));
+      } else {
+        __threadfence_block();                       // this warp's reads of the slot come first
+        const int before = atomicAdd(released + slot, 1);
+        if (before == round * nwarps + nwarps - 1 && g + NST < total && !*abortf) {
+          __threadfence_block();
+          fence_proxy_async_smem();                  // ... before the bulk copy that overwrites it
+          issue(g + NST, s_plane);
+          atomicAdd(&s_issued, 1);
+        }
       }
-      if (HELP && ch == cpb - 1) mbar_arrive(svfree + (zl & 1));
     }
 
     const bool out_due = (ch == cpb - 1) && (!FWD || zi + 1 == z1);
@@ -984,7 +1015,7 @@ static cudaError_t launch_mac_tf(const MacParams &p0, cudaStream_t s) {
   }
   const dim3 grid(ctas);
   const int threads = 32 * th.cw * th.shares * (th.sides == 1 ? 2 : 1);
-  const int block = threads + (FWD && TF == 1 ? 32 : 0);   // and the helper warp
+  const int block = threads + (FWD && TF == 1 ? 64 : 0);   // and the helper and copy warps
   void (*fn)(MacParams);
   if (th.sides == 1) {
     fn = th.ppt == 1 ? k_mac<TF, FWD, 1, 256, 1> : threads <= 256 ? k_mac<TF, FWD, 2, 256, 1> : k_mac<TF, FWD, 2, 384, 1>;
