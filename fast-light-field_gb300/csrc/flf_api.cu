@@ -851,25 +851,28 @@ int join_streams(flf_ctx *ctx, cudaStream_t s) {
   return FLF_OK;
 }
 
-// Stored rows per ring stage where none were asked for: the even number whose
-// chunks cost least (a chunk costs about four rows' time in barriers and copies
-// beside its own rows) among those that leave room for `want` CTAs per SM, as
-// many as the registers of nt frames allow.  Nnum 15, two stages, one frame: 12
-// rows forward, 16 back (three CTAs; full field 1864 us with 12 rows against 1992
-// with 10 and 2038 with 16 in two CTAs).
+// Stored rows per ring stage where none were asked for: a chunk costs about four
+// rows' time beside its own rows, so the most (up to 24) that leave room for `want`
+// CTAs per SM, as many as the registers of nt frames allow (six of a small Nnum's
+// two-warp CTAs), evened out over the chunks of a half block.  Nnum 15 (72 rows), two stages, one frame: 12 rows forward,
+// 15 back (three CTAs; full field 1864 us with 12 rows against 1992 with 10 and 2038
+// with 16 in two CTAs); four frames, 450 px, 31 planes back 996 us with 6 rows, 925
+// with 8, 864 with 12 and 1062 with 16 in one CTA.
 int auto_chunk_rows(const Layout &L, int nt, int stages, bool fwd) {
   const size_t sm_bytes = 228 * 1024, cta_reserve = 1024 + 512;   // of the SM; system and static use of a CTA
-  for (int want = nt <= 2 ? 3 : 2; want >= 1; want--) {
-    int best = 0, cost = 1 << 30;
-    for (int ch = want > 1 ? 6 : 2; ch <= 16; ch += 2) {
+  for (int want = L.NP <= 64 ? 6 : nt <= 2 ? 3 : 2; want >= 1; want--) {
+    int most = 0;
+    for (int ch = want > 1 ? 6 : 1; ch <= 24; ch++) {
       const size_t b = mac_smem_bytes(L, nt, stages, ch, fwd);
       if (b > kMacSmemMax || want * (b + cta_reserve) > sm_bytes) break;
-      const int c = (2 * L.nrow + ch - 1) / ch * (ch + 4);
-      if (c <= cost) { cost = c; best = ch; }
+      most = ch;
     }
-    if (best) return best;
+    if (most) {
+      const int chunks = (L.nrow + most - 1) / most;
+      return (L.nrow + chunks - 1) / chunks;
+    }
   }
-  return 2;
+  return 1;
 }
 
 // Launch shape of the multiply-accumulate of nt frames in direction dir: the

@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 64 : 0), MacOcc<TF, TH,
   unsigned long long *svfull = full + NST;               // [2] operand table built (helper's lanes arrive)
   unsigned long long *svfree = svfull + 2;               // [2] operand table read (a lane of each warp arrives)
   unsigned long long *empty = svfree + 2;                // copy warp: [NST] chunk read (a lane of each warp arrives)
-  int *released = reinterpret_cast<int *>(empty);        // else: [NST] warps done with each slot, ever
+  int *released = reinterpret_cast<int *>(empty);        // else: [NST] warps done with each slot
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nwarps = (blockDim.x >> 5) - (HELP ? 2 : 0);  // streaming warps
@@ -446,8 +446,8 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 64 : 0), MacOcc<TF, TH,
   const bool selfp0 = (uy == 0) || (2 * uy == G.f), selfp1 = (ux == 0) || (2 * ux == G.f);
   const int z0 = zgi * G.zgroup;
   const int z1 = min(z0 + G.zgroup, G.nz);
-  const int nrq = nhalf * R;                     // stored rows of the quad per plane
-  const int cpb = (nrq + CH - 1) / CH;           // chunks per (quad, plane)
+  const int cph = (R + CH - 1) / CH;             // chunks per half block, none across two
+  const int cpb = nhalf * cph;                   // chunks per (quad, plane)
   const int total = (z1 - z0) * cpb;
   const size_t halfElems = (size_t)R * NP;       // float4
 
@@ -465,9 +465,10 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 64 : 0), MacOcc<TF, TH,
   auto issue = [&](int gn, const int *planes) {
     if (gn == drop) return;
     const int zl_n = gn / cpb, ch_n = gn - zl_n * cpb, sl = gn % NST;
-    const int r0 = ch_n * CH;
-    const int nr = min(CH, nrq - r0);
-    const float4 *src = G.P + ((long long)planes[zl_n] * G.nkp + hb0) * (long long)halfElems + (long long)r0 * NP;
+    const int bs_n = ch_n >= cph ? 1 : 0;
+    const int r0 = (ch_n - bs_n * cph) * CH;
+    const int nr = min(CH, R - r0);
+    const float4 *src = G.P + ((long long)planes[zl_n] * G.nkp + hb0 + bs_n) * (long long)halfElems + (long long)r0 * NP;
     const unsigned bytes = (unsigned)(nr * NP * sizeof(float4));
     mbar_arrive_expect_tx(full + sl, bytes);
     bulk_g2s(ring + (size_t)sl * CH * NP, src, bytes, full + sl);
@@ -538,54 +539,50 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 64 : 0), MacOcc<TF, TH,
   acc.zero();
 
   bool dead = false;
-  int zl = 0, ch = 0, slot = 0;
-  int round = 0;
+  // The chunk's place, stepped along: half block, its first row, ring slot and phase.
+  int zl = 0, bs = 0, lo = 0, slot = 0;
+  unsigned phase = 0;
+  const float4 *stage = ring;
+  const float4 *svz = sv0 + side0 * 2 * TF;      // operands of the plane, the thread's first side
   for (int g = 0; g < total; g++) {
     const int zi = z0 + zl;
-    if (FWD && !HELP && ch == 0 && zl > 0) {
+    const bool first = bs == 0 && lo == 0 && zl > 0;                // first chunk of a later plane
+    const bool last = bs == nhalf - 1 && lo + CH >= R;              // last chunk of a plane
+    if (FWD && !HELP && first) {
       bar_sync(nthreads);   // every warp is done with plane zi - 1
       build_sv<TF>(sv0, p, G, zi, rowS, nhalf, selfp0, selfp1, kq, tid, nthreads);
       bar_sync(nthreads);
     }
-    if (*abortf) dead = true;
     // table zl: the helper's fill number zl >> 1 of buffer zl & 1 (buffer 0's first one is not counted)
-    if (!dead && ((HELP && ch == 0 && zl > 0 && !mbar_wait(svfull + (zl & 1), ((zl - 1) >> 1) & 1, p.wait_ns)) ||
-                  !mbar_wait(full + slot, round & 1, p.wait_ns))) {
+    if (!dead && ((HELP && first && !mbar_wait(svfull + (zl & 1), ((zl - 1) >> 1) & 1, p.wait_ns)) ||
+                  !mbar_wait(full + slot, phase, p.wait_ns))) {
       dead = true;
       *abortf = 1;
       atomicExch(p.err, 2);
     }
     if (!dead) {
-      const int r0 = ch * CH;
-      const int r1 = min(nrq, r0 + CH);
-      const float4 *stage = ring + (size_t)slot * CH * NP;
-      // the chunk's rows, one half block at a time: the transposable ones feed
-      // both sides, the others the half block's own.  (One row per loop turn: the
-      // loops of two rows were slower throughout, the more code a row is - Nnum 15,
-      // 450 px, 31 planes: one frame 328 and 319 us a projection forward, four
-      // with side warps 951 and 916 - and rows read ahead by hand slower too, 996.)
-      for (int bs = r0 >= R ? 1 : 0; bs * R < r1; bs++) {
-        const int base = bs * R;
-        const int lo = max(r0, base) - base, hi = min(r1, base + R) - base;   // half-block rows
-        const float4 *svb = sv0 + (HELP ? (zl & 1) * svn : 0) + ((size_t)bs * R * 2 + side0) * 2 * TF;
-        const float4 *srow = stage + (base - r0) * NP;
-        if constexpr (SD == 1) {
-          const int re = bs == side0 ? hi : min(hi, nT);
+      // the chunk's rows: the transposable ones feed both sides, the others the
+      // half block's own.  (One row per loop turn: loops of two rows were slower
+      // throughout, the more code a row is - Nnum 15, 450 px, 31 planes: one frame
+      // 328 and 319 us a projection forward, four with side warps 951 and 916 - and
+      // rows read ahead by hand slower too, 996.)
+      const int nr = min(CH, R - lo), nb = min(nr, nT - lo);   // rows; transposable ones (may be negative)
+      const float4 *e = stage + h * NP, *q = svz + ((size_t)bs * R + lo + h) * 4 * TF;
+      const int estep = H * NP, qstep = H * 4 * TF;
+      int n = h;
+      if constexpr (SD == 1) {
+        const int ne = bs == side0 ? nr : nb;
 #pragma unroll 1
-          for (int r = lo + h; r < re; r += H) mac_row<TF, PPT, 1, 0, 1>(srow + r * NP, off, svb + r * 4 * TF, acc);
+        for (; n < ne; n += H, e += estep, q += qstep) mac_row<TF, PPT, 1, 0, 1>(e, off, q, acc);
+      } else {
+#pragma unroll 1
+        for (; n < nb; n += H, e += estep, q += qstep) mac_row<TF, PPT, 2, 0, 2>(e, off, q, acc);
+        if (bs == 0) {
+#pragma unroll 1
+          for (; n < nr; n += H, e += estep, q += qstep) mac_row<TF, PPT, 2, 0, 1>(e, off, q, acc);
         } else {
-          const int rb = min(hi, nT);
 #pragma unroll 1
-          for (int r = lo + h; r < rb; r += H) mac_row<TF, PPT, 2, 0, 2>(srow + r * NP, off, svb + r * 4 * TF, acc);
-          if (bs == 0) {
-#pragma unroll 1
-            for (int r = max(lo, nT) + h; r < hi; r += H)
-              mac_row<TF, PPT, 2, 0, 1>(srow + r * NP, off, svb + r * 4 * TF, acc);
-          } else {
-#pragma unroll 1
-            for (int r = max(lo, nT) + h; r < hi; r += H)
-              mac_row<TF, PPT, 2, 1, 2>(srow + r * NP, off, svb + r * 4 * TF, acc);
-          }
+          for (; n < nr; n += H, e += estep, q += qstep) mac_row<TF, PPT, 2, 1, 2>(e, off, q, acc);
         }
       }
     }
@@ -593,11 +590,11 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 64 : 0), MacOcc<TF, TH,
     if (lane == 0 && !dead) {
       if (HELP) {
         mbar_arrive(empty + slot);
-        if (ch == cpb - 1) mbar_arrive(svfree + (zl & 1));
+        if (last) mbar_arrive(svfree + (zl & 1));
       } else {
         __threadfence_block();                       // this warp's reads of the slot come first
-        const int before = atomicAdd(released + slot, 1);
-        if (before == round * nwarps + nwarps - 1 && g + NST < total && !*abortf) {
+        if (atomicAdd(released + slot, 1) == nwarps - 1 && g + NST < total && !*abortf) {
+          released[slot] = 0;
           __threadfence_block();
           fence_proxy_async_smem();                  // ... before the bulk copy that overwrites it
           issue(g + NST, s_plane);
@@ -606,7 +603,7 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 64 : 0), MacOcc<TF, TH,
       }
     }
 
-    const bool out_due = (ch == cpb - 1) && (!FWD || zi + 1 == z1);
+    const bool out_due = last && (!FWD || zi + 1 == z1);
     if (out_due) {
       // the row shares add their channel values into outs in share order
       if (FWD) bar_sync(nthreads);   // every warp is done with the operand tables
@@ -675,8 +672,21 @@ __global__ void __launch_bounds__(TH + (FWD && TF == 1 ? 64 : 0), MacOcc<TF, TH,
       acc.zero();
       if (g + 1 < total) bar_sync(nthreads);   // the exchange buffer is free again
     }
-    if (++ch == cpb) { ch = 0; zl++; }
-    if (++slot == NST) { slot = 0; round++; }
+    lo += CH;
+    if (lo >= R) {
+      lo = 0;
+      if (++bs == nhalf) {
+        bs = 0;
+        zl++;
+        if (HELP) svz += (zl & 1) ? svn : -svn;
+      }
+    }
+    stage += CH * NP;
+    if (++slot == NST) {
+      slot = 0;
+      stage = ring;
+      phase ^= 1;
+    }
   }
   // Never leave a bulk copy in flight into this CTA's shared memory.
   __syncthreads();
