@@ -1228,22 +1228,35 @@ __global__ void __launch_bounds__(tma16_threads(S), 1)
 // the gradient is the same bits on every run; with one chunk (p.part null) the
 // CTA adds its tile to dW itself (one writer per element), and the nine (dz, dy)
 // have CTAs of their own (ny = 1), three warps sharing a row.
-// 16 -> 16 channels at 4 x 24 x 128 x 128, weight and bias gradient together: 1880
-// us with one CTA per tap (x and dy staged 27 times, an index division per 16
-// bytes) and one channel per thread in the bias sums, 161 us now.
-constexpr int kWgRows = 4, kWgSlots = 5, kWgWarps = 12;
+// A thirteenth warp keeps the ring filled with tensor-map copies (a row block of x
+// with its halo, one of dy; zeros outside the volume; the 32- or 64-byte swizzle is
+// the one ldmatrix wants), a full and an empty barrier per slot, so a row block costs
+// its reader no index arithmetic and no CTA barrier.
+// 16 -> 16 channels at 4 x 24 x 128 x 128: 129 us with 16-byte copies by the readers
+// (tensor pipe 29 % busy; seven of eight instructions staged), 68 us (56 %) now, the
+// copies alone 44; 24 x 456 x 456 with the bias sums 492 -> 265 us, 32 -> 32 at 12 x
+// 228 x 228 183 -> 140, 64 -> 64 at 6 x 114 x 114 116 -> 94.  (One CTA per tap, staging
+// x and dy 27 times, took 1880 us with the bias sums.)
+constexpr int kWgRows = 4, kWgSlots = 5, kWgWarps = 12, kWgThreads = 32 * (kWgWarps + 1);
+template <int CM, int CN, int TX> struct WgTile {
+  static constexpr int XV = TX + 2;
+  static constexpr size_t XB = (size_t)kWgRows * XV * CM * sizeof(bf16), DB = (size_t)kWgRows * TX * CN * sizeof(bf16);
+  static constexpr size_t XS = (XB + 1023) / 1024 * 1024, SLOT = XS + DB;   // a slot: x rows | dy rows
+  static constexpr size_t RING = kWgSlots * SLOT, RED = (size_t)9 * CM * CN * sizeof(float);
+  static constexpr size_t BARS = RING > RED ? RING : RED, SMEM = BARS + (2 * kWgSlots + 1) * 8;
+  static_assert(BARS % 8 == 0 && SLOT % 1024 == 0, "the swizzle counts from the slot's base");
+};
 template <int CM, int CN, int TX>
-constexpr size_t wgrad_smem() {
-  const size_t ring = (size_t)kWgSlots * kWgRows * ((TX + 2) * CM + TX * CN) * sizeof(bf16);
-  const size_t red = (size_t)9 * CM * CN * sizeof(float);
-  return ring > red ? ring : red;
-}
-template <int CM, int CN, int TX>
-__global__ void __launch_bounds__(32 * kWgWarps, 1) k_conv3d_wgrad(WgradParams p) {
-  constexpr int RA = CM / 8, RB = CN / 8, XV = TX + 2, NT = 32 * kWgWarps;
-  extern __shared__ __align__(128) unsigned char wgsm[];
-  bf16 *Xs = reinterpret_cast<bf16 *>(wgsm);                               // [slot][row][XV][CM]
-  bf16 *Ds = Xs + (size_t)kWgSlots * kWgRows * XV * CM;                    // [slot][row][TX][CN]
+__global__ void __launch_bounds__(kWgThreads, 1)
+    k_conv3d_wgrad(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtensorMap td, WgradParams p) {
+  typedef WgTile<CM, CN, TX> T;
+  constexpr int RA = CM / 8, RB = CN / 8, XV = T::XV, NT = kWgThreads;
+  constexpr int U = CM * CN > 256 ? 1 : 2;
+  extern __shared__ __align__(1024) unsigned char wgsm[];
+  volatile int *abort_s = reinterpret_cast<volatile int *>(wgsm + T::BARS + 2 * kWgSlots * 8);
+  const uint32_t ring = su32(wgsm), bar_s = ring + (uint32_t)T::BARS;
+  auto full = [&](uint32_t n) { return bar_s + 8u * (n % kWgSlots); };                // load n has arrived
+  auto empty = [&](uint32_t n) { return bar_s + 8u * (kWgSlots + n % kWgSlots); };    // its last reader is done
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int parts = p.ny == 3 ? 3 : 9;                                     // (dz) or (dz, dy) per chunk
   const int part = blockIdx.x % parts;
@@ -1257,6 +1270,14 @@ __global__ void __launch_bounds__(32 * kWgWarps, 1) k_conv3d_wgrad(WgradParams p
   const int nblk = (p.Y + kWgRows - 1) / kWgRows, nseg = (p.X + TX - 1) / TX;
   const long long items = (long long)p.B * p.Z * nseg * nblk;
   const long long i1 = min(items, (chunk + 1) * p.chunk);
+  if (tid == 0) {
+    for (int i = 0; i < kWgSlots; i++) {
+      net_mbar_init(full(i), 1);
+      net_mbar_init(empty(i), kWgWarps);
+    }
+    *abort_s = 0;
+  }
+  __syncthreads();
 
   float acc[3][CM / 16][CN / 8][4];
 #pragma unroll
@@ -1269,88 +1290,103 @@ __global__ void __launch_bounds__(32 * kWgWarps, 1) k_conv3d_wgrad(WgradParams p
         for (int e = 0; e < 4; e++) acc[d][i][j][e] = 0.f;
   const int mat = lane >> 3, r8 = lane & 7;
 
-  for (long long it = chunk * p.chunk; it < i1;) {
+  uint32_t n = 0;          // loads so far (producer), number of the run's first load (the others)
+  for (long long it = chunk * p.chunk; it < i1 && !*abort_s;) {
     // a run: consecutive row blocks [kb, ke) of one (b, z, segment)
     const int kb = (int)(it % nblk);
     const int ke = (int)min((long long)nblk, kb + (i1 - it));
     const long long col = it / nblk;
     it += ke - kb;
-    const int seg = (int)(col % nseg);
+    const int x0 = (int)(col % nseg) * TX;
     const long long bz = col / nseg;
     const int z = (int)(bz % p.Z), zx = z + dz - 1;
     if (zx < 0 || zx >= p.Z) continue;
-    const int x0 = seg * TX, xw = min(TX, p.X - x0);
-    const int k16 = (xw + 15) >> 4;                                        // 16-voxel steps
-    const bf16 *xs = p.x + ((bz - z + zx) * p.Y * p.X + x0 - 1) * p.Ci + ci0;   // voxel x0 - 1 of row 0
-    const bf16 *ds = p.dy + (bz * p.Y * p.X + x0) * p.Co + co0;
-    // rows of block k into its slot; voxels outside the volume (and dy beyond the
-    // segment or the run) are zeros
-    auto load = [&](int k) {
-      const int slot = (k - kb + 1) % kWgSlots;
-      const int xu = (16 * k16 + 2) * RA, du = 16 * k16 * RB;
-      for (int i = tid; i < kWgRows * xu; i += NT) {
-        const int r = i / xu, e = i - r * xu, v = e / RA, c = e - v * RA;
-        const int y = kWgRows * k + r, x = x0 - 1 + v;
-        const bool ok = y >= 0 && y < p.Y && x >= 0 && x < p.X;
-        cp16(su32(Xs + ((size_t)(slot * kWgRows + r) * XV + v) * CM) + ((c ^ swz<RA>(v)) << 4),
-             ok ? xs + ((long long)y * p.X + v) * p.Ci + c * 8 : p.x, ok);
-      }
-      if (k >= kb && k < ke)
-        for (int i = tid; i < kWgRows * du; i += NT) {
-          const int r = i / du, e = i - r * du, v = e / RB, c = e - v * RB;
-          const int y = kWgRows * k + r;
-          const bool ok = y < p.Y && v < xw;
-          cp16(su32(Ds + ((size_t)(slot * kWgRows + r) * TX + v) * CN) + ((c ^ swz<RB>(v)) << 4),
-               ok ? ds + ((long long)y * p.X + v) * p.Co + c * 8 : p.dy, ok);
+    if (warp == kWgWarps) {
+      // the copies: x rows of blocks kb - 1 .. ke, dy rows of kb .. ke - 1; voxels outside
+      // the volume arrive as zeros
+      if (lane == 0) {
+        const int b = (int)(bz / p.Z);
+        for (int k = kb - 1; k <= ke; k++, n++) {
+          if (n >= kWgSlots && !role_wait(empty(n), (n / kWgSlots - 1) & 1, abort_s, 40)) break;
+          const uint32_t slot = ring + (n % kWgSlots) * (uint32_t)T::SLOT;
+          const bool own = k >= kb && k < ke;
+          net_expect_tx(full(n), (uint32_t)(T::XB + (own ? T::DB : 0)));
+          tma_load_5d(slot, &tx, ci0, x0 - 1, kWgRows * k, zx, b, full(n));
+          if (own) tma_load_5d(slot + (uint32_t)T::XS, &td, co0, x0, kWgRows * k, z, b, full(n));
         }
-    };
-    for (int k = kb - 1; k <= kb + 2; k++) {
-      if (k <= ke) load(k);
-      cp_commit();
+      }
+      continue;
     }
+    const int k16 = (min(TX, p.X - x0) + 15) >> 4;                         // 16-voxel steps
+    if (!role_wait(full(n), (n / kWgSlots) & 1, abort_s, 41) ||
+        !role_wait(full(n + 1), ((n + 1) / kWgSlots) & 1, abort_s, 41))
+      break;
     for (int k = kb; k < ke; k++) {
-      cp_wait<1>();        // blocks up to k + 1 have arrived
-      __syncthreads();     // for every warp, and block k - 2's slot is free
-      if (k + 3 <= ke) load(k + 3);
-      cp_commit();
+      const uint32_t m = n + (k - kb + 1);                                 // block k's load
+      if (!role_wait(full(m + 1), ((m + 1) / kWgSlots) & 1, abort_s, 41)) break;
       if (kWgRows * k + wr < p.Y) {
         const int j = wr + wy - 1;                                         // x row of the tap, relative to the block
-        const int xk = j < 0 ? k - 1 : j >= kWgRows ? k + 1 : k;
-        const bf16 *xr = Xs + (size_t)(((xk - kb + 1) % kWgSlots) * kWgRows + (j & (kWgRows - 1))) * XV * CM;
-        const bf16 *dr = Ds + (size_t)(((k - kb + 1) % kWgSlots) * kWgRows + wr) * TX * CN;
+        const uint32_t xn = j < 0 ? m - 1 : j >= kWgRows ? m + 1 : m;
+        const uint32_t xs = ring + (xn % kWgSlots) * (uint32_t)T::SLOT;
+        const uint32_t ds = ring + (m % kWgSlots) * (uint32_t)T::SLOT + (uint32_t)T::XS;
+        // ldmatrix addresses of the first step; the swizzle repeats after 16 voxels.
+        // A[ci][voxel] from rows of ci: transposed 8x8 blocks, d voxels further
+        uint32_t xa[3], da;
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+          const int v = (j & (kWgRows - 1)) * XV + 16 * k0s + d + r8 + 8 * (mat >> 1);
+          xa[d] = xs + v * (2 * CM) + (((mat & 1) ^ swz<RA>(v)) << 4);
+        }
+        {
+          const int v = wr * TX + 16 * k0s + r8 + 8 * (mat & 1);
+          da = ds + v * (2 * CN) + (((mat >> 1) ^ swz<RB>(v)) << 4);
+        }
+#pragma unroll U
         for (int ks = k0s; ks < k16; ks += kss) {
           uint32_t bq[CN / 16][4];
 #pragma unroll
-          for (int n2 = 0; n2 < CN / 16; n2++) {
-            const int row = 16 * ks + r8 + 8 * (mat & 1), c = n2 * 2 + (mat >> 1);
-            ldsm4t(su32(dr + row * CN) + ((c ^ swz<RB>(row)) << 4), bq[n2][0], bq[n2][1], bq[n2][2], bq[n2][3]);
-          }
+          for (int n2 = 0; n2 < CN / 16; n2++) ldsm4t(da ^ (n2 << 5), bq[n2][0], bq[n2][1], bq[n2][2], bq[n2][3]);
+          da += kss * 32 * CN;
 #pragma unroll
           for (int d = 0; d < 3; d++) {
-            // A[ci][voxel] from rows of ci: transposed 8x8 blocks, d voxels further
 #pragma unroll
             for (int mt = 0; mt < CM / 16; mt++) {
-              const int row = 16 * ks + d + r8 + 8 * (mat >> 1), c = mt * 2 + (mat & 1);
               uint32_t a[4];
-              ldsm4t(su32(xr + row * CM) + ((c ^ swz<RA>(row)) << 4), a[0], a[1], a[2], a[3]);
+              ldsm4t(xa[d] ^ (mt << 5), a[0], a[1], a[2], a[3]);
 #pragma unroll
               for (int n2 = 0; n2 < CN / 16; n2++) {
                 mma_bf16(acc[d][mt][2 * n2], a, bq[n2][0], bq[n2][1]);
                 mma_bf16(acc[d][mt][2 * n2 + 1], a, bq[n2][2], bq[n2][3]);
               }
             }
+            xa[d] += kss * 32 * CM;
           }
         }
       }
+      __syncwarp();
+      if (lane == 0) net_arrive(empty(m - 1));       // block k - 1 has no later reader here
     }
-    cp_wait<0>();
-    __syncthreads();       // the next run's loads reuse the slots
+    if (lane == 0 && !*abort_s) {
+      net_arrive(empty(n + ke - kb));
+      net_arrive(empty(n + ke - kb + 1));
+    }
+    n += ke - kb + 2;
+  }
+  __syncthreads();   // every warp has left the ring (normally, or on an abort)
+  if (*abort_s) {
+    // copies still in flight land before the CTA exits: wait for the last load of every slot
+    if (warp == kWgWarps && lane == 0)
+      for (uint32_t sl = 0; sl < kWgSlots && sl < n; sl++) {
+        const uint32_t last = sl + ((n - 1 - sl) / kWgSlots) * kWgSlots;
+        if (!net_mbar_wait(full(last), (last / kWgSlots) & 1, 1000000000ULL)) atomicExch(&g_net_err, 42);
+      }
+    return;
   }
   // add the rows' (and steps') sums in a fixed order (reuses the ring)
   float *red = reinterpret_cast<float *>(wgsm);                            // [dy][dx][CM][CN]
   const int ny = p.ny, group = ny == 3 ? wr : warp, ngroups = kWgWarps / ny;
   for (int g = 0; g < ngroups; g++) {
-    if (group == g) {
+    if (group == g && warp < kWgWarps) {
       float *rw = red + (ny == 3 ? wy : 0) * 3 * CM * CN;
 #pragma unroll
       for (int d = 0; d < 3; d++)
@@ -2474,11 +2510,26 @@ cudaError_t launch_conv3d(ConvParams p, long long ws_elems, cudaStream_t s) {
 
 template <int CM, int CN, int TX>
 static cudaError_t launch_wgrad_t(const WgradParams &p, dim3 grid, cudaStream_t s) {
-  constexpr size_t sm = wgrad_smem<CM, CN, TX>();
+  typedef WgTile<CM, CN, TX> T;
+  PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
+  if (!enc) return cudaErrorNotSupported;
+  // [B][Z][Y][X][C] BF16, innermost first; one box = the channels of a tile x a segment x a row block
+  auto encode = [&](CUtensorMap *map, const bf16 *a, int C, int ct, int xv) {
+    const cuuint64_t vb = 2ull * C;   // bytes per voxel
+    const cuuint64_t dims[5] = {(cuuint64_t)C, (cuuint64_t)p.X, (cuuint64_t)p.Y, (cuuint64_t)p.Z, (cuuint64_t)p.B};
+    const cuuint64_t strides[4] = {vb, vb * p.X, vb * p.X * p.Y, vb * p.X * p.Y * p.Z};
+    const cuuint32_t box[5] = {(cuuint32_t)ct, (cuuint32_t)xv, (cuuint32_t)kWgRows, 1, 1};
+    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16 *>(a), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, ct == 16 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  };
+  CUtensorMap tx, td;
+  if (!encode(&tx, p.x, p.Ci, CM, T::XV) || !encode(&td, p.dy, p.Co, CN, TX)) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute((const void *)k_conv3d_wgrad<CM, CN, TX>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM);
   if (e != cudaSuccess) return e;
-  FLF_NET_LAUNCH(k_conv3d_wgrad<CM, CN, TX><<<grid, 32 * kWgWarps, sm, s>>>(p));
+  FLF_NET_LAUNCH(k_conv3d_wgrad<CM, CN, TX><<<grid, kWgThreads, T::SMEM, s>>>(tx, td, p));
   return cudaGetLastError();
 }
 
