@@ -186,7 +186,7 @@ struct MergeParams {
   Strided out;              // destination (or x for RL updates)
   Strided aux;              // y (EPI_DIVIDE) or Htf (EPI_RL_PREVEDEL)
   Strided norm;             // EPI_RL_STANDARD normaliser (p may be NULL)
-  Div16 dlx, dn;            // set by the launcher
+  Div16 dlx4, dn;           // set by the launcher
 };
 
 struct ResampleParams {     // bilinear resample of img [H][W] at yq [ny] x xq [nx] -> out [ny][nx]
