@@ -840,7 +840,7 @@ __device__ __forceinline__ void head_rows(float (&o)[RH], const float (&v)[RH + 
     for (int dy = 0; dy < 3; dy++) o[r] += in ? v[r + dy][DZ * 3 + dy] : 0.f;
 }
 
-template <int CI, int CO, int R, int S, bool HEAD, bool SW32, bool X1 = false, bool POOL = false>
+template <int CI, int CO, int R, int S, bool HEAD, bool SW32, bool X1, bool POOL, bool MASK>
 __global__ void __launch_bounds__(tma16_threads(S), 1)
     k_conv3d_tma16(const __grid_constant__ CUtensorMap tx, ConvParams p, HeadOut h, Tma16Grid g) {
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -1045,7 +1045,28 @@ __global__ void __launch_bounds__(tma16_threads(S), 1)
       decode(it, b, zlo, nz, y0, x0);
       const int x = x0 + qd * 32 + lane;
       float pacc[POOL ? CH : 1];   // POOL: the 2x2x2 average of the output, summed over a plane pair
+      // the ReLU mask of an output plane, loaded a plane ahead: in line with the accumulators'
+      // loads its latency was longer than a plane's MMAs (16 -> 16 at 22 x 387 x 128 53 us with
+      // a mask, 25 without)
+      uint4 mk[MASK ? R : 1][MASK ? CH / 8 : 1], mnext[MASK ? R : 1][MASK ? CH / 8 : 1];
+      auto load_mask = [&](int i) {
+#pragma unroll
+        for (int r = 0; r < (MASK ? R : 0); r++)
+#pragma unroll
+          for (int v = 0; v < CH / 8; v++)
+            if (x < p.X && y0 + r < p.Y)
+              mnext[r][v] = *reinterpret_cast<const uint4 *>(
+                  p.mask + ((((long long)b * p.Z + zlo + i) * p.Y + y0 + r) * p.X + x) * CO + hf * CH + v * 8);
+      };
+      if constexpr (MASK) load_mask(0);
       for (int i = 0; i < nz; i++) {
+        if constexpr (MASK) {
+#pragma unroll
+          for (int r = 0; r < R; r++)
+#pragma unroll
+            for (int v = 0; v < CH / 8; v++) mk[r][v] = mnext[r][v];
+          if (i + 1 < nz) load_mask(i + 1);
+        }
         // output plane z = zlo + i reads slabs n+i (dz 0), n+i+1 (dz 1), n+i+2 (dz 2); the issuers'
         // commits complete in any order, so the first plane waits for all three
         bool here = true;
@@ -1122,11 +1143,9 @@ __global__ void __launch_bounds__(tma16_threads(S), 1)
             const long long off = ((((long long)b * p.Z + z) * p.Y + y) * p.X + x) * CO + hf * CH;
 #pragma unroll
             for (int v = 0; v < CH / 8; v++) {
-              uint4 mk;
-              if (p.mask) mk = *reinterpret_cast<const uint4 *>(p.mask + off + v * 8);
               uint4 outv;
               __nv_bfloat162 *hv = reinterpret_cast<__nv_bfloat162 *>(&outv);
-              const __nv_bfloat162 *m2 = reinterpret_cast<const __nv_bfloat162 *>(&mk);
+              const __nv_bfloat162 *m2 = reinterpret_cast<const __nv_bfloat162 *>(&mk[MASK ? r : 0][MASK ? v : 0]);
 #pragma unroll
               for (int k = 0; k < 4; k++) {
                 float v0 = o[v * 8 + 2 * k] + bias[v * 8 + 2 * k];
@@ -1135,7 +1154,7 @@ __global__ void __launch_bounds__(tma16_threads(S), 1)
                   v0 = fmaxf(v0, 0.f);
                   v1 = fmaxf(v1, 0.f);
                 }
-                if (p.mask) {
+                if (MASK) {
                   const float2 mf = __bfloat1622float2(m2[k]);
                   if (!(mf.x > 0.f)) v0 = 0.f;
                   if (!(mf.y > 0.f)) v1 = 0.f;
@@ -1242,7 +1261,7 @@ template <int CM, int CN, int TX> struct WgTile {
   static constexpr int XV = TX + 2;
   static constexpr size_t XB = (size_t)kWgRows * XV * CM * sizeof(bf16), DB = (size_t)kWgRows * TX * CN * sizeof(bf16);
   static constexpr size_t XS = (XB + 1023) / 1024 * 1024, SLOT = XS + DB;   // a slot: x rows | dy rows
-  static constexpr size_t RING = kWgSlots * SLOT, RED = (size_t)9 * CM * CN * sizeof(float);
+  static constexpr size_t RING = kWgSlots * SLOT, RED = (size_t)4 * 9 * CM * CN * sizeof(float);   // 4 x 9 or 12 x 3 taps
   static constexpr size_t BARS = RING > RED ? RING : RED, SMEM = BARS + (2 * kWgSlots + 1) * 8;
   static_assert(BARS % 8 == 0 && SLOT % 1024 == 0, "the swizzle counts from the slot's base");
 };
@@ -1382,34 +1401,32 @@ __global__ void __launch_bounds__(kWgThreads, 1)
       }
     return;
   }
-  // add the rows' (and steps') sums in a fixed order (reuses the ring)
-  float *red = reinterpret_cast<float *>(wgsm);                            // [dy][dx][CM][CN]
-  const int ny = p.ny, group = ny == 3 ? wr : warp, ngroups = kWgWarps / ny;
-  for (int g = 0; g < ngroups; g++) {
-    if (group == g && warp < kWgWarps) {
-      float *rw = red + (ny == 3 ? wy : 0) * 3 * CM * CN;
+  // every row's (and step's) sums side by side (reuses the ring), then added in row order
+  float *red = reinterpret_cast<float *>(wgsm);                            // [group][dy][dx][CM][CN]
+  const int ny = p.ny, group = ny == 3 ? wr : warp, ngroups = kWgWarps / ny, gsz = ny * 3 * CM * CN;
+  if (warp < kWgWarps) {
+    float *rw = red + group * gsz + (ny == 3 ? wy : 0) * 3 * CM * CN + (lane >> 2) * CN + 2 * (lane & 3);
 #pragma unroll
-      for (int d = 0; d < 3; d++)
+    for (int d = 0; d < 3; d++)
 #pragma unroll
-        for (int mt = 0; mt < CM / 16; mt++)
+      for (int mt = 0; mt < CM / 16; mt++)
 #pragma unroll
-          for (int nt = 0; nt < CN / 8; nt++)
+        for (int nt = 0; nt < CN / 8; nt++)
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-              const int ci = mt * 16 + (lane >> 2) + 8 * (e >> 1), co = nt * 8 + 2 * (lane & 3) + (e & 1);
-              float *o = rw + (d * CM + ci) * CN + co;
-              *o = g ? *o + acc[d][mt][nt][e] : acc[d][mt][nt][e];
-            }
-    }
-    __syncthreads();
+          for (int e = 0; e < 2; e++)
+            *reinterpret_cast<float2 *>(rw + (d * CM + mt * 16 + 8 * e) * CN + nt * 8) =
+                make_float2(acc[d][mt][nt][2 * e], acc[d][mt][nt][2 * e + 1]);
   }
+  __syncthreads();
   const long long nw = 27LL * p.Ci * p.Co;
-  for (int i = tid; i < ny * 3 * CM * CN; i += NT) {
+  for (int i = tid; i < gsz; i += NT) {
+    float v = red[i];
+    for (int g = 1; g < ngroups; g++) v += red[g * gsz + i];
     const int t = i / (CM * CN), e = i - t * CM * CN, ci = e / CN, co = e - ci * CN;
     const int tap = dz * 9 + (ny == 3 ? t : (part % 3) * 3 + t);
     const long long o = ((long long)tap * p.Ci + ci0 + ci) * p.Co + co0 + co;
-    if (p.part) p.part[chunk * nw + o] = red[i];
-    else p.dw[o] += red[i];
+    if (p.part) p.part[chunk * nw + o] = v;
+    else p.dw[o] += v;
   }
 }
 
@@ -1852,8 +1869,8 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
-template <int CI, int CO, int R, int S, bool HEAD, bool SW32, bool X1 = false, bool POOL = false>
-static cudaError_t launch_tma16(const ConvParams &p, const HeadOut &h, cudaStream_t s) {
+template <int CI, int CO, int R, int S, bool HEAD, bool SW32, bool X1, bool POOL, bool MASK>
+static cudaError_t launch_tma16_as(const ConvParams &p, const HeadOut &h, cudaStream_t s) {
   constexpr int KS = CI / 16;
   constexpr size_t SLOT = SW32 ? KS * (((R + 2) * 136 * 32 + 1023) / 1024 * 1024)
                                : 2 * (((R + 2) * 130 * 16 + 127) / 128 * 128);
@@ -1862,7 +1879,7 @@ static cudaError_t launch_tma16(const ConvParams &p, const HeadOut &h, cudaStrea
   static_assert(SMEM <= 227 * 1024, "shared memory of one CTA");
   static int sms = 0;
   if (!sms) {
-    cudaError_t e = cudaFuncSetAttribute(k_conv3d_tma16<CI, CO, R, S, HEAD, SW32, X1, POOL>,
+    cudaError_t e = cudaFuncSetAttribute(k_conv3d_tma16<CI, CO, R, S, HEAD, SW32, X1, POOL, MASK>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
     if (e != cudaSuccess) return e;
     int dev = 0, n = 0;
@@ -1907,8 +1924,15 @@ static cudaError_t launch_tma16(const ConvParams &p, const HeadOut &h, cudaStrea
   g.zchunks = (p.Z + g.zc - 1) / g.zc;
   g.items = (long long)p.B * g.zchunks * g.yblocks * g.xsegs;
   const unsigned grid = (unsigned)(g.items < sms ? g.items : sms);
-  FLF_NET_LAUNCH(k_conv3d_tma16<CI, CO, R, S, HEAD, SW32, X1, POOL><<<grid, tma16_threads(S), SMEM, s>>>(map, p, h, g));
+  FLF_NET_LAUNCH(k_conv3d_tma16<CI, CO, R, S, HEAD, SW32, X1, POOL, MASK><<<grid, tma16_threads(S), SMEM, s>>>(map, p, h, g));
   return cudaGetLastError();
+}
+
+template <int CI, int CO, int R, int S, bool HEAD, bool SW32, bool X1 = false, bool POOL = false>
+static cudaError_t launch_tma16(const ConvParams &p, const HeadOut &h, cudaStream_t s) {
+  if constexpr (!HEAD)
+    if (p.mask) return launch_tma16_as<CI, CO, R, S, HEAD, SW32, X1, POOL, true>(p, h, s);
+  return launch_tma16_as<CI, CO, R, S, HEAD, SW32, X1, POOL, false>(p, h, s);
 }
 
 // ---------------------------------------------------------------------------
