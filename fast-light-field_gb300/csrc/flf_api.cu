@@ -899,8 +899,7 @@ size_t mac_shape_bytes(const Layout &L, int stages, int chunk_rows, int split) {
 
 // Frames one multiply-accumulate pass takes: mac_max_frames(), or fewer where
 // the ring, the staged spectra and the operand tables of that many frames do
-// not fit shared memory with the current launch shape (Nnum 19 at 12 rows per
-// stage: 2 frames).
+// not fit shared memory with the current launch shape (Nnum 29: 3 frames).
 int frames_per_pass(const flf_ctx *ctx) {
   for (int tf = mac_max_frames(); tf > 1; tf--) {
     bool fits = true;

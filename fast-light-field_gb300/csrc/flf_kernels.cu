@@ -368,7 +368,9 @@ __device__ __forceinline__ void mac_row(const float4 *row, const int (&off)[PPT]
 // Nnum 23 with two 719 -> 642; back projection, whose outputs need registers,
 // loses 3 to 5 % by the same.)
 template <int TF, int TH, int SD, bool FWD> struct MacOcc {
-  static constexpr int v = SD == 1 ? (TH == 256 ? (TF == 2 && FWD ? 3 : 2) : TF == 2 && FWD ? 2 : 1) : TH == 128 ? (TF <= 2 ? 3 : 2) : (TF == 1 ? 2 : 1);
+  static constexpr int v = SD == 1     ? (TH == 256 ? (TF == 2 && FWD ? 3 : 2) : TF == 2 && FWD ? 2 : 1)
+                           : TH == 128 ? (TF <= 2 ? 3 : 2)
+                                       : (TF == 1 ? 2 : 1);
 };
 
 // One CTA = one frequency quad {(uy, ux), (ux, uy)} and a group of planes.
@@ -389,14 +391,14 @@ template <int TF, int TH, int SD, bool FWD> struct MacOcc {
 // per 1808-byte row (Nnum 15) an SM takes 77 cycles at the measured copy rate,
 // against 32 of FMA issue and 46 of shared memory (PPT = 2: two column warps
 // read the row once and 64 B of operands each; one pair per lane would read the
-// operands four times, four pairs would keep 64 accumulators a lane).  With three
-// and four frames the FMAs bound it (registers allow two CTAs per SM).
+// operands four times, four pairs would keep 64 accumulators a lane).  From two
+// frames on it is FMA issue (two-lane FMAs take two cycles of a scheduler), and
+// about 440 SM cycles a chunk beside its rows.
 // Measured (GB300, Nnum 15, sum of the launches of a projection; complex form
-// first): 1005 x 1005 px, 41 planes, one frame: back 2776 -> 1704 us (3.7 -> 6.0
-// TB/s), forward 3006 -> 1789 us (290 more with the operand tables built between
-// planes from staged spectra); 437 x 608 px, 31 planes, three frames: back
-// 3202 -> 1107 us; 450 x 450 px, 31 planes, four frames a launch: forward
-// 477 -> 202 us, back 462 -> 203 us a launch.
+// first): 1005 x 1005 px, 41 planes, one frame: back 2776 -> 1509 us (3.7 -> 6.8
+// TB/s, the copy rate), forward 3006 -> 1536 us; 437 x 608 px, 31 planes, three
+// frames: back 3202 -> 953 us; 450 x 450 px, 31 planes, four frames a launch:
+// forward 477 -> 185 us, back 462 -> 172 us a launch.
 // The stored rows stream through a ring of shared-memory stages filled by
 // bulk copies (crossing plane boundaries).  Forward projection accumulates the
 // planes of the group (the group sums are added by the inverse transform), and

@@ -105,7 +105,7 @@ int flf_backward(flf_ctx *ctx, const float *img_dev, float *vol_dev, int T, int 
  *    must already exist for this Y x X (call flf_prepare earlier), otherwise
  *    FLF_E_STATE is returned instead of building them.
  *  - The intermediate spectra and channel images live in one fixed device
- *    array of FLF_NOALLOC_SCRATCH_BYTES (16 MiB) inside the library: one
+ *    array of FLF_NOALLOC_SCRATCH_BYTES (16 MiB, and 1.5 MiB for its layout) inside the library: one
  *    frame's channel images and spectra plus the output spectra and channel
  *    images of as many planes as fit.  A GPU holds this array from the first
  *    flf_ctx_create on it until the process exits.  Geometries that need more
@@ -114,7 +114,7 @@ int flf_backward(flf_ctx *ctx, const float *img_dev, float *vol_dev, int T, int 
  *    rejected with FLF_E_ARG; use flf_backward.
  *  - The array is set up when the context is created: flf_ctx_create looks
  *    up its device address with the context's device current, which (under
- *    CUDA's lazy module loading) is also when the 16 MiB is committed on that
+ *    CUDA's lazy module loading) is also when the array is committed on that
  *    GPU.  The call itself does no set-up, but under lazy loading its first
  *    launch of each kernel makes the driver load that kernel's code into
  *    device memory: make one call at set-up time (or run with
