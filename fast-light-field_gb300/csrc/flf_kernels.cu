@@ -1048,13 +1048,24 @@ static cudaError_t launch_mac_tf(const MacParams &p0, cudaStream_t s) {
   const dim3 grid(ctas);
   const int threads = 32 * th.cw * th.shares * (th.sides == 1 ? 2 : 1);
   const int block = threads + (FWD && TF == 1 ? 64 : 0);   // and the helper and copy warps
-  void (*fn)(MacParams);
+  // (only the shapes that mac_threads gives for these frames and this direction are built)
+  void (*fn)(MacParams) = nullptr;
   if (th.sides == 1) {
-    fn = th.ppt == 1 ? k_mac<TF, FWD, 1, 256, 1> : threads <= 256 ? k_mac<TF, FWD, 2, 256, 1> : k_mac<TF, FWD, 2, 384, 1>;
+    if (th.ppt == 1) {
+      if constexpr (TF >= 2) fn = k_mac<TF, FWD, 1, 256, 1>;
+    } else if (threads <= 256) {
+      fn = k_mac<TF, FWD, 2, 256, 1>;
+    } else {
+      if constexpr (TF >= 2 || !FWD) fn = k_mac<TF, FWD, 2, 384, 1>;
+    }
+  } else if (th.ppt == 1) {
+    if constexpr (TF == 1) fn = k_mac<TF, FWD, 1, 128, 2>;
+  } else if (threads <= 128) {
+    if constexpr (TF <= 2) fn = k_mac<TF, FWD, 2, 128, 2>;
   } else {
-    fn = threads <= 128 ? (th.ppt == 2 ? k_mac<TF, FWD, 2, 128, 2> : k_mac<TF, FWD, 1, 128, 2>)
-                        : (th.ppt == 2 ? k_mac<TF, FWD, 2, 256, 2> : k_mac<TF, FWD, 1, 256, 2>);
+    fn = k_mac<TF, FWD, 2, 256, 2>;
   }
+  if (!fn) return cudaErrorInvalidValue;
   cudaError_t e = set_smem((const void *)fn, sm);
   if (e != cudaSuccess) return e;
   fn<<<grid, block, sm, s>>>(p);
