@@ -1945,7 +1945,7 @@ int flf_autotune(flf_ctx *ctx, int T, int Y, int X, int *out4, void *stream) {
         if (2 * split_c[b] * ntp > 256) continue;
         for (int ch : chunk_c) {
           if (mac_shape_bytes(ctx->L, stages_c[a], ch, split_c[b]) > kMacSmemMax ||   // flf_set_tuned takes it
-              mac_smem_bytes(ctx->L, nt, stages_c[a], ch, true) > kMacSmemMax)
+              mac_smem_bytes(ctx->L, nt, stages_c[a], ch, d == FLF_DIR_FORWARD) > kMacSmemMax)   // this direction's launch
             continue;
           e = mac_group_launch(ctx, gi, d, nt, ps, stages_c[a], ch, split_c[b], s);   // warm-up
           if (e == cudaSuccess) e = cudaEventRecord(e0, s);

@@ -787,8 +787,11 @@ size_t rfft2_smem_bytes(int f, int imgs, int fp64) {
   const size_t isz = (size_t)f * (f / 2 + 1);
   return cs * ((size_t)f + 2 * (size_t)imgs * isz);
 }
+// (a refusal is reported here and must not come up again as the next launch's last error)
 static cudaError_t set_smem(const void *fn, size_t bytes) {
-  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
 }
 
 // ----------------------------------------------------------------------------
