@@ -810,6 +810,11 @@ __device__ __forceinline__ bool role_wait(uint32_t bar, uint32_t parity, volatil
     }
   }
 }
+// role_wait of a whole warp that goes on to .sync.aligned instructions: the lanes may differ (one sees
+// the phase complete, another the abort flag or its own time limit), so the warp takes one decision
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int *abort_s, int code) {
+  return __all_sync(0xffffffffu, role_wait(bar, parity, abort_s, code) ? 1 : 0);
+}
 __device__ __forceinline__ void tmem_ld16(uint32_t addr, float *v) {
   uint32_t u[16];
   asm volatile(
@@ -1310,7 +1315,7 @@ __global__ void __launch_bounds__(kWgThreads, 1)
   const int mat = lane >> 3, r8 = lane & 7;
 
   uint32_t n = 0;          // loads so far (producer), number of the run's first load (the others)
-  for (long long it = chunk * p.chunk; it < i1 && !*abort_s;) {
+  for (long long it = chunk * p.chunk; it < i1 && !__any_sync(0xffffffffu, *abort_s);) {
     // a run: consecutive row blocks [kb, ke) of one (b, z, segment)
     const int kb = (int)(it % nblk);
     const int ke = (int)min((long long)nblk, kb + (i1 - it));
@@ -1337,12 +1342,12 @@ __global__ void __launch_bounds__(kWgThreads, 1)
       continue;
     }
     const int k16 = (min(TX, p.X - x0) + 15) >> 4;                         // 16-voxel steps
-    if (!role_wait(full(n), (n / kWgSlots) & 1, abort_s, 41) ||
-        !role_wait(full(n + 1), ((n + 1) / kWgSlots) & 1, abort_s, 41))
+    if (!warp_wait(full(n), (n / kWgSlots) & 1, abort_s, 41) ||
+        !warp_wait(full(n + 1), ((n + 1) / kWgSlots) & 1, abort_s, 41))
       break;
     for (int k = kb; k < ke; k++) {
       const uint32_t m = n + (k - kb + 1);                                 // block k's load
-      if (!role_wait(full(m + 1), ((m + 1) / kWgSlots) & 1, abort_s, 41)) break;
+      if (!warp_wait(full(m + 1), ((m + 1) / kWgSlots) & 1, abort_s, 41)) break;
       if (kWgRows * k + wr < p.Y) {
         const int j = wr + wy - 1;                                         // x row of the tap, relative to the block
         const uint32_t xn = j < 0 ? m - 1 : j >= kWgRows ? m + 1 : m;
