@@ -727,8 +727,9 @@ __global__ void __launch_bounds__(128) k_conv3d_tc16(ConvParams p, int tiles_x, 
 // and out[z][y0+r][x] = sum over (dz, dy) of D[z-1+dz][r+dy][x][dz*3+dy], so a
 // slab of R+2 input rows costs 3 (R+2) MMAs for R output rows instead of 9 R.
 //   warp 0     producer: one thread issues the TMA loads;
-//   MMA issuers (up to four warps, one thread each): take the slabs in turn,
-//              issue all MMAs of a slab, then commit to the slab's accumulator
+//   MMA issuers (up to four warps, one thread each): take the slabs in turn
+//              (the head's two threads share every slab's rows), issue all MMAs
+//              of a slab, then commit to the slab's accumulator
 //              barrier and to its shared-memory slot; before a slab's MMAs a
 //              thread tests its next slab's barriers without blocking, so that
 //              test's latency overlaps the MMAs (a blocking wait follows only
@@ -758,8 +759,14 @@ constexpr int TMA16_NACC = 5;   // TMEM accumulator slots (R x 3 CO columns each
 // told from the one two phases before it by its parity alone, so a thread may only wait for slab n
 // once slab n - S (the slab ring) and n - 2 NACC (the accumulator ring) are known complete: they
 // divide S, so that the same thread handled slab n - S, and there are at most NACC of them.
-__host__ __device__ constexpr int tma16_issuers(int S) { return S % 4 == 0 ? 4 : S % 3 == 0 ? 3 : S % 2 == 0 ? 2 : 1; }
-__host__ __device__ constexpr int tma16_threads(int S) { return 32 * (1 + tma16_issuers(S) + 8); }
+// The 3x3x1 layer (X1), with a third of the MMAs per slab, takes two: 73.4 us at 24 x 456 x 456, 78.1
+// with four.  The head, whose epilogue needs more registers than 13 warps leave, has two that share
+// every slab's rows: 50.3 us, 52.8 with four by slab (which spill; 17.7 against 19.3 at 13 x 203 x 331,
+// but 9.3 against 9.0 at 24 x 128 x 128 and 6.1 against 5.7 at 3 x 24 x 40), 50.4 with two by slab.
+__host__ __device__ constexpr int tma16_issuers(int S, bool HEAD, bool X1) {
+  return HEAD || X1 ? 2 : S % 4 == 0 ? 4 : S % 3 == 0 ? 3 : S % 2 == 0 ? 2 : 1;
+}
+__host__ __device__ constexpr int tma16_threads(int S, bool HEAD, bool X1) { return 32 * (1 + tma16_issuers(S, HEAD, X1) + 8); }
 
 namespace {
 
@@ -846,7 +853,7 @@ __device__ __forceinline__ void head_rows(float (&o)[RH], const float (&v)[RH + 
 }
 
 template <int CI, int CO, int R, int S, bool HEAD, bool SW32, bool X1, bool POOL, bool MASK>
-__global__ void __launch_bounds__(tma16_threads(S), 1)
+__global__ void __launch_bounds__(tma16_threads(S, HEAD, X1), 1)
     k_conv3d_tma16(const __grid_constant__ CUtensorMap tx, ConvParams p, HeadOut h, Tma16Grid g) {
   extern __shared__ __align__(1024) unsigned char smem[];
   constexpr int PYH = R + 2, NACC = TMA16_NACC;
@@ -860,8 +867,10 @@ __global__ void __launch_bounds__(tma16_threads(S), 1)
   static_assert(!(HEAD && X1), "the head is a full 3x3x3 convolution");
   static_assert(!POOL || (CO == 16 && R == 2 && !HEAD && !X1),
                 "the pooled output is for 16 output channels and two rows per item");
-  constexpr int NISS = tma16_issuers(S);      // MMA-issuing threads (warps 1 .. NISS)
+  constexpr int NISS = tma16_issuers(S, HEAD, X1);   // MMA-issuing threads (warps 1 .. NISS)
+  constexpr bool ROWS = HEAD;                 // they share every slab's rows (otherwise each takes whole slabs)
   static_assert(S % NISS == 0 && NISS <= NACC, "see tma16_issuers");
+  static_assert(!ROWS || PYH % NISS == 0, "the issuers take the same number of rows");
   constexpr int CH = CO / 2;                  // output channels per epilogue warp
   static_assert((CI == 16 || CI == 32) && (CO == 16 || CO == 32), "16 or 32 channels in and out");
   static_assert(SW32 || CI == 16, "the unswizzled slab layout is for 16 input channels");
@@ -917,10 +926,10 @@ __global__ void __launch_bounds__(tma16_threads(S), 1)
   if (tid == 0) {
     for (int k = 0; k < S; k++) {
       net_mbar_init(full(k), 1);
-      net_mbar_init(empty(k), 1);
+      net_mbar_init(empty(k), ROWS ? NISS : 1);
     }
     for (int k = 0; k < NACC; k++) {
-      net_mbar_init(tfull(k), 1);
+      net_mbar_init(tfull(k), ROWS ? NISS : 1);
       net_mbar_init(tempty(k), 256);
     }
     net_mbar_init(fin, NISS);
@@ -970,9 +979,10 @@ __global__ void __launch_bounds__(tma16_threads(S), 1)
     }
   } else if (warp <= NISS) {
     if (lane == 0) {
-      // ---- MMA issuers: warp 1 + j takes the slabs n = j, j + NISS, ... (output rows, or for the
-      // head input rows) ----
-      constexpr int RI = HEAD ? PYH : R;
+      // ---- MMA issuers: warp 1 + j takes the slabs n = j, j + NISS, ... (output rows), or of every
+      // slab the rows j RI .. j RI + RI - 1 (input rows of the head) ----
+      constexpr int RI = ROWS ? PYH / NISS : R;
+      const int r0 = ROWS ? (warp - 1) * RI : 0;
       // instruction descriptor: F32 accumulate, BF16 A and B, both K-major, N = 3 CO, M = 128
       const uint32_t idesc =
           (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NN >> 3) << 17) | ((128u >> 4) << 24);
@@ -991,7 +1001,7 @@ __global__ void __launch_bounds__(tma16_threads(S), 1)
         int b, zlo, nz, y0, x0;
         decode(it, b, zlo, nz, y0, x0);
         for (int k = 0; k < nz + 2; k++, n++) {
-          if (n % NISS != (uint32_t)(warp - 1)) continue;
+          if (!ROWS && n % NISS != (uint32_t)(warp - 1)) continue;
           const uint32_t acc = n % NACC;
           ok = (pre_full & pre_empty) ||
                (role_wait(full(n % S), (n / S) & 1, abort_s, 5) &&
@@ -1002,7 +1012,7 @@ __global__ void __launch_bounds__(tma16_threads(S), 1)
             // there, so their latency overlaps this slab's MMAs (a blocking wait follows only if a
             // phase was not yet complete).  A phase seen complete stays complete until this thread's
             // own commits let the slot be refilled.
-            const uint32_t n1 = n + NISS;
+            const uint32_t n1 = n + (ROWS ? 1 : NISS);
             pre_full = mbar_test(full(n1 % S), (n1 / S) & 1);
             pre_empty = n1 < NACC ? 1u : mbar_test(tempty(n1 % NACC), ((n1 / NACC) - 1) & 1);
           }
@@ -1025,8 +1035,8 @@ __global__ void __launch_bounds__(tma16_threads(S), 1)
                 for (int r = 0; r < RI; r++) {
                   const uint64_t ad = ((uint64_t)a_hi << 32) |
                                       (uint64_t)(al + kh * (PLANE >> 4) +
-                                                 (uint32_t)(((r + dy) * PXW + dx) * VOX));
-                  umma_f16(dcol + r * NN, ad, bd, idesc, (blk > 0 || kh > 0) ? 1u : 0u);
+                                                 (uint32_t)(((r0 + r + dy) * PXW + dx) * VOX));
+                  umma_f16(dcol + (r0 + r) * NN, ad, bd, idesc, (blk > 0 || kh > 0) ? 1u : 0u);
                 }
               }
             }
@@ -1072,11 +1082,24 @@ __global__ void __launch_bounds__(tma16_threads(S), 1)
             for (int v = 0; v < CH / 8; v++) mk[r][v] = mnext[r][v];
           if (i + 1 < nz) load_mask(i + 1);
         }
-        // output plane z = zlo + i reads slabs n+i (dz 0), n+i+1 (dz 1), n+i+2 (dz 2); the issuers'
-        // commits complete in any order, so the first plane waits for all three
+        // output plane z = zlo + i reads slabs n+i (dz 0), n+i+1 (dz 1), n+i+2 (dz 2).  Issuers that share
+        // the slabs commit in slab order: the last one's barrier covers the others.  The commits of issuers
+        // that take slabs in turn complete in any order, so the first plane waits for all three (a loop in
+        // the plain layers, 82.5 us at 24 x 456 x 456 against 84.6 unrolled; unrolled with a mask, 16 -> 16
+        // at 22 x 387 x 128 31.5 against 40.1 us, 32 -> 32 at 12 x 228 x 228 42.4 against 53.1, with X1 or
+        // the pooled output 73.5 and 101.8 against 76.3 and 104.0)
+        const uint32_t last = n + i + 2;
         bool here = true;
-        for (uint32_t m = n + i + (i ? 2 : 0); m <= n + i + 2 && here; m++)
-          here = role_wait(tfull(m % NACC), (m / NACC) & 1, abort_s, 7);
+        if constexpr (ROWS || MASK || X1 || POOL) {
+          if (!ROWS && i == 0) {
+            here = role_wait(tfull(n % NACC), (n / NACC) & 1, abort_s, 7);
+            here = here && role_wait(tfull((n + 1) % NACC), ((n + 1) / NACC) & 1, abort_s, 7);
+          }
+          here = here && role_wait(tfull(last % NACC), (last / NACC) & 1, abort_s, 7);
+        } else {
+          for (uint32_t m = i ? last : n; m <= last && here; m++)
+            here = role_wait(tfull(m % NACC), (m / NACC) & 1, abort_s, 7);
+        }
         // tcgen05.ld is .sync.aligned: the whole warp takes one decision
         if (!__all_sync(0xffffffffu, here ? 1 : 0)) {
           ok = false;
@@ -1929,13 +1952,13 @@ static cudaError_t launch_tma16_as(const ConvParams &p, const HeadOut &h, cudaSt
   g.zchunks = (p.Z + g.zc - 1) / g.zc;
   g.items = (long long)p.B * g.zchunks * g.yblocks * g.xsegs;
   const unsigned grid = (unsigned)(g.items < sms ? g.items : sms);
-  FLF_NET_LAUNCH(k_conv3d_tma16<CI, CO, R, S, HEAD, SW32, X1, POOL, MASK><<<grid, tma16_threads(S), SMEM, s>>>(map, p, h, g));
+  FLF_NET_LAUNCH(k_conv3d_tma16<CI, CO, R, S, HEAD, SW32, X1, POOL, MASK><<<grid, tma16_threads(S, HEAD, X1), SMEM, s>>>(map, p, h, g));
   return cudaGetLastError();
 }
 
 template <int CI, int CO, int R, int S, bool HEAD, bool SW32, bool X1 = false, bool POOL = false>
 static cudaError_t launch_tma16(const ConvParams &p, const HeadOut &h, cudaStream_t s) {
-  if constexpr (!HEAD)
+  if constexpr (!HEAD && !X1 && !POOL)   // those take no mask
     if (p.mask) return launch_tma16_as<CI, CO, R, S, HEAD, SW32, X1, POOL, true>(p, h, s);
   return launch_tma16_as<CI, CO, R, S, HEAD, SW32, X1, POOL, false>(p, h, s);
 }

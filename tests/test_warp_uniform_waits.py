@@ -50,8 +50,8 @@ def test_waits_of_whole_warps_take_one_decision():
             continue
         if "__all_sync(0xffffffffu" in stmt:
             continue
-        var = re.match(r"\s*(?:for\s*\(.*\)\s*)?(\w+) = role_wait", stmt, re.S) or re.search(r"(\w+) = role_wait", stmt)
-        assert var and re.search(r"__all_sync\(0xffffffffu, %s\b" % var.group(1), text[pos:pos + 600]), stmt
+        var = re.search(r"(\w+) = (?:\1 && )?role_wait", stmt)
+        assert var and re.search(r"__all_sync\(0xffffffffu, %s\b" % var.group(1), text[pos:pos + 1000]), stmt
 
 
 def test_abort_flag_is_read_by_the_warp_as_one():
