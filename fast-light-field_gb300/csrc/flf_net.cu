@@ -1279,6 +1279,8 @@ __global__ void __launch_bounds__(tma16_threads(S, HEAD, X1), 1)
 // with its halo, one of dy; zeros outside the volume; the 32- or 64-byte swizzle is
 // the one ldmatrix wants), a full and an empty barrier per slot, so a row block costs
 // its reader no index arithmetic and no CTA barrier.
+// EDGE: rows that are not whole steps of 16 voxels, whose last step needs care (below); a choice per
+// step that costs 2 to 5 % (32 -> 32 at 12 x 228 x 228 101.9 -> 107.5 us), so rows of whole steps go without.
 // 16 -> 16 channels at 4 x 24 x 128 x 128: 129 us with 16-byte copies by the readers
 // (tensor pipe 29 % busy; seven of eight instructions staged), 68 us (56 %) now, the
 // copies alone 44; 24 x 456 x 456 with the bias sums 492 -> 265 us, 32 -> 32 at 12 x
@@ -1293,7 +1295,7 @@ template <int CM, int CN, int TX> struct WgTile {
   static constexpr size_t BARS = RING > RED ? RING : RED, SMEM = BARS + (2 * kWgSlots + 1) * 8;
   static_assert(BARS % 8 == 0 && SLOT % 1024 == 0, "the swizzle counts from the slot's base");
 };
-template <int CM, int CN, int TX>
+template <int CM, int CN, int TX, bool EDGE>
 __global__ void __launch_bounds__(kWgThreads, 1)
     k_conv3d_wgrad(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtensorMap td, WgradParams p) {
   typedef WgTile<CM, CN, TX> T;
@@ -1364,7 +1366,11 @@ __global__ void __launch_bounds__(kWgThreads, 1)
       }
       continue;
     }
-    const int k16 = (min(TX, p.X - x0) + 15) >> 4;                         // 16-voxel steps
+    const int nx = min(TX, p.X - x0), k16 = (nx + 15) >> 4;                // voxels of a row, 16-voxel steps
+    // The last step may run past the row, where dy is zero.  The x rows there are zero too but one:
+    // voxel nx of tap dx = -1 is the row's last, which zero does not cancel if it is not finite.  The
+    // lane that would address it (step kd) takes the next voxel, a zero outside the volume.
+    const int kd = (nx & 15) == r8 + 8 * (mat >> 1) ? nx >> 4 : -1;
     if (!warp_wait(full(n), (n / kWgSlots) & 1, abort_s, 41) ||
         !warp_wait(full(n + 1), ((n + 1) / kWgSlots) & 1, abort_s, 41))
       break;
@@ -1399,7 +1405,7 @@ __global__ void __launch_bounds__(kWgThreads, 1)
 #pragma unroll
             for (int mt = 0; mt < CM / 16; mt++) {
               uint32_t a[4];
-              ldsm4t(xa[d] ^ (mt << 5), a[0], a[1], a[2], a[3]);
+              ldsm4t((EDGE && d == 0 && ks == kd ? xa[1] : xa[d]) ^ (mt << 5), a[0], a[1], a[2], a[3]);
 #pragma unroll
               for (int n2 = 0; n2 < CN / 16; n2++) {
                 mma_bf16(acc[d][mt][2 * n2], a, bq[n2][0], bq[n2][1]);
@@ -2560,8 +2566,8 @@ cudaError_t launch_conv3d(ConvParams p, long long ws_elems, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-template <int CM, int CN, int TX>
-static cudaError_t launch_wgrad_t(const WgradParams &p, dim3 grid, cudaStream_t s) {
+template <int CM, int CN, int TX, bool EDGE>
+static cudaError_t launch_wgrad_as(const WgradParams &p, dim3 grid, cudaStream_t s) {
   typedef WgTile<CM, CN, TX> T;
   PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
   if (!enc) return cudaErrorNotSupported;
@@ -2578,11 +2584,16 @@ static cudaError_t launch_wgrad_t(const WgradParams &p, dim3 grid, cudaStream_t 
   };
   CUtensorMap tx, td;
   if (!encode(&tx, p.x, p.Ci, CM, T::XV) || !encode(&td, p.dy, p.Co, CN, TX)) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute((const void *)k_conv3d_wgrad<CM, CN, TX>,
+  cudaError_t e = cudaFuncSetAttribute((const void *)k_conv3d_wgrad<CM, CN, TX, EDGE>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM);
   if (e != cudaSuccess) return e;
-  FLF_NET_LAUNCH(k_conv3d_wgrad<CM, CN, TX><<<grid, kWgThreads, T::SMEM, s>>>(tx, td, p));
+  FLF_NET_LAUNCH(k_conv3d_wgrad<CM, CN, TX, EDGE><<<grid, kWgThreads, T::SMEM, s>>>(tx, td, p));
   return cudaGetLastError();
+}
+
+template <int CM, int CN, int TX>
+static cudaError_t launch_wgrad_t(const WgradParams &p, dim3 grid, cudaStream_t s) {
+  return p.X % 16 ? launch_wgrad_as<CM, CN, TX, true>(p, grid, s) : launch_wgrad_as<CM, CN, TX, false>(p, grid, s);
 }
 
 // One CTA per SM (the ring takes most of the shared memory): as many chunks as
