@@ -31,7 +31,7 @@
 //                     CTA, whose staged rows serve the nine taps of that dz;
 //                     each chunk writes a partial sum and k_wgrad_reduce adds
 //                     them in chunk order (no atomics, so training repeats bit
-//                     for bit).
+//                     for bit).  k_conv3d_wgrad_tap: small volumes.
 //   small kernels     bias gradient, 2x2x2 average pooling and its adjoint,
 //                     nearest 2x2x2 upsampling + skip and its adjoint with the
 //                     ReLU mask, MSE loss gradient, Adam, bead rendering.
@@ -1464,12 +1464,138 @@ __global__ void __launch_bounds__(kWgThreads, 1)
   }
 }
 
+// Weight gradient of a small volume (wgrad_by_tap).  CTA = (voxel chunk, tap) x
+// (ci tile CM, co tile CN); the 4 warps take alternate k16 steps of its voxels
+// (split-K) and are summed in shared memory at the end.  Every tap stages x and dy
+// for itself, but the many short CTAs have no barriers to set up, no ring to fill
+// and small sums to join: k_conv3d_wgrad takes 8 to 13 us however small the volume.
+// Partial sums as there.
+template <int CM, int CN>
+__global__ void __launch_bounds__(128) k_conv3d_wgrad_tap(WgradParams p) {
+  constexpr int BK = 64, NS = 3, RA = CM / 8, RBc = CN / 8;
+  __shared__ __align__(128) bf16 Xs[NS][BK * CM];
+  __shared__ __align__(128) bf16 Ds[NS][BK * CN];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const long long M = (long long)p.B * p.Z * p.Y * p.X;
+  const int tap = blockIdx.x % 27;
+  const long long chunk = blockIdx.x / 27;
+  const int ctiles = p.Co / CN;
+  const int ci0 = (blockIdx.y / ctiles) * CM, co0 = (blockIdx.y % ctiles) * CN;
+  const long long v0 = chunk * p.chunk;
+  const long long v1 = v0 + p.chunk < M ? v0 + p.chunk : M;
+  const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
+  const int KS = (int)((v1 - v0 + BK - 1) / BK);
+
+  auto load = [&](int ks, int st) {
+    for (int i = tid; i < BK * (RA + RBc); i += 128) {
+      const int row = i / (RA + RBc), c = i - row * (RA + RBc);
+      const long long vv = v0 + (long long)ks * BK + row;
+      const bool in = vv < v1;
+      if (c < RA) {
+        bool ok = false;
+        const bf16 *src = p.x;
+        if (in) {
+          const Vox q = decode(vv, p.Z, p.Y, p.X);
+          const int z = q.z + dz, y = q.y + dy, x = q.x + dx;
+          ok = z >= 0 && z < p.Z && y >= 0 && y < p.Y && x >= 0 && x < p.X;
+          if (ok) src = p.x + ((((long long)q.b * p.Z + z) * p.Y + y) * p.X + x) * p.Ci + ci0 + c * 8;
+        }
+        cp16(su32(&Xs[st][row * CM]) + ((c ^ swz<RA>(row)) << 4), src, ok);
+      } else {
+        const int cc = c - RA;
+        const bf16 *src = in ? p.dy + vv * p.Co + co0 + cc * 8 : p.dy;
+        cp16(su32(&Ds[st][row * CN]) + ((cc ^ swz<RBc>(row)) << 4), src, in);
+      }
+    }
+  };
+
+  float acc[CM / 16][CN / 8][4];
+#pragma unroll
+  for (int i = 0; i < CM / 16; i++)
+#pragma unroll
+    for (int j = 0; j < CN / 8; j++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) acc[i][j][e] = 0.f;
+
+#pragma unroll
+  for (int s = 0; s < NS - 1; s++) {
+    if (s < KS) load(s, s);
+    cp_commit();
+  }
+  const int mat = lane >> 3, r8 = lane & 7;
+  for (int ks = 0; ks < KS; ks++) {
+    cp_wait<NS - 2>();
+    __syncthreads();
+    const int st = ks % NS;
+    const int kr = warp * 16;   // this warp's 16 voxels of the stage
+    uint32_t a[CM / 16][4];
+#pragma unroll
+    for (int mt = 0; mt < CM / 16; mt++) {
+      // A[ci][k] from Xs[k][ci]: transposed 8x8 blocks (k rows, ci chunk)
+      const int row = kr + r8 + 8 * (mat >> 1);
+      const int c = mt * 2 + (mat & 1);
+      ldsm4t(su32(&Xs[st][row * CM]) + ((c ^ swz<RA>(row)) << 4), a[mt][0], a[mt][1], a[mt][2], a[mt][3]);
+    }
+#pragma unroll
+    for (int n2 = 0; n2 < CN / 16; n2++) {
+      const int row = kr + r8 + 8 * (mat & 1);
+      const int c = n2 * 2 + (mat >> 1);
+      uint32_t b0, b1, b2, b3;
+      ldsm4t(su32(&Ds[st][row * CN]) + ((c ^ swz<RBc>(row)) << 4), b0, b1, b2, b3);
+#pragma unroll
+      for (int mt = 0; mt < CM / 16; mt++) {
+        mma_bf16(acc[mt][2 * n2], a[mt], b0, b1);
+        mma_bf16(acc[mt][2 * n2 + 1], a[mt], b2, b3);
+      }
+    }
+    const int nk = ks + NS - 1;
+    if (nk < KS) load(nk, nk % NS);
+    cp_commit();
+  }
+  cp_wait<0>();
+  __syncthreads();
+  // sum the 4 warps' partial tiles in shared memory (reuses the ring)
+  float *red = reinterpret_cast<float *>(&Xs[0][0]);
+  static_assert(sizeof(Xs) >= sizeof(float) * CM * CN, "reduction buffer");
+  for (int i = tid; i < CM * CN; i += 128) red[i] = 0.f;
+  __syncthreads();
+  for (int w = 0; w < 4; w++) {
+    if (warp == w) {
+#pragma unroll
+      for (int mt = 0; mt < CM / 16; mt++)
+#pragma unroll
+        for (int nt = 0; nt < CN / 8; nt++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            const int ci = mt * 16 + (lane >> 2) + 8 * (e >> 1);
+            const int co = nt * 8 + 2 * (lane & 3) + (e & 1);
+            red[ci * CN + co] += acc[mt][nt][e];
+          }
+    }
+    __syncthreads();
+  }
+  const long long nw = 27LL * p.Ci * p.Co;
+  for (int i = tid; i < CM * CN; i += 128) {
+    const int ci = i / CN, co = i - ci * CN;
+    const long long o = ((long long)tap * p.Ci + ci0 + ci) * p.Co + co0 + co;
+    if (p.part) p.part[chunk * nw + o] = red[i];
+    else p.dw[o] += red[i];
+  }
+}
+
 // dw[i] += sum over the chunks of part[chunk][i], in chunk order.
+// MANY: eight loads at a time, for the some 50 chunks of k_conv3d_wgrad; for the few of
+// k_conv3d_wgrad_tap that takes up to 1 us of 8 longer.
+template <bool MANY>
 __global__ void k_wgrad_reduce(const float *part, float *dw, long long n, int chunks) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     float s = 0.f;
+    if constexpr (MANY) {
 #pragma unroll 8
-    for (int c = 0; c < chunks; c++) s += part[(long long)c * n + i];
+      for (int c = 0; c < chunks; c++) s += part[(long long)c * n + i];
+    } else {
+      for (int c = 0; c < chunks; c++) s += part[(long long)c * n + i];
+    }
     dw[i] += s;
   }
 }
@@ -2596,6 +2722,51 @@ static cudaError_t launch_wgrad_t(const WgradParams &p, dim3 grid, cudaStream_t 
   return p.X % 16 ? launch_wgrad_as<CM, CN, TX, true>(p, grid, s) : launch_wgrad_as<CM, CN, TX, false>(p, grid, s);
 }
 
+// k_conv3d_wgrad_tap: chunks of whole 64-voxel stages, about four CTAs per SM.
+static cudaError_t launch_wgrad_tap(WgradParams p, int CM, int CN, long long slices, cudaStream_t s, int num_sms) {
+  const long long M = (long long)p.B * p.Z * p.Y * p.X, nw = 27LL * p.Ci * p.Co;
+  const int tiles = (p.Ci / CM) * (p.Co / CN);
+  long long chunks = std::max(1LL, std::min((4LL * num_sms + 27 * tiles - 1) / (27 * tiles), slices));
+  p.chunk = ((M + chunks - 1) / chunks + 63) / 64 * 64;
+  chunks = (M + p.chunk - 1) / p.chunk;
+  if (chunks == 1) p.part = nullptr;
+  const dim3 grid((unsigned)(chunks * 27), (unsigned)tiles);
+  void (*fn)(WgradParams) = CM == 16 ? (CN == 16   ? k_conv3d_wgrad_tap<16, 16>
+                                        : CN == 32 ? k_conv3d_wgrad_tap<16, 32>
+                                                   : k_conv3d_wgrad_tap<16, 64>)
+                                     : (CN == 16   ? k_conv3d_wgrad_tap<32, 16>
+                                        : CN == 32 ? k_conv3d_wgrad_tap<32, 32>
+                                                   : k_conv3d_wgrad_tap<32, 64>);
+  FLF_NET_LAUNCH(fn<<<grid, 128, 0, s>>>(p));
+  if (p.part) FLF_NET_LAUNCH(k_wgrad_reduce<false><<<grid_for(nw, 256), 256, 0, s>>>(p.part, p.dw, nw, (int)chunks));
+  return cudaGetLastError();
+}
+
+// Whether the weight gradient of M voxels goes tap by tap: where that is faster.
+// With a workspace of enough slices (us tap by tap and k_conv3d_wgrad, both with the
+// reduction): 16 -> 16 at M = 108 4.6, 8.2; 1152 6.6, 7.9; 3200 9.1, 12.2; 4096 10.0, 8.9;
+// 16 -> 32 at 768 6.9, 9.4; 2304 10.2, 10.7; 2700 10.6, 9.5; 32 -> 32 at 108 6.9, 13.4; 2304
+// 12.9, 14.3; 2700 13.2, 13.3; 4096 16.0, 14.0; 64 -> 32 at 1440 13.1, 13.4; 2304 16.5, 14.9.
+// 64-wide tiles: as long as one wave of one-stage CTAs takes them, and few slices to add:
+// 32 -> 64 at 768 12.2, 13.6; 1152 14.5, 13.5; 64 -> 64 at 540 13.8, 14.3; 720 17.8, 14.5;
+// 64 -> 128 at 288 14.0, 14.6; 540 18.0, 14.7; 128 -> 128 at 108 13.2, 16.2; 168 19.9, 16.0.
+// Without a workspace a tap's CTA walks all voxels, and k_conv3d_wgrad's one chunk all row
+// blocks of all (b, z, segment), which cost it about half a microsecond each: 16 -> 16 at
+// 12 x 8 x 8 15.6, 24.0, at 3 x 16 x 16 15.6, 12.2; 32 -> 64 at 3 x 6 x 6 12.2, 13.9, at 3 x 7 x 8 15.1, 13.9.
+static bool wgrad_by_tap(const WgradParams &p, int CM, int CN, long long items, long long runs, long long slices,
+                         int num_sms) {
+  const long long M = (long long)p.B * p.Z * p.Y * p.X, stages = (M + 63) / 64;
+  const long long tiles = (long long)(p.Ci / CM) * (p.Co / CN), size = CM * CN;
+  if (slices >= std::min(stages, (4LL * num_sms + 27 * tiles - 1) / (27 * tiles))) {
+    if (CN == 64) return stages <= 16 && 27 * stages * tiles <= 4LL * num_sms;
+    return M * tiles <= (size == 256 ? 3600 : size == 512 ? 2500 : 3000);
+  }
+  return size == 256   ? M < 100 + 31 * (items + runs)
+         : CN == 64    ? M < 30 + 12 * (items + runs)
+         : size == 512 ? M < 63 + 21 * (items + runs)
+                       : M < 120 + 18 * (items + runs);
+}
+
 // One CTA per SM (the ring takes most of the shared memory): as many chunks as
 // fill them, within the workspace's slices.
 cudaError_t launch_conv3d_wgrad(WgradParams p, long long ws_elems, cudaStream_t s, int num_sms) {
@@ -2604,12 +2775,12 @@ cudaError_t launch_conv3d_wgrad(WgradParams p, long long ws_elems, cudaStream_t 
   const int CM = p.Ci % 32 == 0 ? 32 : 16, CN = p.Co % 32 == 0 ? 32 : 16, TX = CM + CN == 32 ? 128 : 64;
   const int tiles = (p.Ci / CM) * (p.Co / CN);
   const long long nw = 27LL * p.Ci * p.Co;
-  const long long items = (long long)p.B * p.Z * ((p.X + TX - 1) / TX) * ((p.Y + kWgRows - 1) / kWgRows);
-  long long chunks = num_sms / (3LL * tiles);
-  if (chunks > items) chunks = items;
-  if (!p.part) chunks = 1;                                         // no workspace: one writer per element
-  else if (chunks > ws_elems / nw) chunks = ws_elems / nw;         // partial tiles must fit the workspace
-  if (chunks < 1) chunks = 1;
+  const long long runs = (long long)p.B * p.Z * ((p.X + TX - 1) / TX), items = runs * ((p.Y + kWgRows - 1) / kWgRows);
+  const long long slices = p.part ? ws_elems / nw : 1;             // no workspace: one writer per element
+  const int CNT = p.Co % 64 == 0 ? 64 : CN;
+  if (wgrad_by_tap(p, CM, CNT, items, runs, slices, num_sms)) return launch_wgrad_tap(p, CM, CNT, slices, s, num_sms);
+  long long chunks = std::min(num_sms / (3LL * tiles), items);
+  chunks = std::max(1LL, std::min(chunks, slices));                // partial tiles must fit the workspace
   p.chunk = (items + chunks - 1) / chunks;
   chunks = (items + p.chunk - 1) / p.chunk;
   if (chunks == 1) p.part = nullptr;
@@ -2618,7 +2789,7 @@ cudaError_t launch_conv3d_wgrad(WgradParams p, long long ws_elems, cudaStream_t 
   cudaError_t e = CM == 32 ? (CN == 32 ? launch_wgrad_t<32, 32, 64>(p, grid, s) : launch_wgrad_t<32, 16, 64>(p, grid, s))
                            : (CN == 32 ? launch_wgrad_t<16, 32, 64>(p, grid, s) : launch_wgrad_t<16, 16, 128>(p, grid, s));
   if (e != cudaSuccess) return e;
-  if (p.part) FLF_NET_LAUNCH(k_wgrad_reduce<<<grid_for(nw, 256), 256, 0, s>>>(p.part, p.dw, nw, (int)chunks));
+  if (p.part) FLF_NET_LAUNCH(k_wgrad_reduce<true><<<grid_for(nw, 256), 256, 0, s>>>(p.part, p.dw, nw, (int)chunks));
   return cudaGetLastError();
 }
 

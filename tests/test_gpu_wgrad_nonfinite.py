@@ -11,14 +11,15 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("X", [1, 15, 16, 17, 31, 63, 64, 65, 72, 127, 129, 260])
+@pytest.mark.parametrize("planes", [(1, 3, 6), (2, 12, 13)])     # small volumes go tap by tap
 @pytest.mark.parametrize("Ci,Co", [(16, 16), (16, 32), (32, 16), (32, 32), (64, 64)])
 @pytest.mark.parametrize("slices", [0, 64])
-def test_nonfinite_activation_stays_in_its_taps(built_lib, X, Ci, Co, slices):
+def test_nonfinite_activation_stays_in_its_taps(built_lib, planes, X, Ci, Co, slices):
     import torch
     import _flf
     _flf.load_library()
     g = torch.Generator().manual_seed(X)
-    shape = (1, 3, 6, X)
+    shape = planes + (X,)
     x = torch.randn(shape + (Ci,), generator=g).bfloat16()
     dy = torch.randn(shape + (Co,), generator=g).bfloat16()
     x[0, 1, 2, X - 1, 3] = float("inf")
