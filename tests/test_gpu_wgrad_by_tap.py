@@ -46,3 +46,19 @@ def test_either_side_of_the_rule(built_lib, shape, Ci, Co, slices):
 @pytest.mark.parametrize("slices", [0, 1, 3, 64])
 def test_row_blocks_at_their_edges(built_lib, X, Ci, Co, slices):
     check((2, 5, 13, X), Ci, Co, slices)
+
+
+@pytest.mark.parametrize("C", [8, 16, 24, 64, 128])
+@pytest.mark.parametrize("M", [1, 7, 63, 64, 65, 128])
+def test_bias_gradient_of_few_rows(built_lib, C, M):
+    """Up to 64 rows one channel per thread, then 16-byte loads."""
+    import torch
+    import _flf
+    lib = _flf.load_library()
+    g = torch.randn((M, C), generator=torch.Generator().manual_seed(C + M)).bfloat16()
+    db = torch.ones(C, device="cuda")
+    ws = torch.full((256,), float("nan"), device="cuda")
+    d = g.cuda()
+    assert lib.flf_bias_grad(d.data_ptr(), db.data_ptr(), M, C, ws.data_ptr(), ws.numel(), None) == 0
+    want = g.double().sum(0)
+    assert float((db.cpu().double() - 1 - want).abs().max()) <= 1e-5 * float(g.double().abs().sum(0).max() + 1)
