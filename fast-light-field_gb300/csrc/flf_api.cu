@@ -52,6 +52,7 @@ struct Geometry {
                                  // (stages, chunk rows forward, backward, split); 0: context options
   std::vector<Group> groups;
   std::vector<int> plane_group, plane_slot;
+  bool one_by_one = false;    // never merge the groups' launches: their workspaces did not fit (ensure_workspaces)
   int *d_lists = nullptr;     // plane ids of all groups, one after the other, then their slots
   bool built(int dir) const {
     for (const Group &g : groups)
@@ -98,6 +99,7 @@ struct flf_ctx {
   int opt_streams = 2;           // transform groups alternate over this many streams (1 or 2)
   int opt_release_psf = 0;       // free the PSF quadrants after the precompute of both directions
   long long opt_wait_us = 1000000;   // limit of the multiply-accumulate's waits for a ring slot
+  size_t opt_ws_limit = 0;       // test of refused allocations: bytes a projection's workspaces may take (0: no limit)
   int opt_drop_chunk = -1;       // test of the bounded waits: a chunk the first CTA never issues
   bool psf_released = false;
   cudaStream_t s2 = nullptr;     // the second stream, and the events that fork / chain / join it
@@ -732,9 +734,9 @@ void ws_needs(const flf_ctx *ctx, const PlaneSet &ps, int nt, bool fwd, size_t &
 // 21 planes in 5 groups 347 and 303 us, 31 planes 478 and 429; 675 px, 31 planes in 7
 // groups 898 and 799; 1005 px, 41 planes in 6 groups 2081 and 1998 (back 1964 and
 // 1961); 450 px, 11 planes in 3 groups 167 and 163; 5 planes in 2 groups 83 and 89.
-bool merge_groups(const PlaneSet &ps, int nt) {
+bool merge_groups(const flf_ctx *ctx, const PlaneSet &ps, int nt) {
   const int k = ps.groups();
-  return nt == 1 && k >= 3 && k <= kMacMaxGroups;
+  return nt == 1 && k >= 3 && k <= kMacMaxGroups && !ctx->geo.one_by_one;
 }
 
 // Planes per CTA of such a launch (of one frame): about 16 CTAs per SM in all.
@@ -760,7 +762,7 @@ WsSizes ws_sizes(const flf_ctx *ctx, const PlaneSet &ps, int nt, bool fwd) {
   WsSizes w;
   const size_t cset = sizeof(float) * chan_set_floats(ctx), NN = ctx->L.NN;
   w.Cimg = cset * nt;
-  if (!merge_groups(ps, nt)) {
+  if (!merge_groups(ctx, ps, nt)) {
     size_t a, b, c;
     ws_needs(ctx, ps, nt, fwd, a, b, c);
     w.S = ws_slots(ctx) * slot_bytes(a); w.O = ws_slots(ctx) * slot_bytes(b); w.Cvol = ws_slots(ctx) * slot_bytes(c);
@@ -779,19 +781,35 @@ WsSizes ws_sizes(const flf_ctx *ctx, const PlaneSet &ps, int nt, bool fwd) {
   return w;
 }
 
-// The workspaces of a run of T frames in passes of TF.
+// The workspaces of a run of T frames in passes of TF.  A merged launch holds the
+// spectra and images of all groups at once, where two of the largest group do
+// otherwise: if they do not fit, this geometry's groups go one by one from then on.
 int ensure_workspaces(flf_ctx *ctx, const PlaneSet &ps, int T, int TF, bool fwd, bool bwd) {
-  WsSizes w;
-  for (int nt : {std::min(T, TF), T % TF}) {
-    if (!nt) continue;
-    if (fwd) w.grow(ws_sizes(ctx, ps, nt, true));
-    if (bwd) w.grow(ws_sizes(ctx, ps, nt, false));
+  for (bool retried = false;; retried = true) {
+    WsSizes w;
+    bool merged = false;
+    for (int nt : {std::min(T, TF), T % TF}) {
+      if (!nt) continue;
+      merged = merged || merge_groups(ctx, ps, nt);
+      if (fwd) w.grow(ws_sizes(ctx, ps, nt, true));
+      if (bwd) w.grow(ws_sizes(ctx, ps, nt, false));
+    }
+    int rc = FLF_OK;
+    if (ctx->opt_ws_limit && w.S + w.O + w.Cvol + w.Cimg > ctx->opt_ws_limit)
+      rc = fail(ctx, FLF_E_NOMEM, "workspaces exceed test_workspace_limit");
+    if (rc == FLF_OK) rc = ensure_ws(ctx, ctx->wsS, w.S);
+    if (rc == FLF_OK) rc = ensure_ws(ctx, ctx->wsO, w.O);
+    if (rc == FLF_OK) rc = ensure_ws(ctx, ctx->wsCvol, w.Cvol);
+    if (rc == FLF_OK) rc = ensure_ws(ctx, ctx->wsCimg, w.Cimg);
+    if (rc != FLF_OK && retried) ctx->geo.one_by_one = false;   // that did not help
+    if (rc != FLF_E_NOMEM || !merged) return rc;
+    ctx->geo.one_by_one = true;
+    for (Workspace *o : {&ctx->wsS, &ctx->wsO, &ctx->wsCvol, &ctx->wsCimg}) {
+      if (o->p) cudaFree(o->p);
+      *o = Workspace();
+    }
+    ctx->mem_epoch++;
   }
-  int rc = ensure_ws(ctx, ctx->wsS, w.S);
-  if (rc == FLF_OK) rc = ensure_ws(ctx, ctx->wsO, w.O);
-  if (rc == FLF_OK) rc = ensure_ws(ctx, ctx->wsCvol, w.Cvol);
-  if (rc == FLF_OK) rc = ensure_ws(ctx, ctx->wsCimg, w.Cimg);
-  return rc;
 }
 
 // Workspace slots: one per stream the transform groups alternate over.
@@ -1059,7 +1077,7 @@ int forward_merged(flf_ctx *ctx, const float *vol, long long vol_sz, const Plane
 // image and, with `num`, stores num / (H x) (the standard RL error image).
 int forward_chunk(flf_ctx *ctx, const float *vol, long long vol_sz, const PlaneSet &ps, int t0, int nt,
                   float *chan, const float *num, ChanImg &out, cudaStream_t s) {
-  if (merge_groups(ps, nt)) return forward_merged(ctx, vol, vol_sz, ps, t0, chan, num, out, s);
+  if (merge_groups(ctx, ps, nt)) return forward_merged(ctx, vol, vol_sz, ps, t0, chan, num, out, s);
   out = ChanImg();
   out.p = chan;
   Geometry &Gm = ctx->geo;
@@ -1179,7 +1197,7 @@ int backward_merged(flf_ctx *ctx, const ChanImg &img, const PlaneSet &ps, Stride
 // (aux / norm address volumes).
 int backward_chunk(flf_ctx *ctx, const ChanImg &img, const PlaneSet &ps, int nt, Strided out, Strided aux,
                    Strided norm, int epi, cudaStream_t s) {
-  if (merge_groups(ps, nt)) return backward_merged(ctx, img, ps, out, aux, norm, epi, s);
+  if (merge_groups(ctx, ps, nt)) return backward_merged(ctx, img, ps, out, aux, norm, epi, s);
   const float *chan = img.p;
   Geometry &Gm = ctx->geo;
   const Layout &L = ctx->L;
@@ -1843,6 +1861,11 @@ int flf_set_option(flf_ctx *ctx, const char *name, long long value) {
   if (!strcmp(name, "test_drop_chunk")) {
     if (value < -1 || value > 1000000) return fail(ctx, FLF_E_ARG, "test_drop_chunk must be -1 or a chunk index");
     ctx->opt_drop_chunk = (int)value;
+    return FLF_OK;
+  }
+  if (!strcmp(name, "test_workspace_limit")) {
+    if (value < 0) return fail(ctx, FLF_E_ARG, "test_workspace_limit must be 0 (none) or a number of bytes");
+    ctx->opt_ws_limit = (size_t)value;
     return FLF_OK;
   }
   if (!strcmp(name, "release_psf")) {

@@ -190,6 +190,11 @@ int flf_profile_read(flf_ctx *ctx, char *buf, size_t len);
  * the current image shape are built, for PSF sets whose quadrants and
  * matrices do not both fit; another image shape then needs the PSFs uploaded
  * again).  Results agree to rounding whatever the values.
+ * "test_workspace_limit" (0: none - the default; else bytes) makes projections
+ * whose workspaces need more than that fail as on an out-of-memory cudaMalloc.  A
+ * single frame of three or more transform groups holds the workspaces of
+ * all groups at once; where they do not fit, the groups of that image shape go one
+ * by one, until flf_clear_cache.
  * Two options exist to test the bounded waits of the multiply-accumulate:
  * "mac_wait_limit_us" (100..1e7, default 1e6: how long a wait for a ring
  * slot may last before the kernel gives up, sets the error flag that the next
