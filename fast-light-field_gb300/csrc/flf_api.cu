@@ -1875,7 +1875,7 @@ int flf_set_option(flf_ctx *ctx, const char *name, long long value) {
     return FLF_OK;
   }
   if (!strcmp(name, "mac_ctas_per_sm")) {
-    if (value < 1 || value > 64) return fail(ctx, FLF_E_ARG, "mac_ctas_per_sm must be in [1, 64]");
+    if (value < 0 || value > 64) return fail(ctx, FLF_E_ARG, "mac_ctas_per_sm must be in [1, 64], or 0 (by rule)");
     ctx->opt_ctas_per_sm = (int)value;
     return FLF_OK;
   }
@@ -1900,12 +1900,15 @@ int flf_set_option(flf_ctx *ctx, const char *name, long long value) {
   if (!strcmp(name, "mac_stages") || cr_all || cr_fwd || cr_bwd || !strcmp(name, "mac_split")) {
     const int st = !strcmp(name, "mac_stages") ? (int)value : ctx->opt_stages;
     // (rows chosen per launch fit every ring; shapes are accepted as with 12 rows)
-    const int crf = (cr_all || cr_fwd) ? (int)value : ctx->opt_chunk_rows[FLF_DIR_FORWARD] ? ctx->opt_chunk_rows[FLF_DIR_FORWARD] : 12;
-    const int crb = (cr_all || cr_bwd) ? (int)value : ctx->opt_chunk_rows[FLF_DIR_BACKWARD] ? ctx->opt_chunk_rows[FLF_DIR_BACKWARD] : 12;
+    auto rows = [&](bool asked, int dir) {
+      const long long cr = asked ? value : ctx->opt_chunk_rows[dir];
+      return cr ? (int)cr : 12;
+    };
+    const int crf = rows(cr_all || cr_fwd, FLF_DIR_FORWARD), crb = rows(cr_all || cr_bwd, FLF_DIR_BACKWARD);
     const int sp = !strcmp(name, "mac_split") ? (int)value : ctx->opt_split;
     if (st < 2 || st > 16) return fail(ctx, FLF_E_ARG, "mac_stages must be in [2, 16]");
     for (int cr : {crf, crb})
-      if (cr < 2 || cr > 64 || (cr & 1)) return fail(ctx, FLF_E_ARG, "mac_chunk_rows must be even, in [2, 64]");
+      if (cr < 2 || cr > 64 || (cr & 1)) return fail(ctx, FLF_E_ARG, "mac_chunk_rows must be even, in [2, 64], or 0 (by rule)");
     const int ntp = (ctx->L.nthr + 31) / 32 * 32;
     if (sp < 1 || sp > 4 || 2 * sp * ntp > 256)
       return fail(ctx, FLF_E_ARG, "mac_split must be in [1, 4] with at most 256 threads per block "
@@ -1914,8 +1917,8 @@ int flf_set_option(flf_ctx *ctx, const char *name, long long value) {
       if (mac_shape_bytes(ctx->L, st, cr, sp) > kMacSmemMax)
         return fail(ctx, FLF_E_ARG, "pipeline of %d stages x %d rows exceeds shared memory", st, cr);
     ctx->opt_stages = st;
-    if (cr_all || cr_fwd) ctx->opt_chunk_rows[FLF_DIR_FORWARD] = crf;
-    if (cr_all || cr_bwd) ctx->opt_chunk_rows[FLF_DIR_BACKWARD] = crb;
+    if (cr_all || cr_fwd) ctx->opt_chunk_rows[FLF_DIR_FORWARD] = (int)value;
+    if (cr_all || cr_bwd) ctx->opt_chunk_rows[FLF_DIR_BACKWARD] = (int)value;
     ctx->opt_split = sp;
     return FLF_OK;
   }
@@ -2007,6 +2010,10 @@ int flf_set_tuned(flf_ctx *ctx, int Y, int X, const int *in4) {
   Geometry &Gm = ctx->geo;
   if (!Gm.valid || Gm.Y != Y || Gm.X != X)
     return fail(ctx, FLF_E_STATE, "no prepared geometry for %d x %d: call flf_prepare first", Y, X);
+  if (!in4[0] && !in4[1] && !in4[2] && !in4[3]) {   // back to the context's options
+    for (int i = 0; i < 4; i++) Gm.tuned[i] = 0;
+    return FLF_OK;
+  }
   const int ntp = (ctx->L.nthr + 31) / 32 * 32;
   if (in4[0] < 2 || in4[0] > 16 || in4[3] < 1 || in4[3] > 4 || in4[3] * ntp > 256)
     return fail(ctx, FLF_E_ARG, "invalid launch shape");

@@ -174,18 +174,23 @@ int flf_profile_read(flf_ctx *ctx, char *buf, size_t len);
  * projector.py:26-36).  Options: "mac_stages" (shared-memory pipeline
  * stages of the multiply-accumulate, 2..16), "mac_chunk_rows" (stored rows
  * per stage, even, 2..64, both directions; "mac_chunk_rows_forward" and
- * "mac_chunk_rows_backward" set one), "mac_split" (threads sharing an orbit's rows,
- * 1..4; the CTA has two such groups, one per frequency pair of a quad, of at
- * most 256 threads in all), "mac_ctas_per_sm" (1..64, default 16: the CTAs
- * per SM the grouping of planes per CTA aims at; fewer CTAs stream more planes
- * each), "plane_transform_sizes" (1: each plane uses the smallest
+ * "mac_chunk_rows_backward" set one; 0, the default: by a rule on Nnum, frames
+ * and stages), "mac_split" (1..4, default 1: row shares of a CTA in units of about
+ * 128 threads, at most 256 threads in all; without effect where each frequency pair
+ * of a quad has two or more warps of its own: three frames at Nnum 13 and 15, two
+ * frames or back projection from Nnum 17 on),
+ * "mac_ctas_per_sm" (1..64: the CTAs per SM the grouping of planes per CTA aims
+ * at; fewer CTAs stream more planes each; 0, the default: 16, and 8 in back
+ * projections of two frames and more), "plane_transform_sizes" (1: each plane uses the smallest
  * transform its PSF allows, planes grouped by size - the default; 0: one
  * size for all planes) and "geometry_cache" (0..16, default 2: how many
  * transfer-matrix sets of other image shapes stay resident, most recent
  * first, so that a series alternating image sizes does not rebuild them) and
  * "streams" (1 or 2, default 2: the transform groups of a projection
  * alternate over this many streams, so one group's transforms overlap the
- * next group's multiply-accumulate) and "release_psf" (0 or 1, default 0:
+ * next group's multiply-accumulate; a single frame of three to eight groups, which
+ * share one multiply-accumulate launch, has their transforms on four streams
+ * unless this is 1) and "release_psf" (0 or 1, default 0:
  * free the uploaded PSF quadrants once both directions' transfer matrices of
  * the current image shape are built, for PSF sets whose quadrants and
  * matrices do not both fit; another image shape then needs the PSFs uploaded
@@ -406,7 +411,8 @@ int flf_graph_destroy(flf_graph *graph);
 int flf_autotune(flf_ctx *ctx, int T, int Y, int X, int *out4, void *stream);
 
 /* Apply a launch shape found earlier by flf_autotune (for example read back
- * from a cache file) to the prepared geometry of Y x X images. */
+ * from a cache file) to the prepared geometry of Y x X images; four zeros drop
+ * the one that was applied, so that the options count again. */
 int flf_set_tuned(flf_ctx *ctx, int Y, int X, const int *in4);
 
 /* Rectification resample (replaces the interpolation of the reference's
