@@ -953,18 +953,6 @@ void mac_add_group(MacParams &mp, const Group &G, int dir, const int *planes, in
   g.S = (const float2 *)S; g.O = (float4 *)O;
 }
 
-// One multiply-accumulate launch of group gi over all its planes for nt
-// frames, on the workspaces (flf_autotune's timing unit).
-cudaError_t mac_group_launch(flf_ctx *ctx, size_t gi, int dir, int nt, const PlaneSet &ps, int stages, int chunk,
-                             int split, cudaStream_t s) {
-  const Group &G = ctx->geo.groups[gi];
-  MacParams mp = mac_params(ctx, dir, nt);
-  mp.stages = stages; mp.chunk_rows = chunk; mp.split = split;
-  mac_add_group(mp, G, dir, ps.slots[gi], ps.n[gi], zgroup_for(ctx, ps.n[gi], G.nquads, ctas_per_sm(ctx, dir, nt)),
-                ctx->wsS.p, ctx->wsO.p);
-  return launch_mac(mp, dir == FLF_DIR_FORWARD, s);
-}
-
 SplitParams split_params(const flf_ctx *ctx, const float *src, long long src_sz, long long src_st,
                          const int *planes, int nz, int nt, float *dst) {
   const Geometry &Gm = ctx->geo;
@@ -1908,7 +1896,7 @@ int flf_set_option(flf_ctx *ctx, const char *name, long long value) {
     const int sp = !strcmp(name, "mac_split") ? (int)value : ctx->opt_split;
     if (st < 2 || st > 16) return fail(ctx, FLF_E_ARG, "mac_stages must be in [2, 16]");
     for (int cr : {crf, crb})
-      if (cr < 2 || cr > 64 || (cr & 1)) return fail(ctx, FLF_E_ARG, "mac_chunk_rows must be even, in [2, 64], or 0 (by rule)");
+      if (cr < 2 || cr > 64) return fail(ctx, FLF_E_ARG, "mac_chunk_rows must be in [2, 64], or 0 (by rule)");
     const int ntp = (ctx->L.nthr + 31) / 32 * 32;
     if (sp < 1 || sp > 4 || 2 * sp * ntp > 256)
       return fail(ctx, FLF_E_ARG, "mac_split must be in [1, 4] with at most 256 threads per block "
@@ -1937,55 +1925,78 @@ int flf_autotune(flf_ctx *ctx, int T, int Y, int X, int *out4, void *stream) {
   if (rc != FLF_OK) return rc;
   Geometry &Gm = ctx->geo;
   const int nt = std::min(T, frames_per_pass(ctx));
-  size_t sSf, sOf, sCf, sSb, sOb, sCb;
-  ws_needs(ctx, ps, nt, true, sSf, sOf, sCf);
-  ws_needs(ctx, ps, nt, false, sSb, sOb, sCb);
-  rc = ensure_ws(ctx, ctx->wsS, std::max(sSf, sSb));
-  if (rc == FLF_OK) rc = ensure_ws(ctx, ctx->wsO, std::max(sOf, sOb));
+  rc = ensure_workspaces(ctx, ps, nt, nt, true, true);
   if (rc != FLF_OK) return rc;
-  CUDA_TRY(ctx, cudaMemsetAsync(ctx->wsS.p, 0, ctx->wsS.bytes, s));
-  // time the group that streams the most matrix bytes
-  size_t gi = 0;
-  double most = -1;
-  for (size_t g = 0; g < Gm.groups.size(); g++) {
-    const double b = (double)Gm.groups[g].nkp * ps.n[g];
-    if (b > most) { most = b; gi = g; }
-  }
+  // One pass of a projection as a call runs it (all groups, their streams and transforms),
+  // on zeros: every plane reads, or writes, the frames of one scratch buffer.  (The largest
+  // group's launch alone favours shapes that are slower beside the others': Nnum 21, 420 px,
+  // 7 planes, two frames back 209 us by rule, 224 with the shape it chose.)
+  const long long YX = (long long)Y * X;
+  Workspace frames;
+  if ((rc = ensure_ws(ctx, frames, sizeof(float) * nt * YX)) != FLF_OK) return rc;
+  const auto kept = ctx->kstats;
+  const bool profiling = ctx->profiling;
+  ctx->profiling = false;
+  int before[4];
+  std::copy(Gm.tuned, Gm.tuned + 4, before);
+  float *cimg = (float *)ctx->wsCimg.p;
+  auto project = [&](int dir) {
+    ChanImg img;
+    img.p = cimg;
+    if (dir == FLF_DIR_FORWARD)
+      return forward_chunk(ctx, (const float *)frames.p, 0, ps, 0, nt, cimg, nullptr, img, s);
+    const Strided none{nullptr, 0, 0};
+    return backward_chunk(ctx, img, ps, nt, Strided{(float *)frames.p, 0, YX}, none, none, EPI_STORE, s);
+  };
   const int ntp = (ctx->L.nthr + 31) / 32 * 32;
   const int stages_c[] = {2, 3};
-  const int chunk_c[] = {8, 10, 12, 16, 20};
   const int split_c[] = {1, 2};
-  cudaEvent_t e0, e1;
-  CUDA_TRY(ctx, cudaEventCreate(&e0));
-  CUDA_TRY(ctx, cudaEventCreate(&e1));
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  cudaError_t e = cudaMemsetAsync(frames.p, 0, frames.bytes, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(cimg, 0, ctx->wsCimg.bytes, s);
+  if (e == cudaSuccess) e = cudaEventCreate(&e0);
+  if (e == cudaSuccess) e = cudaEventCreate(&e1);
   // best[dir][stages][split] = (time, chunk)
   double bt[2][2][2];
   int bc[2][2][2];
   for (int d = 0; d < 2; d++)
     for (int a = 0; a < 2; a++)
       for (int b = 0; b < 2; b++) { bt[d][a][b] = 1e30; bc[d][a][b] = 0; }
-  cudaError_t e = cudaSuccess;
-  for (int d = 0; d < 2 && e == cudaSuccess; d++)
-    for (int a = 0; a < 2 && e == cudaSuccess; a++)
-      for (int b = 0; b < 2 && e == cudaSuccess; b++) {
+  for (int d = 0; d < 2 && e == cudaSuccess && rc == FLF_OK; d++)
+    for (int a = 0; a < 2 && e == cudaSuccess && rc == FLF_OK; a++)
+      for (int b = 0; b < 2 && e == cudaSuccess && rc == FLF_OK; b++) {
         if (2 * split_c[b] * ntp > 256) continue;
-        for (int ch : chunk_c) {
+        const bool fwd = d == FLF_DIR_FORWARD;
+        const MacThreads th = mac_threads(ctx->L, split_c[b], nt, fwd), th0 = mac_threads(ctx->L, split_c[0], nt, fwd);
+        if (b && th.shares == th0.shares) {   // the split makes no difference here
+          bt[d][a][b] = bt[d][a][0]; bc[d][a][b] = bc[d][a][0];
+          continue;
+        }
+        // the rows that the rule takes are among the candidates, so that a tuned shape is
+        // the best of them and no slower than an untuned launch
+        for (int ch : {auto_chunk_rows(ctx->L, nt, stages_c[a], fwd), 8, 10, 12, 16, 20}) {
           if (mac_shape_bytes(ctx->L, stages_c[a], ch, split_c[b]) > kMacSmemMax ||   // flf_set_tuned takes it
-              mac_smem_bytes(ctx->L, nt, stages_c[a], ch, d == FLF_DIR_FORWARD) > kMacSmemMax)   // this direction's launch
+              mac_smem_bytes(ctx->L, nt, stages_c[a], ch, fwd) > kMacSmemMax)   // this direction's launch
             continue;
-          e = mac_group_launch(ctx, gi, d, nt, ps, stages_c[a], ch, split_c[b], s);   // warm-up
-          if (e == cudaSuccess) e = cudaEventRecord(e0, s);
-          for (int k = 0; k < 3 && e == cudaSuccess; k++) e = mac_group_launch(ctx, gi, d, nt, ps, stages_c[a], ch, split_c[b], s);
-          if (e == cudaSuccess) e = cudaEventRecord(e1, s);
+          Gm.tuned[0] = stages_c[a]; Gm.tuned[1 + d] = ch; Gm.tuned[3] = split_c[b];
+          rc = project(d);   // warm-up
+          if (rc == FLF_OK) e = cudaEventRecord(e0, s);
+          for (int k = 0; k < 3 && rc == FLF_OK; k++) rc = project(d);
+          if (rc == FLF_OK && e == cudaSuccess) e = cudaEventRecord(e1, s);
           if (e == cudaSuccess) e = cudaEventSynchronize(e1);
           float ms = 0;
-          if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-          if (e != cudaSuccess) break;
+          if (rc == FLF_OK && e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+          if (rc != FLF_OK || e != cudaSuccess) break;
           if (ms < bt[d][a][b]) { bt[d][a][b] = ms; bc[d][a][b] = ch; }
         }
       }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
+  if (e0) cudaEventDestroy(e0);
+  if (e1) cudaEventDestroy(e1);
+  cudaFree(frames.p);
+  ctx->kstats = kept;
+  ctx->profiling = profiling;
+  std::copy(before, before + 4, Gm.tuned);
+  if (rc != FLF_OK) return rc;
   if (e != cudaSuccess) return fail(ctx, FLF_E_CUDA, "autotune launch failed: %s", cudaGetErrorString(e));
   if ((rc = check_device_flag(ctx)) != FLF_OK) return rc;
   int ba = 0, bb = 0;
@@ -2018,7 +2029,7 @@ int flf_set_tuned(flf_ctx *ctx, int Y, int X, const int *in4) {
   if (in4[0] < 2 || in4[0] > 16 || in4[3] < 1 || in4[3] > 4 || in4[3] * ntp > 256)
     return fail(ctx, FLF_E_ARG, "invalid launch shape");
   for (int d = 1; d <= 2; d++)
-    if (in4[d] < 2 || in4[d] > 64 || (in4[d] & 1) ||
+    if (in4[d] < 2 || in4[d] > 64 ||
         mac_shape_bytes(ctx->L, in4[0], in4[d], in4[3]) > kMacSmemMax)
       return fail(ctx, FLF_E_ARG, "invalid rows per chunk %d", in4[d]);
   for (int i = 0; i < 4; i++) Gm.tuned[i] = in4[i];

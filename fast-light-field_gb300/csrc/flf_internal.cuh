@@ -222,7 +222,7 @@ struct MacParams {
                             // and through the transpose (1): sa, sb at u, sa, sb at u* (-1: none);
                             // then the row flags (.x)
   int stages;               // shared-memory ring stages of the bulk-copy pipeline
-  int chunk_rows;           // stored rows per stage (even)
+  int chunk_rows;           // stored rows per stage
   int split;                // threads per quad in units of about 128 (1..4)
   int shares;               // row shares (set by the launcher)
   int *err;                 // set nonzero when a bounded wait gives up

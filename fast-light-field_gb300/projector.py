@@ -28,6 +28,11 @@ __all__ = ["Projector_base", "Projector_gb300", "Projector_allC", "Projector_gpu
            "CheckPlanes"]
 
 
+# Form of the multiply-accumulate that launch shapes are measured for: part of the key of a cached
+# shape, changed with the kernel, so that a file of an earlier form is measured anew.
+MAC_KERNEL = "channel-pairs"
+
+
 class Projector_base(object):
     """numpy helpers shared by projectors (reference projector.py:769-790)."""
 
@@ -172,8 +177,8 @@ class Projector_gb300(Projector_base):
 
         With ``cache_path`` the choice is stored in, and on later calls read back
         from, a JSON file keyed by device, Nnum, plane count, PSF sizes, image
-        shape, frames per launch and transform size, so tuning runs once per
-        configuration."""
+        shape, frames per launch, transform size and form of the kernel, so tuning
+        runs once per configuration."""
         ctx = self.context(hMatrix)
         self._prepare(ctx, Y, X, hMatrix)
         key = cache = None
@@ -182,7 +187,7 @@ class Projector_gb300(Projector_base):
             key = "|".join(str(v) for v in (
                 torch.cuda.get_device_name(self._dev()), hMatrix.Nnum, hMatrix.numZ,
                 tuple(tuple(hMatrix.PSFShape(cc)) for cc in range(hMatrix.numZ)), Y, X,
-                min(int(T), 4), self.fft_size, self._shape_key[3]))
+                min(int(T), 4), self.fft_size, self._shape_key[3], MAC_KERNEL))
             try:
                 with open(cache_path) as f:
                     cache = json.load(f)

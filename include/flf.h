@@ -173,7 +173,7 @@ int flf_profile_read(flf_ctx *ctx, char *buf, size_t len);
  * block-shape knobs gBlockSelection / gCalculateRowsBlocks,
  * projector.py:26-36).  Options: "mac_stages" (shared-memory pipeline
  * stages of the multiply-accumulate, 2..16), "mac_chunk_rows" (stored rows
- * per stage, even, 2..64, both directions; "mac_chunk_rows_forward" and
+ * per stage, 2..64, both directions; "mac_chunk_rows_forward" and
  * "mac_chunk_rows_backward" set one; 0, the default: by a rule on Nnum, frames
  * and stages), "mac_split" (1..4, default 1: row shares of a CTA in units of about
  * 128 threads, at most 256 threads in all; without effect where each frequency pair
@@ -401,9 +401,10 @@ int flf_graph_destroy(flf_graph *graph);
 /* Autotuner (the GB300 counterpart of the reference's FFTW planning mode,
  * SetPlanningMode, and of its block-shape knobs, projector.py:26-36): for
  * T frames of Y x X images, builds the transfer matrices if needed, then
- * times the multiply-accumulate of both directions on the transform group
- * that streams the most bytes, over ring stages {2, 3} x rows per chunk
- * {8, 10, 12, 16, 20} x row split {1, 2} (shapes that fit shared memory).
+ * times a projection of as many frames as one pass takes in both directions,
+ * over ring stages {2, 3} x rows per chunk
+ * {8, 10, 12, 16, 20 and the rule's own} x row split {1, 2} where it makes a
+ * difference (shapes that fit shared memory).
  * The fastest shape is kept with this image shape's transfer matrices and
  * used by every later call on it; out4 = {stages, rows per chunk forward,
  * rows per chunk backward, split}.  Runs work on `stream` and waits for it.
