@@ -1104,12 +1104,13 @@ int forward_chunk(flf_ctx *ctx, const float *vol, long long vol_sz, const PlaneS
     LAUNCH(ctx, "k_split", chan_bytes(ctx, nt * nplanes) + 4.0 * Y * X * nt * nplanes, s, launch_split(sp, s));
 
     Rfft2Params rp = rfft2_params(ctx, G, cvol, nt * nplanes * NN, wS);
-    LAUNCH(ctx, "k_rfft2", chan_bytes(ctx, nt * nplanes) + 8.0 * sp1 * NN * nt * nplanes, s, launch_rfft2(rp, 0, s));
+    LAUNCH(ctx, "k_rfft2", chan_bytes(ctx, nt * nplanes) + 8.0 * G.qspec() * NN * nt * nplanes, s, launch_rfft2(rp, 0, s));
 
     const double pbytes = (double)nplanes * G.nkp * L.nrow * L.RS * sizeof(float2);
     MacParams mp = mac_params(ctx, FLF_DIR_FORWARD, nt);
     mac_add_group(mp, G, FLF_DIR_FORWARD, ps.slots[gi], nplanes, zgroup, wS, wO);
-    LAUNCH(ctx, "k_mac_fwd", pbytes + 8.0 * sp1 * NN * nt * ((double)nplanes + nzg), s, launch_mac(mp, true, s));
+    LAUNCH(ctx, "k_mac_fwd", pbytes + 8.0 * NN * nt * ((double)G.qspec() * nplanes + (double)sp1 * nzg), s,
+           launch_mac(mp, true, s));
 
     if (k > 0 && nslot > 1) CUDA_TRY(ctx, cudaStreamWaitEvent(s, ctx->ev_chain, 0));
     Irfft2Params ip = irfft2_params(ctx, G, wO, nt * NN, chan);
@@ -1211,20 +1212,20 @@ int backward_chunk(flf_ctx *ctx, const ChanImg &img, const PlaneSet &ps, int nt,
     void *wS = (char *)ctx->wsS.p + slot * sS;
     float2 *wO = (float2 *)((char *)ctx->wsO.p + slot * sO);
     const Group &G = Gm.groups[gi];
-    const size_t sp1 = G.spec();
+    const double qs = (double)G.qspec();
 
     Rfft2Params rp = rfft2_params(ctx, G, chan, nt * NN, wS);
-    LAUNCH(ctx, "k_rfft2", chan_bytes(ctx, nt) + 8.0 * sp1 * NN * nt, s, launch_rfft2(rp, 0, s));
+    LAUNCH(ctx, "k_rfft2", chan_bytes(ctx, nt) + 8.0 * qs * NN * nt, s, launch_rfft2(rp, 0, s));
 
     const double pbytes = (double)nplanes * G.nkp * L.nrow * L.RS * sizeof(float2);
     const int zgb = zgroup_for(ctx, nplanes, G.nquads, ctas_per_sm(ctx, FLF_DIR_BACKWARD, nt));
     MacParams mp = mac_params(ctx, FLF_DIR_BACKWARD, nt);
     mac_add_group(mp, G, FLF_DIR_BACKWARD, ps.slots[gi], nplanes, zgb, wS, wO);
-    LAUNCH(ctx, "k_mac_bwd", pbytes + 8.0 * sp1 * NN * nt * (1.0 + nplanes), s, launch_mac(mp, false, s));
+    LAUNCH(ctx, "k_mac_bwd", pbytes + 8.0 * qs * NN * nt * (1.0 + nplanes), s, launch_mac(mp, false, s));
 
     Irfft2Params ip = irfft2_params(ctx, G, wO, nt * nplanes * NN, cvol);
     ip.final_pass = 1; ip.quads = 1;
-    LAUNCH(ctx, "k_irfft2", 8.0 * sp1 * NN * nt * nplanes + chan_bytes(ctx, nt * nplanes), s, launch_irfft2(ip, s));
+    LAUNCH(ctx, "k_irfft2", 8.0 * qs * NN * nt * nplanes + chan_bytes(ctx, nt * nplanes), s, launch_irfft2(ip, s));
 
     MergeParams mg = merge_params(ctx, cvol, ps.ids[gi], nplanes, nt, epi, out, aux, norm);
     const int npix = epi == EPI_STORE ? 1 : (epi == EPI_RL_STANDARD && norm.p ? 4 : 3);
