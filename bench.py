@@ -44,9 +44,9 @@ METRIC = "volumes/s to plain-RL(8 it) accuracy: learned warm-start vs plain RL, 
 
 # DRAM bytes (read + write) per k_mac launch over the bytes it streams, from one
 # ncu --set full capture of the full-field f = 96 launches (4 planes, 1225
-# frequency quads: 1.022 forward, 1.016 back projection).  The matrices dominate
+# frequency quads: 1.004 forward, 1.007 back projection).  The matrices dominate
 # both, so the traffic of a launch scales with the bytes it streams.
-MAC_TRAFFIC_RATIO = 1.02
+MAC_TRAFFIC_RATIO = 1.006
 UNIT = "volumes/s"
 
 WORKLOADS = {
@@ -287,10 +287,11 @@ def survey_psf_bytes(N, Y, X, hs):
 
 
 def mac_roofline(prof, survey_bytes, what):
-    """Roofline of k_mac from a per-kernel profile pass: achieved = the compulsory
-    PSF-spectrum bytes of the projections profiled (survey_psf_bytes) over the
-    kernel's total CUDA-event time, against the measured HBM copy peak; the
-    kernel's own streamed bytes and their fraction beside it."""
+    """Roofline of k_mac from a per-kernel profile pass: achieved = the bytes the
+    kernel streams over its total CUDA-event time, against the measured HBM copy
+    peak.  Beside it the same with the PSF-spectrum bytes of the projections
+    profiled (survey_psf_bytes), of which the packed matrices store less, so that
+    this ratio can pass 1."""
     peak, peak_kind = measured_peaks()
     mac = {k: v for k, v in prof.items() if k.startswith("k_mac")}
     tot_ms = sum(v["ms"] for v in mac.values())
@@ -299,7 +300,8 @@ def mac_roofline(prof, survey_bytes, what):
     ach = survey_bytes / (tot_ms / 1000.0) / 1e9 if tot_ms > 0 else 0.0
     own_ach = own / (tot_ms / 1000.0) / 1e9 if tot_ms > 0 else 0.0
     tot_all = sum(w["ms"] for w in prof.values()) or 1.0
-    return {"bound": "hbm", "achieved": round(ach, 1), "peak": peak, "unit": "GB/s", "frac": round(ach / peak, 4),
+    return {"bound": "hbm", "achieved": round(own_ach, 1), "peak": peak, "unit": "GB/s",
+            "frac": round(own_ach / peak, 4),
             "traffic": round(own / n * MAC_TRAFFIC_RATIO),
             "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per k_mac launch, as a ratio to "
                               "the kernel's own streamed bytes (%.3f), times this run's own bytes per launch"
@@ -309,6 +311,7 @@ def mac_roofline(prof, survey_bytes, what):
             "algorithmic_bytes_per_launch": survey_bytes / n,
             "algorithmic_bytes": "sum over planes of K F_z (F_z/2+1) 8 B per projection, K = 36 stored PSFs, "
                                  "F_z = Nnum ceil((Y + h_z - 1) / Nnum); %s" % what,
+            "algorithmic_achieved": round(ach, 1), "algorithmic_over_peak": round(ach / peak, 4),
             "own_bytes_per_launch": own / n, "own_achieved": round(own_ach, 1),
             "own_frac": round(own_ach / peak, 4),
             "kernel_share": {k: round(v["ms"] / tot_all, 4) for k, v in prof.items()}}

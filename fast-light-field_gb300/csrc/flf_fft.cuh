@@ -325,8 +325,8 @@ __device__ __forceinline__ void quad_of(int k, int &lo, int &hi) {
 // ----------------------------------------------------------------------------
 // Forward transform of channel-major images (Rfft2Params mode 0): image g is
 // channel ch = g % NN = b*N + a, Ly x Lx samples of pixels (r*N + b, c*N + a);
-// samples outside the Y x X image read as zero.  Output spectrum
-// dst[g][ky][kx], ky < F, kx <= F/2, natural order.
+// samples outside the Y x X image read as zero.  The output spectrum is in quad
+// order, dst[g][quad][4].
 // ----------------------------------------------------------------------------
 template <int F>
 __global__ void __launch_bounds__(Shape<F>::NT, Shape<F>::MINB) k_rfft2_sized(Rfft2Params p, SizedArgs sa) {

@@ -223,7 +223,7 @@ struct MacParams {
                             // then the row flags (.x)
   int stages;               // shared-memory ring stages of the bulk-copy pipeline
   int chunk_rows;           // stored rows per stage
-  int split;                // threads per quad in units of about 128 (1..4)
+  int split;                // row shares in units of about 128 threads (1..4), where mac_threads asks for it
   int shares;               // row shares (set by the launcher)
   int *err;                 // set nonzero when a bounded wait gives up
   unsigned long long wait_ns;   // limit of each wait for a ring slot (1 s)
